@@ -35,7 +35,8 @@ namespace {
 using namespace pbd;
 
 constexpr uint32_t kNoAllocMaxKeys = 1u << 20;
-constexpr uint32_t kNoAllocMaxTiles = (kNoAllocMaxKeys + kSortTile - 1) / kSortTile;
+constexpr uint32_t kNoAllocMaxTiles = 256;   // look-back rows; sort_plan needs at most 158 for kNoAllocMaxKeys
+static_assert(kNoAllocMaxKeys <= kNoAllocMaxTiles * (uint32_t)(kSortThreads * kSortItemsMax) && kSortSpread <= kNoAllocMaxTiles, "look-back rows");
 // word offsets inside the array
 constexpr size_t kOffKeys = 0;
 constexpr size_t kOffVals = kOffKeys + kNoAllocMaxKeys;
@@ -133,7 +134,7 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
     if (int rc = scratch_for_current_device(&base)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const int npasses = (int)((key_bits + kRadixBits - 1) / kRadixBits);
-    const uint32_t ntiles = (n + kSortTile - 1) / kSortTile;
+    const SortPlan plan = sort_plan(n);
     SortScratch S{base + kOffHist, base + kOffStatus, base + kOffTiles, base + kOffErr, kNoAllocMaxTiles};
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
@@ -142,7 +143,7 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
     }
     S.key_bits = key_bits;
 
-    noalloc_clear_kernel<<<32, 256, 0, st>>>(base, ntiles);
+    noalloc_clear_kernel<<<32, 256, 0, st>>>(base, plan.ntiles);
     const uint32_t gh = std::min<uint32_t>((n + 255) / 256, 1024u);
     noalloc_hist_kernel<<<gh, 256, 0, st>>>(d_keys_in, n, S.hist, npasses, key_bits);
     // Ping-pong between the caller's outputs and the fixed array so that the last pass
@@ -155,10 +156,7 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
         const bool to_out = ((npasses - 1 - pass) % 2) == 0;
         uint32_t* dk = to_out ? d_keys_out : tmp_k;
         uint32_t* dv = to_out ? d_perm_out : tmp_v;
-        if (pass == 0)
-            onesweep_pass<true><<<ntiles, kSortThreads, 0, st>>>(src_k, src_v, dk, dv, n, pass, S);
-        else
-            onesweep_pass<false><<<ntiles, kSortThreads, 0, st>>>(src_k, src_v, dk, dv, n, pass, S);
+        sort_pass(st, plan, src_k, src_v, dk, dv, n, pass, S);
         src_k = dk;
         src_v = dv;
     }

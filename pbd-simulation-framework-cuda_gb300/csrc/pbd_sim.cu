@@ -402,14 +402,12 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     PROF_END();
     ++nl;
     // sortIds
-    const uint32_t ntiles = div_up(N, kSortTile);
+    const SortPlan plan = sort_plan(N);
+    const uint32_t ntiles = plan.ntiles;
     for (int pass = 0; pass < np; ++pass) {
         const int in = pass % 2, out = (pass + 1) % 2;
         PROF_BEGIN("onesweep_pass");
-        if (pass == 0)
-            onesweep_pass<true><<<ntiles, kSortThreads, 0, st>>>(s->keys[in], s->vals[in], s->keys[out], s->vals[out], N, pass, S);
-        else
-            onesweep_pass<false><<<ntiles, kSortThreads, 0, st>>>(s->keys[in], s->vals[in], s->keys[out], s->vals[out], N, pass, S);
+        sort_pass(st, plan, s->keys[in], s->vals[in], s->keys[out], s->vals[out], N, pass, S);
         PROF_END();
         ++nl;
     }
@@ -846,7 +844,7 @@ int create_sim(const pbd_params* prm, uint32_t capacity, const std::vector<Scene
     if (e != cudaSuccess) { delete s; return cuda_fail("cudaGetDevice", e); }
     e = cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, s->device);
     if (e != cudaSuccess) { delete s; return cuda_fail("cudaDeviceGetAttribute", e); }
-    s->max_tiles = div_up(capacity, kSortTile);
+    s->max_tiles = sort_max_tiles(capacity);
     // ---- one arena, 256-byte aligned slices
     const size_t C = capacity, T = table_size(s);
     std::vector<std::pair<void**, size_t>> parts;

@@ -7,19 +7,25 @@
 // Design (one kernel per 8-bit digit, "onesweep" style):
 //  - The digit histograms of every pass are counted once, fused into the predict kernel
 //    (shared-memory histograms flushed with one global atomic per non-empty bin).
-//  - Each pass kernel takes a tile of kSortTile keys.  Tiles are numbered by an atomic
+//  - Each pass kernel takes a tile of keys (sort_plan).  Tiles are numbered by an atomic
 //    counter in launch order, so a tile only ever waits on tiles that are already running.
-//  - Inside a tile every warp ranks its items with __match_any_sync (stable: item order is
-//    warp, then register slot, then lane); warp counts are scanned per digit in shared
-//    memory.
+//  - Inside a tile every warp ranks its items (stable: item order is warp, then register slot,
+//    then lane) from one ballot per digit bit; warp counts are scanned per digit in shared memory.
 //  - Tile digit counts are chained across tiles with decoupled look-back (status word =
-//    2 flag bits + 30 count bits).  Every wait is bounded: after SortScratch::spin_limit polls
-//    (kSpinLimit by default, a few seconds) the tile records PBD device error bit
-//    kErrSortTimeout and carries on, so a lost predecessor can never hang the GPU.  For tests
-//    of that path, SortScratch::hold makes the first tile of every pass withhold its status
-//    (a predecessor that never publishes): every wait on it runs out.
+//    2 flag bits + 30 count bits), kLookBack words in flight at a time.  Every wait is bounded:
+//    after SortScratch::spin_limit polls without progress (kSpinLimit by default, a few seconds)
+//    the tile records PBD device error bit kErrSortTimeout and carries on, so a lost predecessor
+//    can never hang the GPU.  For tests of that path, SortScratch::hold makes the first tile of
+//    every pass withhold its status (a predecessor that never publishes): every wait on it runs out.
 //  - Keys are scattered to shared memory in tile order first, then written out so that
 //    each digit's run lands on consecutive global addresses.
+//
+// What bounds it: the serial chain inside a tile (load, rank item after item through the warp's
+// counts, scan, look back, scatter, write), not DRAM (16 B per key and pass).  So a tile has 512
+// threads with few items each and the ranks come from ballots (__match_any_sync cost ~200 cycles an
+// item).  Three passes, back to back, GB300: 1,000,000 keys 64 -> 46 us, 600,001 keys 47 -> 35,
+// 262,144 keys 42 -> 29, 33,000 keys 35 -> 21, 4,275 keys 31 -> 19 (256 threads x 16 items with
+// __match_any_sync and one status word per look-back step, against the present passes).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -29,10 +35,30 @@ namespace pbd {
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kMaxPasses = 4;
-constexpr int kSortThreads = 256;          // == kRadix: thread d owns digit d
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;   // 4096 keys per tile (2048 and 3072 were slower)
+constexpr int kSortThreads = 512;          // threads 0..255 own a digit each
+constexpr int kLookBack = 8;               // status words a look-back step reads (16 and 4: the same time)
+// Keys per tile: the smallest of 1,024 / 2,048 / 4,096 that needs at most one tile per SM (152), as
+// a tile's time grows with its items per thread (262,144 keys, three passes: 4 items 28 us, 8 items
+// 33, 2 items and two tiles per SM 33); beyond that 6,656 keys, the most that fit in static shared
+// memory with 16 warps (1,000,000 keys: 151 tiles, 46 us against 52 with 245 tiles of
+// 4,096; 4,000,000 keys: 121 us against 126).
+constexpr uint32_t kSortSpread = 152;
+constexpr int kSortItemsMax = 13;
+struct SortPlan {
+    int items;        // keys per thread
+    uint32_t ntiles;
+};
+inline SortPlan sort_plan(uint32_t n) {
+    for (int items : {2, 4, 8})
+        if (n <= kSortSpread * (uint32_t)(kSortThreads * items))
+            return SortPlan{items, (n + kSortThreads * items - 1) / (uint32_t)(kSortThreads * items)};
+    return SortPlan{kSortItemsMax, (n + kSortThreads * kSortItemsMax - 1) / (uint32_t)(kSortThreads * kSortItemsMax)};
+}
+// Status rows that sort_plan needs at most for up to `capacity` keys.
+inline uint32_t sort_max_tiles(uint32_t capacity) {
+    const uint32_t t = sort_plan(capacity).ntiles;
+    return t > kSortSpread ? t : kSortSpread;
+}
 constexpr uint32_t kFlagAggregate = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
@@ -75,126 +101,128 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
-// Exclusive scan of one value per thread over a 256-thread block.  `warp_tot` is 8 words of
-// shared memory.  Returns the exclusive prefix; the block total is written to *total.
-__device__ __forceinline__ uint32_t block_exclusive_scan256(uint32_t v, uint32_t* warp_tot, uint32_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t t = lane < kSortWarps ? warp_tot[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < kSortWarps; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        if (lane < kSortWarps) warp_tot[lane] = t;   // inclusive warp totals
-    }
-    __syncthreads();
-    uint32_t base = warp > 0 ? warp_tot[warp - 1] : 0u;
-    if (total) *total = warp_tot[kSortWarps - 1];
-    return base + x - v;
-}
-
 // One LSD pass over digit `pass` (bits 8*pass .. 8*pass+7).  kFirst: values are the
 // identity (initializeParticleIds, SortReorder.h:199-210) and are generated, not loaded.
-template <bool kFirst>
+template <bool kFirst, int kItems>
 __global__ void __launch_bounds__(kSortThreads)
 onesweep_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
               uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n, int pass,
               SortScratch S) {
-    __shared__ uint32_t s_whist[kSortWarps][kRadix];
-    __shared__ uint32_t s_keys[kSortTile];
-    __shared__ uint32_t s_vals[kSortTile];
+    constexpr int kThreads = kSortThreads, kWarps = kThreads / 32;
+    constexpr int kTile = kThreads * kItems;
+    static_assert(kThreads >= kRadix && kTile <= 65535, "thread d < 256 owns digit d; tile counts are 16-bit");
+    __shared__ uint16_t s_whist[kWarps][kRadix];
+    __shared__ uint32_t s_keys[kTile];
+    __shared__ uint32_t s_vals[kTile];
     __shared__ uint32_t s_goff[kRadix];
     __shared__ uint32_t s_start[kRadix];
-    __shared__ uint32_t s_wtot[kSortWarps];
+    __shared__ uint32_t s_wtot[2][kRadix / 32];
     __shared__ uint32_t s_tile;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(&S.tile_counter[pass], 1u);
-    for (int k = tid; k < kSortWarps * kRadix; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
+    for (int k = tid; k < kWarps * kRadix / 2; k += kThreads) reinterpret_cast<uint32_t*>(&s_whist[0][0])[k] = 0u;
+    const uint32_t hist = tid < kRadix ? S.hist[pass * kRadix + tid] : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     // The previous pass has finished (stream order): clear its look-back row for this tile.
-    if (pass > 0) S.status[((size_t)(pass - 1) * S.max_tiles + tile) * kRadix + tid] = 0u;
+    if (pass > 0 && tid < kRadix) S.status[((size_t)(pass - 1) * S.max_tiles + tile) * kRadix + tid] = 0u;
 
-    const uint32_t base = tile * (uint32_t)kSortTile;
-    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+    const uint32_t base = tile * (uint32_t)kTile;
+    uint32_t key[kItems], val[kItems], rank[kItems];
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t idx = base + warp * (32 * kItems) + k * 32 + lane;
         const bool valid = idx < n;
         key[k] = valid ? kin[idx] : 0xFFFFFFFFu;
         val[k] = kFirst ? idx : (valid ? vin[idx] : 0u);
     }
-    // ---- warp-level stable ranking
-    uint32_t* wh = s_whist[warp];
+    // ---- warp-level stable ranking: the lanes holding the same digit from one ballot per bit
+    uint16_t* wh = s_whist[warp];
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t idx = base + warp * (32 * kItems) + k * 32 + lane;
         const bool valid = idx < n;
         const uint32_t digit = sort_digit(key[k], pass, S.key_bits);
-        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? digit : (uint32_t)kRadix);
+        uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < kRadixBits; ++b) {
+            const uint32_t ones = __ballot_sync(0xffffffffu, (digit >> b) & 1u);
+            peers &= ((digit >> b) & 1u) ? ones : ~ones;
+        }
         const uint32_t before = valid ? wh[digit] : 0u;
         __syncwarp();
-        if (valid && (peers & lt) == 0u) wh[digit] = before + __popc(peers);
+        if (valid && (peers & lt) == 0u) wh[digit] = (uint16_t)(before + __popc(peers));
         __syncwarp();
         rank[k] = before + __popc(peers & lt);
     }
     __syncthreads();
-    // ---- per digit (thread d): warp offsets, tile count, look-back
-    const uint32_t d = tid;
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-        uint32_t c = s_whist[w][d];
-        s_whist[w][d] = run;
-        run += c;
-    }
+    // ---- per digit (thread d): warp offsets and the tile's count, published for the tiles after
+    // this one; then one scan over the digits of both the tile's counts and the whole array's
     uint32_t* st = S.status + (size_t)pass * S.max_tiles * kRadix;
-    uint32_t excl = 0;
-    if (tile == 0) {
-        if (!S.hold) st_relaxed(&st[d], kFlagPrefix | run);
-    } else {
-        st_relaxed(&st[(size_t)tile * kRadix + d], kFlagAggregate | run);
+    const uint32_t d = tid;
+    uint32_t run = 0, rx = 0, hx = 0;
+    if (tid < kRadix) {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t c = s_whist[w][d];
+            s_whist[w][d] = (uint16_t)run;
+            run += c;
+        }
+        if (!(tile == 0 && S.hold)) st_relaxed(&st[(size_t)tile * kRadix + d], (tile == 0 ? kFlagPrefix : kFlagAggregate) | run);
+        rx = run;
+        hx = hist;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, rx, o), b = __shfl_up_sync(0xffffffffu, hx, o);
+            if (lane >= o) { rx += a; hx += b; }
+        }
+        if (lane == 31) { s_wtot[0][warp] = rx; s_wtot[1][warp] = hx; }
+        rx -= run;
+        hx -= hist;
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+#pragma unroll
+        for (int w = 0; w < kRadix / 32 - 1; ++w)
+            if (w < warp) { rx += s_wtot[0][w]; hx += s_wtot[1][w]; }
+        // ---- look back over the tiles before this one, kLookBack status words in flight at a time
+        uint32_t excl = 0, spins = 0;
         int t = (int)tile - 1;
         while (t >= 0) {
-            uint32_t w = 0, spins = 0;
-            for (;;) {
-                w = ld_relaxed(&st[(size_t)t * kRadix + d]);
-                if (w >> 30) break;
-                if (++spins > S.spin_limit) {
-                    atomicOr(S.err, kErrSortTimeout);
-                    w = kFlagPrefix;
-                    break;
+            uint32_t w[kLookBack];
+#pragma unroll
+            for (int k = 0; k < kLookBack; ++k) w[k] = t >= k ? ld_relaxed(&st[(size_t)(t - k) * kRadix + d]) : 0u;
+            int taken = 0;
+            bool done = false, open = true;
+#pragma unroll
+            for (int k = 0; k < kLookBack; ++k) {
+                open = open && !done && (w[k] >> 30) != 0u;
+                if (open) {
+                    excl += w[k] & kValueMask;
+                    ++taken;
+                    done = (w[k] >> 30) == 2u;
                 }
-                __nanosleep(32);
             }
-            excl += w & kValueMask;
-            if ((w >> 30) == 2u) break;
-            --t;
+            if (done) break;
+            t -= taken;
+            if (taken != 0) { spins = 0; continue; }
+            if (++spins > S.spin_limit) {
+                atomicOr(S.err, kErrSortTimeout);
+                break;
+            }
+            __nanosleep(32);
         }
-        st_relaxed(&st[(size_t)tile * kRadix + d], kFlagPrefix | (excl + run));
+        if (tile != 0) st_relaxed(&st[(size_t)tile * kRadix + d], kFlagPrefix | ((excl + run) & kValueMask));
+        s_goff[d] = hx + excl - rx;
+        s_start[d] = rx;
     }
-    // ---- global digit base (exclusive scan of the whole-array histogram) and tile starts
-    const uint32_t hx = block_exclusive_scan256(S.hist[pass * kRadix + d], s_wtot, nullptr);
-    __syncthreads();
-    const uint32_t rx = block_exclusive_scan256(run, s_wtot, nullptr);
-    s_goff[d] = hx + excl - rx;
-    s_start[d] = rx;
     __syncthreads();
     // ---- scatter to shared memory in tile order
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t idx = base + warp * (32 * kItems) + k * 32 + lane;
         if (idx < n) {
             const uint32_t digit = sort_digit(key[k], pass, S.key_bits);
             const uint32_t pos = s_start[digit] + s_whist[warp][digit] + rank[k];
@@ -203,8 +231,8 @@ onesweep_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin
         }
     }
     __syncthreads();
-    const uint32_t tile_n = (n - base) < (uint32_t)kSortTile ? (n - base) : (uint32_t)kSortTile;
-    for (uint32_t i = tid; i < tile_n; i += kSortThreads) {
+    const uint32_t tile_n = (n - base) < (uint32_t)kTile ? (n - base) : (uint32_t)kTile;
+    for (uint32_t i = tid; i < tile_n; i += kThreads) {
         const uint32_t kk = s_keys[i];
         const uint32_t o = s_goff[sort_digit(kk, pass, S.key_bits)] + i;
         if (o < n) {            // always true unless a look-back wait gave up (error word set)
@@ -212,6 +240,20 @@ onesweep_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin
             vout[o] = s_vals[i];
         }
     }
+}
+
+template <int kItems>
+inline void launch_sort_pass(cudaStream_t st, uint32_t ntiles, bool first, const uint32_t* kin, const uint32_t* vin,
+                             uint32_t* kout, uint32_t* vout, uint32_t n, int pass, const SortScratch& S) {
+    if (first) onesweep_pass<true, kItems><<<ntiles, kSortThreads, 0, st>>>(kin, vin, kout, vout, n, pass, S);
+    else onesweep_pass<false, kItems><<<ntiles, kSortThreads, 0, st>>>(kin, vin, kout, vout, n, pass, S);
+}
+// Queue pass `pass` of a sort of n keys (the values of the first pass are the identity).
+inline void sort_pass(cudaStream_t st, const SortPlan& plan, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
+                      uint32_t* vout, uint32_t n, int pass, const SortScratch& S) {
+    const auto launch = plan.items == 2 ? launch_sort_pass<2> : plan.items == 4 ? launch_sort_pass<4>
+                        : plan.items == 8 ? launch_sort_pass<8> : launch_sort_pass<kSortItemsMax>;
+    launch(st, plan.ntiles, pass == 0, kin, vin, kout, vout, n, pass, S);
 }
 
 }  // namespace pbd

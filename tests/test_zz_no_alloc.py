@@ -96,3 +96,14 @@ def test_noalloc_sort_rejects_more_keys_than_its_fixed_memory(need_gpu, pbd):
     rc = pbd.lib().pbd_sort_keys_noalloc(ptr, ptr, ptr, (1 << 20) + 1, 24, None)
     assert rc == pbd.ERR_CAPACITY
     assert b"at most 1048576" in pbd.lib().pbd_last_error()
+
+
+@pytest.mark.parametrize("n", [1024, 1025, 152 * 1024, 152 * 1024 + 1, 152 * 2048 + 1, 152 * 4096, 152 * 4096 + 1, 6656 * 150 + 1])
+def test_noalloc_sort_at_the_edges_of_its_tile_sizes(need_gpu, pbd, n):
+    # the tile size follows n (sort_plan): the last n of a size, the first of the next, one key over
+    rng = np.random.default_rng(n)
+    keys = (rng.integers(0, 1 << 21, size=n, dtype=np.uint64) >> rng.integers(0, 12, size=n, dtype=np.uint64)).astype(np.uint32)
+    order = np.argsort(keys, kind="stable")
+    k, p = _sort_noalloc(pbd, keys, key_bits=21)
+    assert np.array_equal(p, order.astype(np.uint32)) and np.array_equal(k, keys[order])
+    assert pbd.lib().pbd_sort_noalloc_status(None) == pbd.OK
