@@ -224,7 +224,7 @@ template <class V>
 __device__ __forceinline__ void walk_frame_list(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
                                                 const float4* __restrict__ p, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ ce, const NbList& F, uint32_t fm, V& vis) {
-    if (fm != kListOff) {
+    if (!(fm & kListOff)) {
         walk_list(F, i, fm, p, vis);
     } else {
         bool deferred = false;

@@ -17,7 +17,8 @@
 //    to walk_seq.  It takes the particles whose walk meets a cell range longer than
 //    kLongRange -- in practice the range that SortReorder.h:183-184 extends to N (up to M
 //    entries) -- which would otherwise serialise a whole warp behind one thread;
-//  - walk_list: one thread per particle over a stored list.
+//  - walk_list: one thread per particle over a stored list;
+//  - walk_row: one warp per particle over a stored list (the long lists, LongLists).
 #pragma once
 #include <type_traits>
 #include "pbd_device.cuh"
@@ -71,13 +72,27 @@ struct DeferList {
 //    positions it read); the pass right after it reads the same positions (delta after lambda,
 //    viscosity after omega), so every entry left out adds an exact zero there and the short
 //    list gives the full walk's sums bit for bit.
-// A particle whose list does not fit (or whose walk met a long cell range) walks the cells.
-constexpr uint32_t kListOff = 0x80000000u;   // meta: this particle walks the cells
+// A particle whose list does not fit (or whose walk met a long cell range) has its list stored by
+// a warp (LongLists), or walks the cells when those are full.
+constexpr uint32_t kListOff = 0x80000000u;   // meta: no list here (a full list's meta: | kListWalked | its set slot)
+constexpr uint32_t kListWalked = 0x40000000u;   // with kListOff: the first lambda pass walked this particle itself
 struct NbList {
     uint32_t* list;      // kmax x stride entries, slot-major (slot k of particle i at k * stride + i)
     uint32_t* meta;      // per particle: count | contacts << 8, or kListOff
     uint32_t stride;
     uint32_t kmax;       // <= 255
+};
+// The lists of the particles without a full list (the set DF, slot q of the set at row q): stored
+// once per frame by the warp that finishes their first lambda pass, read by a warp in every pass
+// after it.  Walking the cells again in each pass cost two dependent table loads and a position
+// load per cell, one cell after the other (125 cells with two shells): on a 152k-particle dense
+// frame the 125 particles around the cell-end range held up every pass by 100 us and more.
+constexpr uint32_t kLongSlots = 8192;   // rows (16 MB); particles beyond them walk the cells
+constexpr uint32_t kLongMax = 512;      // entries of a row: config.txt's list cap
+struct LongLists {
+    uint32_t* list;      // slots x kLongMax
+    uint32_t* meta;      // per row: count | contacts << 16, or kListOff (longer than kLongMax)
+    uint32_t slots;
 };
 
 // Enumerate the non-empty cell ranges [s, e) of particle i's list in the reference's
@@ -205,6 +220,138 @@ __device__ __forceinline__ uint32_t walk_coop(const DevParams& P, const SceneCtx
     auto endc = [&]() -> bool { vis.end_contacts(cnt); return false; };
     for_each_range(P, S, anchor, cs, ce, range, endc);
     return cnt;
+}
+
+// Cell t of findNeighbours' shell sh, in list order (Collision.h:127-134: edge columns hold every
+// c, interior columns only c = -sh and c = +sh).  The shell has side^3 - (side - 2)^3 cells.
+__device__ __forceinline__ void shell_cell(int sh, int t, int& a, int& b, int& c) {
+    const int side = 2 * sh + 1, slab = side * side, ring = 4 * side - 4;
+    const bool last = t >= slab + (side - 2) * ring;
+    if (t < slab || last) {
+        if (last) t -= slab + (side - 2) * ring;
+        a = last ? sh : -sh;
+        b = t / side - sh;
+        c = t % side - sh;
+        return;
+    }
+    t -= slab;
+    a = t / ring - sh + 1;
+    t %= ring;
+    if (t < side) { b = -sh; c = t - sh; return; }
+    t -= side;
+    if (t < 2 * (side - 2)) { b = t / 2 - sh + 1; c = (t & 1) ? sh : -sh; return; }
+    b = sh;
+    c = t - 2 * (side - 2) - sh;
+}
+
+// One warp stores particle i's list (the entries and order of for_each_range, without i, up to the
+// cap M) into `row`: a lane per cell for the table loads, then a lane per entry, which finds its
+// cell by a search over the lanes' offsets.  Returns the row's meta.
+__device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
+                                              const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                                              uint32_t* row) {
+    const uint32_t lane = lane_id();
+    const uint32_t cap = min(P.M, kLongMax + 1u);   // one past the row's room: too long
+    const bool quirk = (P.flags & PBD_FLAG_CELL_END_QUIRK) && S.n >= 2;
+    uint32_t n = 0, nc = 0;
+    auto cells = [&](bool in, int a, int b, int c) {
+        uint32_t s = 0, len = 0, own = 0;
+        if (in) {
+            const uint32_t h = (morton_axis(__fmaf_rn((float)a, P.d, anchor.x)) << 2) +
+                               (morton_axis(__fmaf_rn((float)b, P.d, anchor.y)) << 1) +
+                               morton_axis(__fmaf_rn((float)c, P.d, anchor.z));
+            if (h < S.cells) {
+                s = __ldg(cs + S.base + h);
+                uint32_t e = __ldg(ce + S.base + h);
+                if (s < P.N) {
+                    if ((quirk && h == S.n - 1) || e > S.end) e = S.end;
+                    if (e > s) {
+                        own = (s <= i && i < e) ? 1u : 0u;
+                        len = min(e - s - own, cap);
+                    }
+                }
+            }
+        }
+        uint32_t off = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFullMask, off, o);
+            if (lane >= (uint32_t)o) off += v;
+        }
+        const uint32_t total = __shfl_sync(kFullMask, off, 31);
+        off -= len;
+        for (uint32_t o0 = 0; o0 < total && n + o0 < cap; o0 += 32u) {
+            const uint32_t o = o0 + lane;
+            uint32_t q = 0;   // the last lane whose offset is not beyond o
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1) {
+                const uint32_t v = __shfl_sync(kFullMask, off, q + step);
+                if (v <= o) q += step;
+            }
+            const uint32_t qs = __shfl_sync(kFullMask, s, q), qo = __shfl_sync(kFullMask, off, q);
+            const uint32_t qi = __shfl_sync(kFullMask, own, q);
+            uint32_t j = qs + (o - qo);
+            if (qi && j >= i) ++j;
+            if (o < total && n + o < P.M && n + o < kLongMax) row[n + o] = j;
+        }
+        n = min(n + total, cap);
+    };
+    if (P.active & PBD_ACTIVE_FIND_CONTACTS) {
+        const int t = (int)lane;
+        cells(t < 27, t / 9 - 1, (t / 3) % 3 - 1, t % 3 - 1);
+        nc = n;
+    }
+    if (P.active & PBD_ACTIVE_FIND_NEIGHBOURS)
+        for (int sh = 2; sh <= (int)P.K && n < cap; ++sh) {
+            const int side = 2 * sh + 1, count = side * side * side - (side - 2) * (side - 2) * (side - 2);
+            for (int t0 = 0; t0 < count && n < cap; t0 += 32) {
+                const int t = t0 + (int)lane;
+                int a = 0, b = 0, c = 0;
+                if (t < count) shell_cell(sh, t, a, b, c);
+                cells(t < count, a, b, c);
+            }
+        }
+    return n > kLongMax ? kListOff : (n | (nc << 16));
+}
+
+// One warp per particle over a stored list (entry k at row[k * st]): lanes evaluate 32 entries at a
+// time, two such groups of position loads in flight, and the contributions that change a sum are
+// added in list order through shuffles, as in walk_coop.
+template <class V>
+__device__ __forceinline__ void walk_row(const uint32_t* row, size_t st, uint32_t n, uint32_t nc, uint32_t i,
+                                         const float4* __restrict__ p, V& vis) {
+    const uint32_t lane = lane_id();
+    auto part = [&](uint32_t k0, uint32_t k1, bool contact) {
+        for (uint32_t kb = k0; kb < k1; kb += 64u) {
+            uint32_t j[2];
+            float4 pj[2];
+            typename ExtraOf<V>::type ex[2];
+#pragma unroll
+            for (uint32_t b = 0; b < 2u; ++b) {
+                const uint32_t k = kb + b * 32u + lane;
+                j[b] = k < k1 ? row[(size_t)k * st] : i;
+            }
+#pragma unroll
+            for (uint32_t b = 0; b < 2u; ++b) {
+                pj[b] = __ldg(p + j[b]);
+                ex[b] = fetch_extra(vis, j[b]);
+            }
+#pragma unroll
+            for (uint32_t b = 0; b < 2u; ++b) {
+                const bool valid = kb + b * 32u + lane < k1;
+                const typename V::Contrib c = valid ? contrib_of(vis, j[b], pj[b], ex[b], contact) : V::zero();
+                uint32_t take = __ballot_sync(kFullMask, valid && V::effective(c));
+                while (take) {
+                    const int k = __ffs(take) - 1;
+                    take &= take - 1u;
+                    vis.add(V::shfl(c, k), contact);
+                }
+            }
+        }
+    };
+    part(0u, nc, true);
+    vis.end_contacts(nc);
+    part(nc, n, false);
 }
 
 // One thread per particle over a stored list (meta not kListOff): the contact entries, then
@@ -630,9 +777,30 @@ __device__ __forceinline__ void run_coop_set(const CoopSet& C, F&& f) {
         }
     }
 }
-// Append i to a set when the set is given (items non-null).
-__device__ __forceinline__ void note_particle(const DeferList& D, uint32_t i) {
-    if (D.items) defer_particle(D, i);
+// Append i to a set when the set is given (items non-null); returns its slot there.  The sets hold
+// every particle of the simulation, so there is always room.
+__device__ __forceinline__ uint32_t note_particle(const DeferList& D, uint32_t i) {
+    if (!D.items) return 0u;
+    const uint32_t k = atomicAdd(D.count, 1u);
+    if (k < D.cap) D.items[k] = i;
+    return k;
+}
+
+// One warp runs particle i's walk in a pass after the frame's first lambda pass: over its full
+// list, its long row or, without either, the cells.
+template <class V>
+__device__ __forceinline__ void walk_warp(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
+                                          const float4* __restrict__ p, const uint32_t* __restrict__ cs,
+                                          const uint32_t* __restrict__ ce, const LongLists& LL, const NbList& F, V& vis) {
+    const uint32_t fm = F.list ? F.meta[i] : kListOff;
+    if (!(fm & kListOff)) {
+        walk_row(F.list + i, F.stride, fm & 0xFFu, (fm >> 8) & 0xFFu, i, p, vis);
+        return;
+    }
+    const uint32_t q = fm & ~(kListOff | kListWalked);
+    const uint32_t m = (F.list && q < LL.slots) ? LL.meta[q] : kListOff;
+    if (m != kListOff) walk_row(LL.list + (size_t)q * kLongMax, 1, m & 0xFFFFu, m >> 16, i, p, vis);
+    else walk_coop(P, S, i, anchor, p, cs, ce, vis);
 }
 
 // ======================================================================================
@@ -687,10 +855,11 @@ struct LambdaVisit {
 __global__ void __launch_bounds__(256)
 lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
               const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux,
-              NbList L, NbList F, DeferList DF, DeferList DN) {
+              NbList L, NbList F, DeferList DF, DeferList DN, uint32_t long_slots) {
     // walks the cells; L.list: record the near lists for the delta pass that follows (the
     // particles left without one noted in DN); F.list: store the full lists (the frame's first
-    // lambda pass; the particles left without one noted in DF)
+    // lambda pass; the particles left without one noted in DF and finished by lambda_long_kernel,
+    // which stores the lists of the first long_slots of them)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const SceneCtx S = scene_ctx(P, i);
@@ -711,21 +880,25 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
             walk_seq(P, S, i, pa[i], p, cs, ce, rec, true, &deferred);
             fm = deferred ? kListOff : rec.meta();
         }
+        uint32_t q = 0;
+        if (fm == kListOff) {
+            q = note_particle(DF, i);
+            fm |= q | ((!deferred && q >= long_slots) ? kListWalked : 0u);
+        }
         F.meta[i] = fm;
-        if (fm == kListOff) note_particle(DF, i);
-        const uint32_t lm = (L.list && fm != kListOff) ? filter_list<true>(F, fm, L, i, pi, P.cut2, p) : kListOff;
+        const bool listed = !(fm & kListOff);
+        const uint32_t lm = (L.list && listed) ? filter_list<true>(F, fm, L, i, pi, P.cut2, p) : kListOff;
         if (L.list) {
             L.meta[i] = lm;
             if (lm == kListOff) note_particle(DN, i);
         }
-        if (!deferred) {
-            if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
-            else if (fm != kListOff) walk_list<true>(F, i, fm, p, vis);
-            else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
-            lambda[i] = vis.finish(S.rho0);
-            if (aux) vis.store_aux(aux, P.N, i);
-            return;
-        }
+        if (!listed && !(fm & kListWalked)) return;
+        if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
+        else if (listed) walk_list<true>(F, i, fm, p, vis);
+        else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
+        lambda[i] = vis.finish(S.rho0);
+        if (aux) vis.store_aux(aux, P.N, i);
+        return;
     } else if (L.list) {
         // the walk stores the near list; the sums then run over it when it fits
         Recorder<NullVisit> rec(NullVisit{}, L, F, false, i, pi, P.cut2);
@@ -752,13 +925,14 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
     if (aux) vis.store_aux(aux, P.N, i);
 }
 
-// One warp computes lambda_i over the cells.
+// One warp computes lambda_i.
 __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
-                                            float* __restrict__ lambda, float4* __restrict__ aux, uint32_t i) {
+                                            float* __restrict__ lambda, float4* __restrict__ aux, uint32_t i,
+                                            const LongLists& LL, const NbList& F) {
     const SceneCtx S = scene_ctx(P, i);
     LambdaVisit vis(P, p[i]);
-    walk_coop(P, S, i, pa[i], p, cs, ce, vis);
+    walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) {
         lambda[i] = vis.finish(S.rho0);
         if (aux) vis.store_aux(aux, P.N, i);
@@ -766,9 +940,29 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
 }
 
 __global__ void __launch_bounds__(128)
-lambda_coop_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
+lambda_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
                    const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux) {
-    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i); });
+    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LongLists{}, NbList{}); });
+}
+
+// After lambda_kernel stored the full lists: the particles left without one (the set DF), a warp
+// each.  Stores their long rows and computes their lambda.
+__global__ void __launch_bounds__(128)
+lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
+                   const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList DF, float4* __restrict__ aux,
+                   const __grid_constant__ LongLists LL, const __grid_constant__ NbList F) {
+    const uint32_t n = min(*DF.count, DF.cap);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < n; q += warps) {
+        const uint32_t i = DF.items[q];
+        if (F.meta[i] & kListWalked) continue;
+        if (q < LL.slots) {
+            const uint32_t m = store_row(P, scene_ctx(P, i), i, pa[i], cs, ce, LL.list + (size_t)q * kLongMax);
+            if (lane_id() == 0) LL.meta[q] = m;
+            __syncwarp();
+        }
+        coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F);
+    }
 }
 
 // The frame's later lambda passes: read the full list (no cell tables), record the near list.
@@ -776,17 +970,17 @@ lambda_coop_kernel(DevParams P, const float4* __restrict__ p, const float4* __re
 // without a near list are noted in DN for the delta pass.  Kept apart from lambda_kernel so that
 // its register budget is the list walk's alone.
 __global__ void __launch_bounds__(256, 5)
-lambda_list_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
-                   CoopSet C, DeferList DN, float4* __restrict__ aux, NbList L, NbList F) {
+                   CoopSet C, DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t fm = F.meta[i];
-    if (fm == kListOff) {
+    if (fm & kListOff) {
         if (L.list) {
             L.meta[i] = kListOff;
             note_particle(DN, i);
@@ -942,19 +1136,20 @@ delta_kernel(DevParams P, uint32_t mode, const float4* __restrict__ pin, const f
     delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
-// One warp runs the delta pass for particle i over the cells.
+// One warp runs the delta pass for particle i.
 __device__ __noinline__ void coop_delta(const DevParams& P, uint32_t mode, const float4* __restrict__ pin,
                                            const float4* __restrict__ pa, float4* __restrict__ pout, float4* __restrict__ x,
                                            float4* __restrict__ v, const float* __restrict__ lambda, const float* __restrict__ w,
                                            float4* __restrict__ delta, const uint32_t* __restrict__ cs,
-                                           const uint32_t* __restrict__ ce, uint32_t i) {
+                                           const uint32_t* __restrict__ ce, uint32_t i, const LongLists& LL,
+                                           const NbList& F) {
     const float4 pi = pin[i];
     const bool need_x = (mode & (kDoCollide | kDoUpdate)) != 0;
     const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float li = (mode & kDoDelta) ? lambda[i] : 0.f;
     const SceneCtx S = scene_ctx(P, i);
     DeltaVisit vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
-    walk_coop(P, S, i, pa[i], pin, cs, ce, vis);
+    walk_warp(P, S, i, pa[i], pin, cs, ce, LL, F, vis);
     if (lane_id() == 0) delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
@@ -966,19 +1161,20 @@ __device__ __noinline__ void coop_delta(const DevParams& P, uint32_t mode, const
 // faster than 5), 5 over the full lists of the density-active workload (6 was 15% slower).
 template <uint32_t kMode, uint32_t kB = kNearBatch>
 __global__ void __launch_bounds__(256, kB == kNearBatch ? 6 : 5)
-delta_list_kernel(DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
+delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
                   float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
                   const float* __restrict__ lambda, const float* __restrict__ w, float4* __restrict__ delta,
-                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, CoopSet C, NbList L) {
+                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, CoopSet C, const __grid_constant__ NbList L, const __grid_constant__ NbList F,
+                  const __grid_constant__ LongLists LL) {
     const uint32_t mode = kMode ? kMode : mode_rt;
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i); });
+        run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i, LL, F); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t meta = L.meta[i];
-    if (meta == kListOff) return;
+    if (meta & kListOff) return;
     const float4 pi = pin[i];
     const bool need_x = (mode & (kDoCollide | kDoUpdate)) != 0;
     const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -990,11 +1186,13 @@ delta_list_kernel(DevParams P, uint32_t mode_rt, const float4* __restrict__ pin,
 }
 
 __global__ void __launch_bounds__(128)
-delta_coop_kernel(DevParams P, uint32_t mode, const float4* __restrict__ pin, const float4* __restrict__ pa, float4* __restrict__ pout,
+delta_coop_kernel(const __grid_constant__ DevParams P, uint32_t mode, const float4* __restrict__ pin, const float4* __restrict__ pa, float4* __restrict__ pout,
                   float4* __restrict__ x, float4* __restrict__ v, const float* __restrict__ lambda, const float* __restrict__ w,
                   float4* __restrict__ delta, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                   DeferList D) {
-    for_each_deferred(D, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i); });
+    for_each_deferred(D, [&](uint32_t i) {
+        coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i, LongLists{}, NbList{});
+    });
 }
 
 // updatePositions on its own (Update.h:11-32), when no delta pass can carry it.
@@ -1077,13 +1275,14 @@ omega_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict
     omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
 }
 
-// One warp computes omega_i over the cells.
+// One warp computes omega_i.
 __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                            const float4* __restrict__ v, const uint32_t* __restrict__ cs,
-                                           const uint32_t* __restrict__ ce, float4* __restrict__ omega, uint32_t i) {
+                                           const uint32_t* __restrict__ ce, float4* __restrict__ omega, uint32_t i,
+                                           const LongLists& LL, const NbList& F) {
     const SceneCtx S = scene_ctx(P, i);
     OmegaVisit vis(P, v, p[i], v[i]);
-    walk_coop(P, S, i, pa[i], p, cs, ce, vis);
+    walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
 }
 
@@ -1095,17 +1294,17 @@ __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __rest
 // workload: 6, 5 was 3.8% slower).
 template <bool kNear>
 __global__ void __launch_bounds__(256, kNear ? 5 : 6)
-omega_list_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
+omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
-                  CoopSet C, DeferList DN, NbList L, NbList F) {
+                  CoopSet C, DeferList DN, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i); });
+        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t fm = F.meta[i];
-    if (fm == kListOff) {
+    if (fm & kListOff) {
         if (L.list) {
             L.meta[i] = kListOff;
             note_particle(DN, i);
@@ -1125,10 +1324,10 @@ omega_list_kernel(DevParams P, const float4* __restrict__ p, const float4* __res
 }
 
 __global__ void __launch_bounds__(128)
-omega_coop_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
+omega_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
                   DeferList D) {
-    for_each_deferred(D, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i); });
+    for_each_deferred(D, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LongLists{}, NbList{}); });
 }
 
 // ======================================================================================
@@ -1254,17 +1453,17 @@ vort_visc_kernel(DevParams P, const float4* __restrict__ p, const float4* __rest
     vort_visc_finish(P, i, vis, vis, vout, fext, w);
 }
 
-// One warp runs vorticity + viscosity for particle i over the cells.
+// One warp runs vorticity + viscosity for particle i.
 __device__ __noinline__ void coop_vort_visc(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                                const float4* __restrict__ vin, float4* __restrict__ vout,
                                                const float4* __restrict__ omega, float4* __restrict__ fext,
                                                const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                                                int do_vort, int do_visc, const float* __restrict__ w, uint32_t i,
-                                               float4* __restrict__ vhost) {
+                                               float4* __restrict__ vhost, const LongLists& LL, const NbList& F) {
     const float4 oi = do_vort ? omega[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const SceneCtx S = scene_ctx(P, i);
     VortViscVisit vis(P, vin, omega, p[i], vin[i], oi, do_vort != 0, do_visc != 0);
-    walk_coop(P, S, i, pa[i], p, cs, ce, vis);
+    walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) vort_visc_finish(P, i, vis, vis, vout, fext, w, vhost);
 }
 
@@ -1278,21 +1477,21 @@ __device__ __noinline__ void coop_vort_visc(const DevParams& P, const float4* __
 // entries: 5 blocks per SM, 6 was 36% slower).
 template <bool kNear>
 __global__ void __launch_bounds__(256, kNear ? 6 : 5)
-vort_visc_list_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                       const float4* __restrict__ vin, float4* __restrict__ vout, const float4* __restrict__ omega,
                       float4* __restrict__ fext, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
-                      int do_vort, int do_visc, const float* __restrict__ w, CoopSet C, NbList Lv, NbList Ln,
-                      float4* __restrict__ vhost) {
+                      int do_vort, int do_visc, const float* __restrict__ w, CoopSet C, const __grid_constant__ NbList Lv, const __grid_constant__ NbList Ln,
+                      float4* __restrict__ vhost, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
         run_coop_set(C, [&](uint32_t i) {
-            coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, vhost);
+            coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, vhost, LL, F);
         });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t meta = Lv.meta[i];
-    if (meta == kListOff) return;
+    if (meta & kListOff) return;
     const float4 oi = do_vort ? omega[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t nm = (do_vort && do_visc && Ln.list) ? Ln.meta[i] : kListOff;
     if (nm != kListOff) {
@@ -1309,12 +1508,12 @@ vort_visc_list_kernel(DevParams P, const float4* __restrict__ p, const float4* _
 }
 
 __global__ void __launch_bounds__(128)
-vort_visc_coop_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ vin,
+vort_visc_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ vin,
                       float4* __restrict__ vout, const float4* __restrict__ omega, float4* __restrict__ fext,
                       const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, int do_vort, int do_visc,
                       const float* __restrict__ w, DeferList D) {
     for_each_deferred(D, [&](uint32_t i) {
-        coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, nullptr);
+        coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, nullptr, LongLists{}, NbList{});
     });
 }
 

@@ -70,7 +70,7 @@ constexpr uint32_t kFullSlim = 128;  // the full list's slots when the list cove
 constexpr int kThreadsParticle = 256;
 constexpr int kThreadsNeighbourDefault = 128;
 constexpr int kThreadsCoop = 128;         // 4 warps, one deferred particle per warp
-constexpr uint32_t kCoopBlocks = 16;      // leading blocks of a list pass that walk its particles without a list
+constexpr uint32_t kCoopBlocks = 64;      // leading blocks of a list pass that walk its particles without a list
 
 inline uint32_t div_up(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
@@ -162,6 +162,7 @@ struct pbd_sim {
     uint32_t max_tiles = 0;
     uint32_t *nb_list = nullptr, *nb_meta = nullptr;   // near lists (recorded by lambda / omega)
     uint32_t *fl_list = nullptr, *fl_meta = nullptr;   // full lists (recorded by the frame's first lambda)
+    LongLists ll{};                                    // the lists of the particles without a full list
     uint32_t *defer_items = nullptr, *defer_count = nullptr, *defer_done = nullptr;
     uint32_t defer_cap = 0;
     // particles without a stored list, walked by the leading blocks of the list passes:
@@ -335,39 +336,40 @@ static bool near_lists_on(const pbd_sim* s, const DevParams& P) {
 // delta_staged_kernel for `mode`, as launch_delta_list.
 static void launch_delta_staged(uint32_t N, cudaStream_t st, const DevParams& P, uint32_t mode, const float4* pin,
                                 const float4* pa, float4* pout, float4* x, float4* v, const float* lam, const float* w,
-                                float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C, const NbList& F) {
+                                float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C, const NbList& F,
+                                const LongLists& LL) {
     constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply;
     const uint32_t g = C.blocks + (N + kStageThreads - 1) / kStageThreads;
     if (mode == kFluid)
-        delta_staged_kernel<kFluid><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F);
+        delta_staged_kernel<kFluid><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F, LL);
     else if (mode == (kFluid | kDoUpdate))
-        delta_staged_kernel<kFluid | kDoUpdate><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F);
+        delta_staged_kernel<kFluid | kDoUpdate><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F, LL);
     else
-        delta_staged_kernel<0><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F);
+        delta_staged_kernel<0><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F, LL);
 }
 
 // delta_list_kernel for `mode`: the fluid frame's two pass modes run specialised code.
 static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevParams& P, uint32_t mode,
                               const float4* pin, const float4* pa, float4* pout, float4* x, float4* v, const float* lam,
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
-                              const NbList& L, bool full) {
+                              const NbList& L, bool full, const NbList& F, const LongLists& LL) {
     constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply;
     const uint32_t g = gn + C.blocks;
     if (full) {   // the frame's full list: entries in batches of kListBatch
         if (mode == kFluid)
-            delta_list_kernel<kFluid, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+            delta_list_kernel<kFluid, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
         else if (mode == (kFluid | kDoUpdate))
-            delta_list_kernel<kFluid | kDoUpdate, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+            delta_list_kernel<kFluid | kDoUpdate, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
         else
-            delta_list_kernel<0, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+            delta_list_kernel<0, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
         return;
     }
     if (mode == kFluid)
-        delta_list_kernel<kFluid><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+        delta_list_kernel<kFluid><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
     else if (mode == (kFluid | kDoUpdate))
-        delta_list_kernel<kFluid | kDoUpdate><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+        delta_list_kernel<kFluid | kDoUpdate><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
     else
-        delta_list_kernel<0><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L);
+        delta_list_kernel<0><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
 }
 
 // Record (or run) one frame of Fluid::compute (Fluid.cu:14-97) on `st`.
@@ -492,16 +494,20 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             const NbList Lr = (act & PBD_ACTIVE_COMPUTE_DELTA_POSITIONS) ? L : L0;
             if (lstaged) {
                 lambda_staged_kernel<<<kCoopBlocks + div_up(N, kStageThreads), kStageThreads, 0, st>>>(
-                    P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF, F);
+                    P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF, F, s->ll);
                 nl += 1;
             } else if (use_full && it > 0) {
                 lambda_list_kernel<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
-                                                                    CF, Lr.list ? DN : DX, aux, Lr, F);
+                                                                    CF, Lr.list ? DN : DX, aux, Lr, F, s->ll);
                 nl += 1;
             } else {
                 lambda_kernel<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux, Lr,
-                                                 use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX);
-                lambda_coop_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux);
+                                                 use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots);
+                if (use_full)
+                    lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
+                                                                    DF, aux, s->ll, F);
+                else
+                    lambda_coop_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux);
                 nl += 2;
             }
             PROF_END();
@@ -518,7 +524,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 const int pout = next_p(cur.p);
                 if (by_list) {
                     launch_delta_list(gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists);
+                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists, F, s->ll);
                     nl += 1;
                 } else {
                     delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -591,11 +597,11 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             const int pout = next_p(cur.p);
             if (dstaged) {
                 launch_delta_staged(N, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                    s->delta, s->cell_start, s->cell_end, CF, F);
+                                    s->delta, s->cell_start, s->cell_end, CF, F, s->ll);
                 nl += 1;
             } else if (by_list) {
                 launch_delta_list(gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists);
+                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists, F, s->ll);
                 nl += 1;
             } else {
                 delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -641,10 +647,10 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
         if (use_full) {
             if (Lo.list)
                 omega_list_kernel<true><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end,
-                                                               s->omega, CF, DNo, Lo, F);
+                                                               s->omega, CF, DNo, Lo, F, s->ll);
             else
                 omega_list_kernel<false><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end,
-                                                               s->omega, CF, DNo, Lo, F);
+                                                               s->omega, CF, DNo, Lo, F, s->ll);
             nl += 1;
         } else {
             omega_kernel<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end, s->omega, D, Lo, DNo);
@@ -666,11 +672,11 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             if (Ln.list)
                 vort_visc_list_kernel<true><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega,
                                                                    s->fext, s->cell_start, s->cell_end, vort, visc, wf,
-                                                                   vfull ? CF : CN, Lv, Ln, vh);
+                                                                   vfull ? CF : CN, Lv, Ln, vh, F, s->ll);
             else
                 vort_visc_list_kernel<false><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega,
                                                                    s->fext, s->cell_start, s->cell_end, vort, visc, wf,
-                                                                   vfull ? CF : CN, Lv, Ln, vh);
+                                                                   vfull ? CF : CN, Lv, Ln, vh, F, s->ll);
             v_read = v_read || vh != nullptr;
             nl += 1;
         } else {
@@ -872,6 +878,8 @@ int create_sim(const pbd_params* prm, uint32_t capacity, const std::vector<Scene
     // kFullSlim; longer lists are walked by a warp per particle instead (correct, slower)
     s->fl_slots = ((prm->active & PBD_ACTIVE_FIND_NEIGHBOURS) && prm->kernel_width_neighbours >= 2) ? kFullMax : kFullSlim;
     parts.push_back({(void**)&s->fl_list, (size_t)s->fl_slots * C * 4}); parts.push_back({(void**)&s->fl_meta, C * 4});
+    s->ll.slots = std::min(capacity, kLongSlots);
+    parts.push_back({(void**)&s->ll.list, (size_t)s->ll.slots * kLongMax * 4}); parts.push_back({(void**)&s->ll.meta, (size_t)s->ll.slots * 4});
     if (s->batched) {
         parts.push_back({(void**)&s->d_scenes, (size_t)s->nscenes * sizeof(SceneParams)});
         parts.push_back({(void**)&s->scene_of, C * 4});

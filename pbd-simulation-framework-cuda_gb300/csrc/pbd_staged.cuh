@@ -274,12 +274,12 @@ __host__ __forceinline__ bool staged_supported(const DevParams& P) {
 
 // computeLambda over the staged neighbourhood (the frame's later lambda passes).
 __global__ void __launch_bounds__(kStageThreads, 6)
-lambda_staged_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+lambda_staged_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                      const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
-                     CoopSet C, NbList F) {
+                     CoopSet C, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     __shared__ StageSmem<NoExtra> sm;
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, nullptr, i); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, nullptr, i, LL, F); });
         return;
     }
     const uint32_t i0 = (blockIdx.x - C.blocks) * kStageThreads;
@@ -288,7 +288,7 @@ lambda_staged_kernel(DevParams P, const float4* __restrict__ p, const float4* __
     const uint32_t i = i0 + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t fm = F.meta[i];
-    if (fm == kListOff) return;   // walked by the cooperative blocks
+    if (fm & kListOff) return;   // walked by the cooperative blocks
     const float4 pi = p[i];
     LambdaVisit vis(P, pi);
     if (staged) walk_staged(P, pa[i], own, sm, vis);
@@ -300,14 +300,14 @@ lambda_staged_kernel(DevParams P, const float4* __restrict__ p, const float4* __
 // staged neighbourhood.
 template <uint32_t kMode>
 __global__ void __launch_bounds__(kStageThreads, 6)
-delta_staged_kernel(DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
+delta_staged_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
                     float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
                     const float* __restrict__ lambda, const float* __restrict__ w, float4* __restrict__ delta,
-                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, CoopSet C, NbList F) {
+                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, CoopSet C, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     __shared__ StageSmem<float> sm;
     const uint32_t mode = kMode ? kMode : mode_rt;
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i); });
+        run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i, LL, F); });
         return;
     }
     const uint32_t i0 = (blockIdx.x - C.blocks) * kStageThreads;
@@ -318,7 +318,7 @@ delta_staged_kernel(DevParams P, uint32_t mode_rt, const float4* __restrict__ pi
     const uint32_t i = i0 + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t fm = F.meta[i];
-    if (fm == kListOff) return;   // walked by the cooperative blocks
+    if (fm & kListOff) return;   // walked by the cooperative blocks
     const float4 pi = pin[i];
     const bool need_x = (mode & (kDoCollide | kDoUpdate)) != 0;
     const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);

@@ -207,3 +207,30 @@ def test_readback_arrays_fed_back_in(need_gpu, pbd, scenes):
         va = np.ctypeslib.as_array(rv, shape=(n, 4))
         assert np.array_equal(xa, sb["x"]) and np.array_equal(va, sb["v"])
     a.close(); b.close()
+
+
+@pytest.mark.parametrize("shells,cap", [(1, 512), (2, 20), (2, 100), (2, 512), (2, 513), (2, 1500), (3, 300), (3, 512)])
+def test_long_rows_bit_identical_to_full_walk(need_gpu, pbd, scenes, shells, cap):
+    """16^3 particles around cell 4095 = (15, 15, 15), whose range the cell-end quirk stretches: the
+    particles within the shells of it have long lists, stored by a warp (up to 512 entries; longer
+    ones walk the cells), cut at the cap inside the 27 cells, inside the shells and beyond"""
+    params = scenes.workload_params(pbd, 32, 1995.0, vorticity=0.0005, viscosity=0.00015, max_neighbours=cap)
+    params.lambda_epsilon = 0.0001
+    params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 4.1, 3.5, shells
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(16, 16, 16, seed=21)
+    a = _run(pbd, params, pos, vel, 3)
+    b = _run(pbd, params, pos, vel, 3, full_walk=True)
+    _same(a, b)
+
+
+def test_more_particles_without_a_list_than_rows(need_gpu, pbd, scenes):
+    """a blob of 12,167 particles at spacing 0.35, most of them with more than 128 entries: the rows
+    (8,192) run out and the rest walk the cells"""
+    params = scenes.workload_params(pbd, 32, 1000.0, vorticity=0.0005, viscosity=0.01)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(23, 23, 23, origin=(6.0, 6.0, 6.0), spacing=0.35, jitter=0.02, seed=22)
+    a = _run(pbd, params, pos, vel, 2)
+    b = _run(pbd, params, pos, vel, 2, full_walk=True)
+    _same(a, b)
