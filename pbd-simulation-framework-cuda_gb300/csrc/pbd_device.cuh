@@ -117,25 +117,42 @@ __device__ __forceinline__ float dist2(float rx, float ry, float rz) {
     return __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
 }
 
+// Square root, its reciprocal and the reciprocal as one instruction each.  Without .ftz the compiler
+// wraps every one in the scaling of denormal inputs (~4 instructions); all normal inputs give the
+// same bits either way (checked over all of them), and a denormal squared distance is below every
+// kernel's lower limit (0.0001), scaled or flushed.
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // ---------------------------------------------------------- pair kernels (Density.h) --
-// poly6Viscosity: W = 315 t^3 t^3 / den, t = hp^2 - d^2, for 0.001 < d < hp - 0.001.
+// poly6Viscosity: W = 315 t^3 t^3 / den, t = hp^2 - d^2, for 0.001 < d < hp - 0.001.  Selected, not
+// branched: the lanes of a warp disagree on the range.
 __device__ __forceinline__ float poly6(const DevParams& P, float dist) {
-    if (dist > 0.001f && dist < P.hp_lim) {
-        float t = __fsub_rn(P.hp2, __fmul_rn(dist, dist));
-        float t3 = t * t * t;
-        return (315.0f * t3 * t3) * P.poly_inv_den;
-    }
-    return 0.0f;
+    const float t = __fsub_rn(P.hp2, __fmul_rn(dist, dist));
+    const float t3 = t * t * t;
+    const float w = (315.0f * t3 * t3) * P.poly_inv_den;
+    return (dist > 0.001f && dist < P.hp_lim) ? w : 0.0f;
 }
 
 // Scalar part of spiky: 15 (hs - d)^2 / (pi hs^6) / |r|_4, so that grad = s * r (r = pi - pj,
 // normalised over all four lanes as the float4 normalize of the reference does).
 __device__ __forceinline__ float spiky_scale(const DevParams& P, float dist, float r2w) {
-    if (dist > 0.0001f && (P.hs - dist) > 0.0001f) {
-        float a = P.hs - dist;
-        return 15.0f * (a * a * P.inv_spiky_den) * rsqrtf(r2w);
-    }
-    return 0.0f;
+    const float a = P.hs - dist;
+    const float s = 15.0f * (a * a * P.inv_spiky_den) * rsqrt_fast(r2w);
+    return (dist > 0.0001f && a > 0.0001f) ? s : 0.0f;
 }
 
 // Integer power by repeated multiplication (the reference's pow(float, int)): r = 1, then

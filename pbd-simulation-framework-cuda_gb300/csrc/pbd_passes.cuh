@@ -825,11 +825,11 @@ struct LambdaVisit {
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
         const float r2 = dist2(rx, ry, rz);
-        if (r2 >= P.cut2) return zero();      // every kernel is exactly 0 there
-        const float dist = sqrtf(r2);
+        const float dist = sqrt_fast(r2);
         const float r2w = __fmaf_rn(rw, rw, r2);
         const float s = spiky_scale(P, dist, r2w);
-        return Contrib{poly6(P, dist), __fmul_rn(__fmul_rn(s, s), r2w), s, rx, ry, rz, rw, 1u};
+        // beyond the cut every kernel is exactly 0: add() leaves the sums alone
+        return Contrib{poly6(P, dist), __fmul_rn(__fmul_rn(s, s), r2w), s, rx, ry, rz, rw, r2 >= P.cut2 ? 0u : 1u};
     }
     __device__ __forceinline__ void add(const Contrib& c, bool) {
         if (!c.near) return;
@@ -852,7 +852,7 @@ struct LambdaVisit {
     }
 };
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)   // 5 (48 registers) spills: 622 -> 649 us on the 1M dense frame
 lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
               const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux,
               NbList L, NbList F, DeferList DF, DeferList DN, uint32_t long_slots) {
@@ -1015,10 +1015,18 @@ enum DeltaMode : uint32_t {
     kDoUpdate = 1u << 5,     // v = (p - x)/dt; x = p
 };
 
-struct DeltaVisit {
+// What a delta visitor knows at compile time: kDeltaAny nothing (the mode, the inverse masses, the
+// exponent and far_pairs_zero are looked at for every entry); kDeltaPlain a pass with the density
+// part, the contacts, config.txt's nSCorr = 4, far pairs exactly zero and no inverse masses;
+// kDeltaMass the same with inverse masses.  The arithmetic is the same.
+enum DeltaKnown : uint32_t { kDeltaAny = 0, kDeltaPlain = 1, kDeltaMass = 2 };
+
+template <uint32_t kKnown>
+struct DeltaVisitT {
     // coef * r is the density part, t * (-r) the contact part; add() applies both with explicit
     // FMAs, so every walker (cells, lists, cooperative warp) rounds them the same way
     struct Contrib { float coef, rx, ry, rz, rw, t; uint32_t flags; };   // flags: 1 delta part, 2 contact part
+    static constexpr bool kKnow = kKnown != kDeltaAny;
     const DevParams& P;
     const float* __restrict__ lambda;
     const float* __restrict__ w;       // inverse masses, or null (all 1, the reference)
@@ -1028,10 +1036,10 @@ struct DeltaVisit {
     float ax = 0.f, ay = 0.f, az = 0.f, aw = 0.f;   // sum of (li + lj + sCorr) * grad
     float4 pacc, xacc;                               // positions with the contact corrections added in order
     float4 xi;
-    __device__ DeltaVisit(const DevParams& P_, const float* lam, const float* w_, float4 pi_, float li_, float wi_,
-                          bool dd, bool dc, float4 xi_)
-        : P(P_), lambda(lam), w(w_), pi(pi_), li(li_), wi(wi_), do_delta(dd), do_collide(dc),
-          all_pairs(P_.far_pairs_zero == 0u), pacc(pi_), xacc(xi_), xi(xi_) {}
+    __device__ DeltaVisitT(const DevParams& P_, const float* lam, const float* w_, float4 pi_, float li_, float wi_,
+                           bool dd, bool dc, float4 xi_)
+        : P(P_), lambda(lam), w(w_), pi(pi_), li(li_), wi(wi_), do_delta(kKnow || dd), do_collide(kKnow || dc),
+          all_pairs(!kKnow && P_.far_pairs_zero == 0u), pacc(pi_), xacc(xi_), xi(xi_) {}
     __device__ void reset() { ax = ay = az = aw = 0.f; pacc = pi; xacc = xi; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.flags != 0u; }
@@ -1042,35 +1050,35 @@ struct DeltaVisit {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float;   // lambda_j
     __device__ __forceinline__ float fetch(uint32_t j) const { return do_delta ? __ldg(lambda + j) : 0.f; }
+    __device__ __forceinline__ bool masses() const { return kKnown == kDeltaPlain ? false : (kKnown == kDeltaMass ? true : w != nullptr); }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, float lj, bool contact) const {
-        Contrib c = zero();
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
-        c.rx = rx; c.ry = ry; c.rz = rz; c.rw = rw;
         const float r2 = dist2(rx, ry, rz);
-        if (!all_pairs && r2 >= P.cut2) return c;
-        const float dist = sqrtf(r2);
+        const float dist = sqrt_fast(r2);
+        const bool near = all_pairs || !(r2 >= P.cut2);
+        Contrib c{0.f, rx, ry, rz, rw, 0.f, 0u};
         if (do_delta) {
             const float s = spiky_scale(P, dist, __fmaf_rn(rw, rw, r2));
-            if (s != 0.0f || all_pairs) {
-                const float W = poly6(P, dist);
-                const float sc = __fmul_rn(-P.k_scorr, powi(__fmul_rn(W, P.inv_wq), P.n_scorr));
-                c.coef = __fmul_rn(__fadd_rn(__fadd_rn(li, lj), sc), s);
-                c.flags |= 1u;
-            }
+            const float q = __fmul_rn(poly6(P, dist), P.inv_wq);
+            const float sc = __fmul_rn(-P.k_scorr, kKnow ? ((q * q) * q) * q : powi(q, P.n_scorr));
+            c.coef = __fmul_rn(__fadd_rn(__fadd_rn(li, lj), sc), s);
+            c.flags = (near && (s != 0.0f || all_pairs)) ? 1u : 0u;
         }
         if (contact && do_collide) {
             const float overlap = P.d - dist;
-            // share of the overlap this particle takes: inverseMass1 / (inverseMass1 + inverseMass2)
-            // (Collision.h:223-225, where both are forced to 1); solids have inverse mass 0
-            float share = 0.5f;
-            if (w) {
-                const float wj = __ldg(w + j);
-                share = (wi + wj) > 0.0f ? wi / (wi + wj) : 0.0f;
-            }
-            if (overlap > 0.0f && dist > 0.00001f && share != 0.0f) {
-                // -share * overlap * (1 - stiffness) along -r / |r|
-                c.t = __fmul_rn(__fmul_rn(-share * overlap, 1.0f / dist), P.one_minus_stiffness);
-                c.flags |= 2u;
+            if (near && overlap > 0.0f && dist > 0.00001f) {
+                // share of the overlap this particle takes: inverseMass1 / (inverseMass1 + inverseMass2)
+                // (Collision.h:223-225, where both are forced to 1); solids have inverse mass 0
+                float share = 0.5f;
+                if (masses()) {
+                    const float wj = __ldg(w + j);
+                    share = (wi + wj) > 0.0f ? wi / (wi + wj) : 0.0f;
+                }
+                if (share != 0.0f) {
+                    // -share * overlap * (1 - stiffness) along -r / |r|
+                    c.t = __fmul_rn(__fmul_rn(-share * overlap, rcp_fast(dist)), P.one_minus_stiffness);
+                    c.flags |= 2u;
+                }
             }
         }
         return c;
@@ -1087,8 +1095,10 @@ struct DeltaVisit {
         }
     }
 };
+using DeltaVisit = DeltaVisitT<kDeltaAny>;
 
-__device__ __forceinline__ void delta_finish(const DevParams& P, float rho0, uint32_t mode, uint32_t i, const DeltaVisit& vis,
+template <class V>
+__device__ __forceinline__ void delta_finish(const DevParams& P, float rho0, uint32_t mode, uint32_t i, const V& vis,
                                              float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
                                              float4* __restrict__ delta) {
     // a solid (inverse mass 0) takes no density correction
@@ -1099,7 +1109,7 @@ __device__ __forceinline__ void delta_finish(const DevParams& P, float rho0, uin
     else if (mode & kLoadDelta) dp = delta[i];
     if (mode & kStoreDelta) delta[i] = dp;
     if (mode & kDoApply) {
-        if (vis.w) { dp.x *= vis.wi; dp.y *= vis.wi; dp.z *= vis.wi; dp.w *= vis.wi; }
+        if (vis.masses()) { dp.x *= vis.wi; dp.y *= vis.wi; dp.z *= vis.wi; dp.w *= vis.wi; }
         pn.x -= dp.x; pn.y -= dp.y; pn.z -= dp.z; pn.w -= dp.w;
     }
     if (mode & kDoUpdate) {
@@ -1156,10 +1166,11 @@ __device__ __noinline__ void coop_delta(const DevParams& P, uint32_t mode, const
 // delta pass 0 of an iteration over the near lists its lambda pass recorded (kB = kNearBatch), or
 // any delta pass over the frame's full list when there are no near lists (kB = kListBatch); the
 // particles without one (the set C) walk the cells.  kMode != 0: the pass
-// mode fixed at compile time (the two passes of a fluid frame), kMode = 0: `mode` at run time.
+// mode fixed at compile time (the two passes of a fluid frame), kMode = 0: `mode` at run time; kKnown:
+// what else is fixed (DeltaKnown).
 // Blocks per SM by the list it walks (measured on GB300): 6 over the near lists (fluid_1m: 2%
 // faster than 5), 5 over the full lists of the density-active workload (6 was 15% slower).
-template <uint32_t kMode, uint32_t kB = kNearBatch>
+template <uint32_t kMode, uint32_t kB, uint32_t kKnown>
 __global__ void __launch_bounds__(256, kB == kNearBatch ? 6 : 5)
 delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
                   float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
@@ -1180,7 +1191,7 @@ delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const f
     const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float li = (mode & kDoDelta) ? lambda[i] : 0.f;
     const SceneCtx S = scene_ctx(P, i);
-    DeltaVisit vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
+    DeltaVisitT<kKnown> vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
     walk_list<false, kB>(L, i, meta, pin, vis);
     delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
@@ -1228,14 +1239,11 @@ struct OmegaVisit {
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, const float4& vj, bool) const {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
         const float r2 = dist2(rx, ry, rz);
-        if (r2 >= P.cut2) return zero();
-        const float dist = sqrtf(r2);
-        const float s = spiky_scale(P, dist, __fmaf_rn(rw, rw, r2));
-        if (s == 0.0f) return zero();
+        const float s = spiky_scale(P, sqrt_fast(r2), __fmaf_rn(rw, rw, r2));
         const float wx = vj.x - vi.x, wy = vj.y - vi.y, wz = vj.z - vi.z;
         const float gx = s * rx, gy = s * ry, gz = s * rz;
         return Contrib{__fsub_rn(__fmul_rn(wy, gz), __fmul_rn(wz, gy)), __fsub_rn(__fmul_rn(wz, gx), __fmul_rn(wx, gz)),
-                       __fsub_rn(__fmul_rn(wx, gy), __fmul_rn(wy, gx)), 1u};
+                       __fsub_rn(__fmul_rn(wx, gy), __fmul_rn(wy, gx)), (r2 >= P.cut2 || s == 0.0f) ? 0u : 1u};
     }
     __device__ __forceinline__ void add(const Contrib& c, bool) {
         if (!c.near) return;
@@ -1373,7 +1381,7 @@ struct VortViscVisitT {
         if constexpr ((kTerms & 1u) != 0u) if (vort) {
             const float4 oj = ex.oj;
             const float dx = oj.x - oi.x, dy = oj.y - oi.y, dz = oj.z - oi.z;
-            const float ol = sqrtf(dist2(dx, dy, dz));
+            const float ol = sqrtf(dist2(dx, dy, dz));   // not sqrt_fast: omegas may differ by less than 1e-19
             // the fast division: the divisors (position differences + 1e-8) stay far below 2^126
             c.gx = __fdividef(ol, (pj.x - pi.x) + 0.00000001f);
             c.gy = __fdividef(ol, (pj.y - pi.y) + 0.00000001f);
@@ -1383,13 +1391,11 @@ struct VortViscVisitT {
         if constexpr ((kTerms & 2u) != 0u) if (visc) {
             const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
             const float r2 = dist2(rx, ry, rz);
-            if (r2 >= P.hp2) return c;
-            const float W = poly6(P, sqrtf(r2));
-            if (W == 0.0f) return c;
+            const float W = poly6(P, sqrt_fast(r2));
             const float4 vj = ex.vj;
             c.sx = (vj.x - vi.x) * W; c.sy = (vj.y - vi.y) * W;
             c.sz = (vj.z - vi.z) * W; c.sw = (vj.w - vi.w) * W;
-            c.flags |= 2u;
+            if (!(r2 >= P.hp2) && W != 0.0f) c.flags |= 2u;
         }
         return c;
     }
@@ -1535,7 +1541,7 @@ struct DensityVisit {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
         const float r2 = dist2(rx, ry, rz);
         if (r2 >= P.cut2) return zero();
-        return Contrib{poly6(P, sqrtf(r2)), 1u};
+        return Contrib{poly6(P, sqrt_fast(r2)), 1u};
     }
     __device__ __forceinline__ void add(const Contrib& c, bool) { if (c.near) A = __fadd_rn(A, c.a); }
 };

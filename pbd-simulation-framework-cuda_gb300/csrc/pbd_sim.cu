@@ -348,28 +348,23 @@ static void launch_delta_staged(uint32_t N, cudaStream_t st, const DevParams& P,
         delta_staged_kernel<0><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F, LL);
 }
 
-// delta_list_kernel for `mode`: the fluid frame's two pass modes run specialised code.
+// delta_list_kernel for `mode`: the fluid frame's two pass modes run code specialised on the mode
+// and, with config.txt's nSCorr and far pairs exactly zero, on those (DeltaKnown).
+template <uint32_t kB>
 static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevParams& P, uint32_t mode,
                               const float4* pin, const float4* pa, float4* pout, float4* x, float4* v, const float* lam,
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
-                              const NbList& L, bool full, const NbList& F, const LongLists& LL) {
-    constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply;
-    const uint32_t g = gn + C.blocks;
-    if (full) {   // the frame's full list: entries in batches of kListBatch
-        if (mode == kFluid)
-            delta_list_kernel<kFluid, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
-        else if (mode == (kFluid | kDoUpdate))
-            delta_list_kernel<kFluid | kDoUpdate, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
-        else
-            delta_list_kernel<0, kListBatch><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
-        return;
-    }
+                              const NbList& L, const NbList& F, const LongLists& LL) {
+    constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply, kLast = kFluid | kDoUpdate;
+    const bool known = P.n_scorr == 4 && P.far_pairs_zero != 0u;
+    auto k = delta_list_kernel<0, kB, kDeltaAny>;
     if (mode == kFluid)
-        delta_list_kernel<kFluid><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
-    else if (mode == (kFluid | kDoUpdate))
-        delta_list_kernel<kFluid | kDoUpdate><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
-    else
-        delta_list_kernel<0><<<g, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
+        k = !known ? delta_list_kernel<kFluid, kB, kDeltaAny>
+                   : (w ? delta_list_kernel<kFluid, kB, kDeltaMass> : delta_list_kernel<kFluid, kB, kDeltaPlain>);
+    else if (mode == kLast)
+        k = !known ? delta_list_kernel<kLast, kB, kDeltaAny>
+                   : (w ? delta_list_kernel<kLast, kB, kDeltaMass> : delta_list_kernel<kLast, kB, kDeltaPlain>);
+    k<<<gn + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
 }
 
 // Record (or run) one frame of Fluid::compute (Fluid.cu:14-97) on `st`.
@@ -523,8 +518,9 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 PROF_BEGIN(by_list ? "delta_list" : "delta");
                 const int pout = next_p(cur.p);
                 if (by_list) {
-                    launch_delta_list(gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists, F, s->ll);
+                    (use_lists ? launch_delta_list<kNearBatch> : launch_delta_list<kListBatch>)(
+                        gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
+                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
                     nl += 1;
                 } else {
                     delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -600,8 +596,9 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                                     s->delta, s->cell_start, s->cell_end, CF, F, s->ll);
                 nl += 1;
             } else if (by_list) {
-                launch_delta_list(gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, !use_lists, F, s->ll);
+                (use_lists ? launch_delta_list<kNearBatch> : launch_delta_list<kListBatch>)(
+                    gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
+                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
                 nl += 1;
             } else {
                 delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,

@@ -234,3 +234,21 @@ def test_more_particles_without_a_list_than_rows(need_gpu, pbd, scenes):
     a = _run(pbd, params, pos, vel, 2)
     b = _run(pbd, params, pos, vel, 2, full_walk=True)
     _same(a, b)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("n_scorr,mass", [(4, False), (4, True), (3, False), (0, True)])
+def test_delta_pass_variants_bit_identical_to_full_walk(need_gpu, pbd, scenes, dense, n_scorr, mass):
+    """the delta pass fixes nSCorr = 4 and the absence of inverse masses at compile time where they
+    hold; every variant gives the bits of the pass that looks at them for every entry"""
+    params = scenes.workload_params(pbd, 24, 1995.0 if dense else 1000.0)
+    params.lambda_epsilon = 0.0001 if dense else 0.1
+    params.n_scorr = n_scorr
+    if dense:
+        params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 4.1, 3.5, 2
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(13, 11, 15, seed=23, spacing=0.95)
+    w = np.where(np.arange(len(pos)) % 7 == 0, 0.0, 1.0).astype(np.float32) if mass else None
+    a = _run(pbd, params, pos, vel, 3, inv_mass=w)
+    b = _run(pbd, params, pos, vel, 3, inv_mass=w, full_walk=True)
+    _same(a, b)
