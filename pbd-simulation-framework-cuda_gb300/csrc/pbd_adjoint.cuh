@@ -225,7 +225,7 @@ __device__ __forceinline__ void walk_frame_list(const DevParams& P, const SceneC
                                                 const float4* __restrict__ p, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ ce, const NbList& F, uint32_t fm, V& vis) {
     if (!(fm & kListOff)) {
-        walk_list(F, i, fm, p, vis);
+        walk_full(F, i, fm, p, vis);
     } else {
         bool deferred = false;
         walk_seq(P, S, i, anchor, p, cs, ce, vis, false, &deferred);
@@ -500,7 +500,7 @@ adj_delta_kernel(DevParams P, const float4* __restrict__ p, const float4* __rest
         // the forward's near list of this iteration (the pairs within the cut), else the cells
         const uint32_t meta = Lt.list ? Lt.meta[i] : kListOff;
         bool deferred = false;
-        if (meta != kListOff) walk_list(Lt, i, meta, p, vis);
+        if (meta != kListOff) walk_near<false, 4>(Lt, i, meta, p, vis);
         else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
         // own terms: this thread alone writes slot i (the partners' terms are in scat)
         gp_out[i] = make_float4(gpin.x + vis.gpi.x, gpin.y + vis.gpi.y, gpin.z + vis.gpi.z, 0.f);
@@ -643,7 +643,7 @@ adj_lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __res
                            make_float3(0.f, 0.f, 0.f)};
             const uint32_t meta = Lt.list ? Lt.meta[i] : kListOff;
             bool deferred = false;
-            if (meta != kListOff) walk_list(Lt, i, meta, p, b);
+            if (meta != kListOff) walk_near<false, 4>(Lt, i, meta, p, b);
             else walk_seq(P, S, i, pa[i], p, cs, ce, b, false, &deferred);
             gp_out[i] = make_float4(g.x + b.gpi.x, g.y + b.gpi.y, g.z + b.gpi.z, 0.f);   // this thread alone writes slot i
         } else {

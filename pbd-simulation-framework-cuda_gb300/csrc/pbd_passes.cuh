@@ -17,7 +17,7 @@
 //    to walk_seq.  It takes the particles whose walk meets a cell range longer than
 //    kLongRange -- in practice the range that SortReorder.h:183-184 extends to N (up to M
 //    entries) -- which would otherwise serialise a whole warp behind one thread;
-//  - walk_list: one thread per particle over a stored list;
+//  - walk_full, walk_near: one thread per particle over a stored list;
 //  - walk_row: one warp per particle over a stored list (the long lists, LongLists).
 #pragma once
 #include <type_traits>
@@ -64,7 +64,7 @@ struct DeferList {
     uint32_t cap;
 };
 
-// Stored lists, both in the reference's list order, slot-major.
+// Stored lists, both in the reference's list order.
 //  - The full list: the frame's first lambda pass walks the cells once (the cells come from the
 //    frame's anchors, so the list is fixed for the frame) and stores every entry, up to the cap
 //    M; the later lambda passes, omega and vorticity read it instead of the cell tables.
@@ -76,12 +76,21 @@ struct DeferList {
 // a warp (LongLists), or walks the cells when those are full.
 constexpr uint32_t kListOff = 0x80000000u;   // meta: no list here (a full list's meta: | kListWalked | its set slot)
 constexpr uint32_t kListWalked = 0x40000000u;   // with kListOff: the first lambda pass walked this particle itself
+// The full list holds four entries side by side (entry k of particle i at full_at): a pass that
+// reads every entry takes four indices per load and steps one address per four entries, a third
+// fewer instructions outside the arithmetic than one load per entry.  The near list is slot-major
+// (slot k of particle i at k * stride + i): its readers stop after ~6 entries, its writers run side
+// by side in the slot.
 struct NbList {
-    uint32_t* list;      // kmax x stride entries, slot-major (slot k of particle i at k * stride + i)
+    uint32_t* list;      // near list: kmax x stride; full list: full_slots(kmax) x stride
     uint32_t* meta;      // per particle: count | contacts << 8, or kListOff
     uint32_t stride;
     uint32_t kmax;       // <= 255
 };
+__host__ __device__ __forceinline__ uint32_t full_slots(uint32_t kmax) { return (kmax + 3u) & ~3u; }
+__device__ __forceinline__ uint32_t* full_at(const NbList& F, uint32_t i, uint32_t k) {
+    return F.list + ((size_t)(k >> 2) * F.stride + i) * 4u + (k & 3u);
+}
 // The lists of the particles without a full list (the set DF, slot q of the set at row q): stored
 // once per frame by the warp that finishes their first lambda pass, read by a warp in every pass
 // after it.  Walking the cells again in each pass cost two dependent table loads and a position
@@ -314,12 +323,12 @@ __device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx
     return n > kLongMax ? kListOff : (n | (nc << 16));
 }
 
-// One warp per particle over a stored list (entry k at row[k * st]): lanes evaluate 32 entries at a
+// One warp per particle over a stored list (entry k at entry(k)): lanes evaluate 32 entries at a
 // time, two such groups of position loads in flight, and the contributions that change a sum are
 // added in list order through shuffles, as in walk_coop.
-template <class V>
-__device__ __forceinline__ void walk_row(const uint32_t* row, size_t st, uint32_t n, uint32_t nc, uint32_t i,
-                                         const float4* __restrict__ p, V& vis) {
+template <class E, class V>
+__device__ __forceinline__ void walk_row(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
+                                         V& vis) {
     const uint32_t lane = lane_id();
     auto part = [&](uint32_t k0, uint32_t k1, bool contact) {
         for (uint32_t kb = k0; kb < k1; kb += 64u) {
@@ -329,7 +338,7 @@ __device__ __forceinline__ void walk_row(const uint32_t* row, size_t st, uint32_
 #pragma unroll
             for (uint32_t b = 0; b < 2u; ++b) {
                 const uint32_t k = kb + b * 32u + lane;
-                j[b] = k < k1 ? row[(size_t)k * st] : i;
+                j[b] = k < k1 ? *entry(k) : i;
             }
 #pragma unroll
             for (uint32_t b = 0; b < 2u; ++b) {
@@ -354,10 +363,7 @@ __device__ __forceinline__ void walk_row(const uint32_t* row, size_t st, uint32_
     part(nc, n, false);
 }
 
-// One thread per particle over a stored list (meta not kListOff): the contact entries, then
-// end_contacts, then the rest.  Entries go in batches of B: the batch's position (and extra)
-// loads are all in flight before the first contribution, and the next batch's indices are
-// loaded while this one is summed.
+// One thread per particle over a stored list (meta not kListOff).
 // Every visitor adds its contributions with explicitly rounded operations (__fadd_rn, or
 // __fmaf_rn where a product goes into the sum), which the compiler never contracts, so the sums
 // get the same bits whichever walker (cells, stored list, cooperative warp) and whichever loop
@@ -368,55 +374,90 @@ __device__ __forceinline__ void walk_row(const uint32_t* row, size_t st, uint32_
 // read with the streaming hint (ld.global.cs: evict first): each is read once per pass, and
 // the cache lines they would take are worth more to the neighbour positions gathered next
 // (3% off the frame on fluid_1m).
-// Batch sizes measured on fluid_1m (1M particles, GB300): full lists 4 (2, 3, 6 and 8 were
-// slower), near lists 1 (2, 3 and 8 slower; a deeper software pipeline too).
-constexpr uint32_t kListBatch = 4;   // full lists (~32 entries)
-constexpr uint32_t kNearBatch = 1;   // near lists (~6 entries)
-template <bool kOwn = false, uint32_t B = kListBatch, class V>
-__device__ __forceinline__ void walk_list_part(const NbList& L, uint32_t i, uint32_t k0, uint32_t k1, bool contact,
-                                               const float4* __restrict__ p, V& vis) {
+
+// A visitor with add_if (its contributions have no side effects) is evaluated for every slot of a
+// group and added under a predicate, so the group's arithmetic runs without branches; the others are
+// visited entry by entry.
+template <class V, class = void> struct AddIf : std::false_type {};
+template <class V> struct AddIf<V, std::void_t<decltype(&V::add_if)>> : std::true_type {};
+template <class V, class = void> struct TestsContacts : std::false_type {};
+template <class V> struct TestsContacts<V, std::void_t<decltype(V::kTestsContacts)>> : std::true_type {};
+
+// The full list, a group of four entries at a time: the group's position (and extra) loads are all
+// in flight before the first contribution, and the next group's indices are loaded meanwhile.
+// Slots past the end hold anything: they are replaced by i itself and not added.
+template <bool kOwn = false, class V>
+__device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t meta, const float4* __restrict__ p, V& vis) {
+    const uint32_t n = meta & 0xFFu, nc = (meta >> 8) & 0xFFu;
+    const uint4* e = reinterpret_cast<const uint4*>(F.list) + i;
+    uint4 q = make_uint4(i, i, i, i);
+    if (n) q = kOwn ? *e : __ldcs(e);
+    uint32_t kb = 0;
+    auto group = [&](auto contacts) {
+        const uint32_t j[4] = {q.x, kb + 1u < n ? q.y : i, kb + 2u < n ? q.z : i, kb + 3u < n ? q.w : i};
+        float4 pj[4];
+        typename ExtraOf<V>::type ex[4];
+#pragma unroll
+        for (uint32_t b = 0; b < 4u; ++b) {
+            pj[b] = __ldg(p + j[b]);
+            ex[b] = fetch_extra(vis, j[b]);
+        }
+        e += F.stride;
+        if (kb + 4u < n) q = kOwn ? *e : __ldcs(e);
+#pragma unroll
+        for (uint32_t b = 0; b < 4u; ++b) {
+            const bool live = kb + b < n, contact = decltype(contacts)::value && kb + b < nc;
+            if constexpr (AddIf<V>::value) vis.add_if(live, contrib_of(vis, j[b], pj[b], ex[b], contact));
+            else if (live) vis.add(contrib_of(vis, j[b], pj[b], ex[b], contact), contact);
+        }
+        kb += 4u;
+    };
+    // a visitor that tests contacts (kTestsContacts): first the groups that hold contact entries, then
+    // the others without the test (with two shells 26 of ~125 entries are contacts: 322 -> 275 us)
+    if constexpr (TestsContacts<V>::value) {
+#pragma unroll 1
+        while (kb < nc) group(std::true_type{});
+#pragma unroll 1
+        while (kb < n) group(std::false_type{});
+    } else {
+#pragma unroll 1
+        while (kb < n) group(std::true_type{});
+    }
+    vis.end_contacts(nc);
+}
+
+// A near list (~6 entries), B entries at a time (on fluid_1m 1; 2, 3 and 8 slower), the next
+// entries' indices in flight.
+template <bool kOwn = false, uint32_t B = 1, class V>
+__device__ __forceinline__ void walk_near(const NbList& L, uint32_t i, uint32_t meta, const float4* __restrict__ p, V& vis) {
+    const uint32_t n = meta & 0xFFu, nc = (meta >> 8) & 0xFFu;
     const size_t st = L.stride;
-    const uint32_t* e = L.list + i + (size_t)k0 * st;   // entry k0; each batch moves it by B entries
+    const uint32_t* e = L.list + i;
     uint32_t jn[B];
 #pragma unroll
-    for (uint32_t b = 0; b < B; ++b) {
-        const uint32_t* a = e + b * st;
-        jn[b] = (k0 + b < k1) ? (kOwn ? *a : __ldcs(a)) : i;
-    }
+    for (uint32_t b = 0; b < B; ++b) jn[b] = b < n ? (kOwn ? e[b * st] : __ldcs(e + b * st)) : i;
 #pragma unroll 1
-    for (uint32_t kb = k0; kb < k1; kb += B) {
+    for (uint32_t kb = 0; kb < n; kb += B) {
         uint32_t j[B];
         float4 pj[B];
         typename ExtraOf<V>::type ex[B];
 #pragma unroll
-        for (uint32_t b = 0; b < B; ++b) j[b] = jn[b];
-#pragma unroll
         for (uint32_t b = 0; b < B; ++b) {
+            j[b] = jn[b];
             pj[b] = __ldg(p + j[b]);
             ex[b] = fetch_extra(vis, j[b]);
         }
         e += B * st;
 #pragma unroll
-        for (uint32_t b = 0; b < B; ++b) {
-            const uint32_t* a = e + b * st;
-            jn[b] = (kb + B + b < k1) ? (kOwn ? *a : __ldcs(a)) : i;
-        }
+        for (uint32_t b = 0; b < B; ++b) jn[b] = kb + B + b < n ? (kOwn ? e[b * st] : __ldcs(e + b * st)) : i;
 #pragma unroll
-        for (uint32_t b = 0; b < B; ++b)
-            if (kb + b < k1) vis.add(contrib_of(vis, j[b], pj[b], ex[b], contact), contact);
+        for (uint32_t b = 0; b < B; ++b) {
+            const bool live = B == 1 || kb + b < n, contact = kb + b < nc;
+            if constexpr (AddIf<V>::value) vis.add_if(live, contrib_of(vis, j[b], pj[b], ex[b], contact));
+            else if (live) vis.add(contrib_of(vis, j[b], pj[b], ex[b], contact), contact);
+        }
     }
-}
-template <bool kOwn = false, uint32_t B = kListBatch, class V>
-__device__ __forceinline__ void walk_list(const NbList& L, uint32_t i, uint32_t meta, const float4* __restrict__ p, V& vis) {
-    const uint32_t n = meta & 0xFFu, nc = (meta >> 8) & 0xFFu;
-    walk_list_part<kOwn, B>(L, i, 0u, nc, true, p, vis);
     vis.end_contacts(nc);
-    walk_list_part<kOwn, B>(L, i, nc, n, false, p, vis);
-}
-// A near list (~6 entries): one entry at a time, the next entry's index in flight.
-template <bool kOwn = false, class V>
-__device__ __forceinline__ void walk_near(const NbList& L, uint32_t i, uint32_t meta, const float4* __restrict__ p, V& vis) {
-    walk_list<kOwn, kNearBatch>(L, i, meta, p, vis);
 }
 
 // Particle i's near list from its full list (meta fm): the entries with r^2 < cut2 at p, in
@@ -424,49 +465,34 @@ __device__ __forceinline__ void walk_near(const NbList& L, uint32_t i, uint32_t 
 // list alone (every entry left out adds an exact zero to every sum of a lambda, omega or delta
 // pass), so the warp runs the kernel arithmetic for ~6 entries per particle instead of ~32.
 // Returns the near list's meta (kListOff when it does not fit).
-// kStepped: entry and output addresses stepped by the strides instead of a product per entry
-// (lambda_list_kernel: 7.6% faster on fluid_1m; omega_list_kernel's 40-register budget takes
-// the two extra pointers badly: 8.8% slower there, so it keeps the products).
-template <bool kOwn = false, bool kStepped = false>
+template <bool kOwn = false>
 __device__ __forceinline__ uint32_t filter_list(const NbList& F, uint32_t fm, const NbList& L, uint32_t i,
                                                 const float4& pi, float cut2, const float4* __restrict__ p) {
     const uint32_t n = fm & 0xFFu, nc = (fm >> 8) & 0xFFu;
-    const size_t st = F.stride, ost = L.stride;
-    const uint32_t* e = F.list + i;
+    const uint4* e = reinterpret_cast<const uint4*>(F.list) + i;
     uint32_t* o = L.list + i;
+    const size_t ost = L.stride;
     uint32_t m = 0, mc = 0;
-    uint32_t jn[kListBatch];
-#pragma unroll
-    for (uint32_t b = 0; b < kListBatch; ++b) {
-        const uint32_t* a = e + b * st;
-        jn[b] = (b < n) ? (kOwn ? *a : __ldcs(a)) : i;
-    }
+    uint4 q = make_uint4(i, i, i, i);
+    if (n) q = kOwn ? *e : __ldcs(e);
 #pragma unroll 1
-    for (uint32_t kb = 0; kb < n; kb += kListBatch) {
-        uint32_t j[kListBatch];
-        float4 pj[kListBatch];
+    for (uint32_t kb = 0; kb < n; kb += 4u) {
+        const uint32_t j[4] = {q.x, kb + 1u < n ? q.y : i, kb + 2u < n ? q.z : i, kb + 3u < n ? q.w : i};
+        float4 pj[4];
 #pragma unroll
-        for (uint32_t b = 0; b < kListBatch; ++b) j[b] = jn[b];
+        for (uint32_t b = 0; b < 4u; ++b) pj[b] = __ldg(p + j[b]);
+        e += F.stride;
+        if (kb + 4u < n) q = kOwn ? *e : __ldcs(e);
 #pragma unroll
-        for (uint32_t b = 0; b < kListBatch; ++b) pj[b] = __ldg(p + j[b]);
-        if constexpr (kStepped) e += kListBatch * st;
-#pragma unroll
-        for (uint32_t b = 0; b < kListBatch; ++b) {
-            const uint32_t* a = kStepped ? e + b * st : F.list + i + (size_t)(kb + kListBatch + b) * F.stride;
-            jn[b] = (kb + kListBatch + b < n) ? (kOwn ? *a : __ldcs(a)) : i;
-        }
-#pragma unroll
-        for (uint32_t b = 0; b < kListBatch; ++b) {
+        for (uint32_t b = 0; b < 4u; ++b) {
             if (kb + b == nc) mc = m;
-            if (kb + b < n) {
-                const float rx = pi.x - pj[b].x, ry = pi.y - pj[b].y, rz = pi.z - pj[b].z;
-                if (dist2(rx, ry, rz) < cut2) {
-                    if (m < L.kmax) {
-                        if constexpr (kStepped) { *o = j[b]; o += ost; }
-                        else L.list[(size_t)m * L.stride + i] = j[b];
-                    }
-                    ++m;
+            const float rx = pi.x - pj[b].x, ry = pi.y - pj[b].y, rz = pi.z - pj[b].z;
+            if (kb + b < n && dist2(rx, ry, rz) < cut2) {
+                if (m < L.kmax) {
+                    *o = j[b];
+                    o += ost;
                 }
+                ++m;
             }
         }
     }
@@ -523,26 +549,47 @@ struct Recorder {
 // loads are dead and vanish), the boundary of the contact entries kept.
 struct ListRecorder {
     struct Contrib {};
-    uint32_t* list;
-    uint32_t stride, kmax, i;
+    const NbList& F;
+    uint32_t i;
     uint32_t n = 0, nc = 0xFFFFFFFFu;
-    __device__ ListRecorder(const NbList& F, uint32_t i_) : list(F.list), stride(F.stride), kmax(F.kmax), i(i_) {}
+    __device__ ListRecorder(const NbList& F_, uint32_t i_) : F(F_), i(i_) {}
     __device__ static Contrib zero() { return Contrib{}; }
     __device__ static bool effective(const Contrib&) { return false; }
     __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ void end_contacts(uint32_t) { nc = n; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) {
-        if (n < kmax) list[(size_t)n * stride + i] = j;
+        if (n < F.kmax) *full_at(F, i, n) = j;
         ++n;
         return Contrib{};
     }
     __device__ __forceinline__ void add(const Contrib&, bool) {}
     __device__ __forceinline__ uint32_t meta() const {
         const uint32_t c = nc == 0xFFFFFFFFu ? n : nc;
-        return n > kmax ? kListOff : (n | (c << 8));
+        return n > F.kmax ? kListOff : (n | (c << 8));
     }
 };
 
+// Appends entries to particle i's full list: four collect in registers and go out as one store.
+struct FullWriter {
+    uint4 q = make_uint4(0u, 0u, 0u, 0u);   // the last four entries, the newest in w
+    uint4* o;
+    size_t st;
+    uint32_t n = 0;                          // entries appended
+    __device__ FullWriter(const NbList& F, uint32_t i) : o(reinterpret_cast<uint4*>(F.list) + i), st(F.stride) {}
+    __device__ __forceinline__ void push(uint32_t j) {
+        q.x = q.y; q.y = q.z; q.z = q.w; q.w = j;
+        if ((++n & 3u) == 0u) {
+            *o = q;
+            o += st;
+        }
+    }
+    __device__ __forceinline__ void flush() {   // the last 1 to 3 entries
+        const uint32_t r = n & 3u;
+        if (r == 1u) *o = make_uint4(q.w, 0u, 0u, 0u);
+        if (r == 2u) *o = make_uint4(q.z, q.w, 0u, 0u);
+        if (r == 3u) *o = make_uint4(q.y, q.z, q.w, 0u);
+    }
+};
 
 // The frame's full list of particle i for a 27-cell neighbourhood (kernelWidthNeighbours 1,
 // findContacts on), indices only: the entries, order, cap M, self-skip and long-range hand-over
@@ -562,10 +609,11 @@ __device__ __forceinline__ uint32_t store_full_list(const DevParams& P, const Sc
         my[c] = morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.y)) << 1;
         mz[c] = morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.z));
     }
-    uint32_t* out = F.list + i;
+    FullWriter out(F, i);
     uint32_t n = 0;
+    bool full = false;   // the cap is reached
 #pragma unroll 1
-    for (int col = 0; col < 9; ++col) {
+    for (int col = 0; col < 9 && !full; ++col) {
         const int a = col / 3, b = col - 3 * (col / 3);
         const uint32_t hxy = (a == 0 ? mx[0] : (a == 1 ? mx[1] : mx[2])) + (b == 0 ? my[0] : (b == 1 ? my[1] : my[2]));
         uint32_t h[3], s3[3], e3[3];
@@ -588,25 +636,23 @@ __device__ __forceinline__ uint32_t store_full_list(const DevParams& P, const Sc
         }
         const uint32_t l01 = len[0] + len[1], T = l01 + len[2];
         if (reach < M && reach <= F.kmax) {   // the column fits below the cap and the list's room
-            uint32_t* o = out + (size_t)n * F.stride;
 #pragma unroll 1
             for (uint32_t t = 0; t < T; ++t) {
                 const uint32_t j = t < len[0] ? s3[0] + t : (t < l01 ? s3[1] + (t - len[0]) : s3[2] + (t - l01));
-                if (j == i) continue;
-                *o = j;
-                o += F.stride;
+                if (j != i) out.push(j);
             }
             n = reach;
             continue;
         }
 #pragma unroll 1
-        for (uint32_t t = 0; t < T; ++t) {
+        for (uint32_t t = 0; t < T && !full; ++t) {
             const uint32_t j = t < len[0] ? s3[0] + t : (t < l01 ? s3[1] + (t - len[0]) : s3[2] + (t - l01));
             if (j == i) continue;
-            if (n < F.kmax) out[(size_t)n * F.stride] = j;
-            if (++n == M) return n > F.kmax ? kListOff : (n | (n << 8));
+            if (n < F.kmax) out.push(j);
+            full = ++n == M;
         }
     }
+    out.flush();
     return n > F.kmax ? kListOff : (n | (n << 8));
 }
 
@@ -619,7 +665,7 @@ template <int kMax>
 __device__ __forceinline__ bool store_cell_group(const DevParams& P, const SceneCtx& S, uint32_t i, const uint32_t* h,
                                                  int ncell, const uint32_t* __restrict__ cs,
                                                  const uint32_t* __restrict__ ce, const NbList& F, bool quirk,
-                                                 uint32_t& n, bool* deferred) {
+                                                 FullWriter& out, uint32_t& n, bool* deferred) {
     const uint32_t N = P.N, M = P.M;
     uint32_t s[kMax], e[kMax], len[kMax];
 #pragma unroll
@@ -635,17 +681,13 @@ __device__ __forceinline__ bool store_cell_group(const DevParams& P, const Scene
         if (valid && reach < M && len[c] > kLongRange) { *deferred = true; return true; }
         reach += len[c] - ((valid && s[c] <= i && i < ec) ? 1u : 0u);
     }
-    uint32_t* out = F.list + i;
     if (reach < M && reach <= F.kmax) {   // the group fits below the cap and the list's room
-        uint32_t* o = out + (size_t)n * F.stride;
 #pragma unroll
         for (int c = 0; c < kMax; ++c)
 #pragma unroll 1
             for (uint32_t t = 0; t < len[c]; ++t) {
                 const uint32_t j = s[c] + t;
-                if (j == i) continue;
-                *o = j;
-                o += F.stride;
+                if (j != i) out.push(j);
             }
         n = reach;
         return false;
@@ -656,7 +698,7 @@ __device__ __forceinline__ bool store_cell_group(const DevParams& P, const Scene
         for (uint32_t t = 0; t < len[c]; ++t) {
             const uint32_t j = s[c] + t;
             if (j == i) continue;
-            if (n < F.kmax) out[(size_t)n * F.stride] = j;
+            if (n < F.kmax) out.push(j);
             if (++n == M) return true;
         }
     return false;
@@ -674,8 +716,10 @@ __device__ __forceinline__ uint32_t store_full_list_shells(const DevParams& P, c
     const bool quirk = (P.flags & PBD_FLAG_CELL_END_QUIRK) && S.n >= 2;
     const int K = (int)P.K;
     uint32_t n = 0, nc = 0xFFFFFFFFu;
+    FullWriter out(F, i);
     auto meta = [&]() -> uint32_t {
         const uint32_t c = nc == 0xFFFFFFFFu ? n : nc;
+        out.flush();
         return n > F.kmax ? kListOff : (n | (c << 8));
     };
     uint32_t h[7];
@@ -685,7 +729,7 @@ __device__ __forceinline__ uint32_t store_full_list_shells(const DevParams& P, c
             const uint32_t hxy = hx + (morton_axis(__fmaf_rn((float)b, P.d, pa.y)) << 1);
 #pragma unroll
             for (int c = 0; c < 3; ++c) h[c] = hxy + morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.z));
-            if (store_cell_group<3>(P, S, i, h, 3, cs, ce, F, quirk, n, deferred)) return *deferred ? kListOff : meta();
+            if (store_cell_group<3>(P, S, i, h, 3, cs, ce, F, quirk, out, n, deferred)) return *deferred ? kListOff : meta();
         }
     }
     nc = n;
@@ -701,7 +745,7 @@ __device__ __forceinline__ uint32_t store_full_list_shells(const DevParams& P, c
                     const int c = edge ? t - sh : (t == 0 ? -sh : sh);
                     h[t] = hxy + morton_axis(__fmaf_rn((float)c, P.d, pa.z));
                 }
-                if (store_cell_group<7>(P, S, i, h, m, cs, ce, F, quirk, n, deferred)) return *deferred ? kListOff : meta();
+                if (store_cell_group<7>(P, S, i, h, m, cs, ce, F, quirk, out, n, deferred)) return *deferred ? kListOff : meta();
             }
         }
     return meta();
@@ -794,12 +838,13 @@ __device__ __forceinline__ void walk_warp(const DevParams& P, const SceneCtx& S,
                                           const uint32_t* __restrict__ ce, const LongLists& LL, const NbList& F, V& vis) {
     const uint32_t fm = F.list ? F.meta[i] : kListOff;
     if (!(fm & kListOff)) {
-        walk_row(F.list + i, F.stride, fm & 0xFFu, (fm >> 8) & 0xFFu, i, p, vis);
+        walk_row([&](uint32_t k) { return full_at(F, i, k); }, fm & 0xFFu, (fm >> 8) & 0xFFu, i, p, vis);
         return;
     }
     const uint32_t q = fm & ~(kListOff | kListWalked);
     const uint32_t m = (F.list && q < LL.slots) ? LL.meta[q] : kListOff;
-    if (m != kListOff) walk_row(LL.list + (size_t)q * kLongMax, 1, m & 0xFFFFu, m >> 16, i, p, vis);
+    const uint32_t* row = LL.list + (size_t)q * kLongMax;
+    if (m != kListOff) walk_row([&](uint32_t k) { return row + k; }, m & 0xFFFFu, m >> 16, i, p, vis);
     else walk_coop(P, S, i, anchor, p, cs, ce, vis);
 }
 
@@ -836,6 +881,15 @@ struct LambdaVisit {
         A = __fadd_rn(A, c.a); B = __fadd_rn(B, c.b);
         Cx = __fmaf_rn(c.s, c.rx, Cx); Cy = __fmaf_rn(c.s, c.ry, Cy);
         Cz = __fmaf_rn(c.s, c.rz, Cz); Cw = __fmaf_rn(c.s, c.rw, Cw);
+    }
+    // add() when `live`, as predicated instructions: as a branch the compiler moves the contribution's
+    // arithmetic into it, and the entries of a group run one after the other
+    __device__ __forceinline__ void add_if(bool live, const Contrib& c) {
+        asm("{ .reg .pred q; setp.ne.u32 q, %6, 0; @q add.rn.f32 %0, %0, %7; @q add.rn.f32 %1, %1, %8;"
+            " @q fma.rn.f32 %2, %9, %10, %2; @q fma.rn.f32 %3, %9, %11, %3; @q fma.rn.f32 %4, %9, %12, %4;"
+            " @q fma.rn.f32 %5, %9, %13, %5; }"
+            : "+f"(A), "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz), "+f"(Cw)
+            : "r"((live && c.near) ? 1u : 0u), "f"(c.a), "f"(c.b), "f"(c.s), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
     }
     // the sums the reverse pass needs: aux[i] = (rho, B, S.x, S.y), aux[N + i] = (S.z, S.w, 0, 0)
     __device__ __forceinline__ void store_aux(float4* __restrict__ aux, uint32_t N, uint32_t i) const {
@@ -894,7 +948,7 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         }
         if (!listed && !(fm & kListWalked)) return;
         if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
-        else if (listed) walk_list<true>(F, i, fm, p, vis);
+        else if (listed) walk_full<true>(F, i, fm, p, vis);
         else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
         lambda[i] = vis.finish(S.rho0);
         if (aux) vis.store_aux(aux, P.N, i);
@@ -990,13 +1044,13 @@ lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
     LambdaVisit vis(P, pi);
-    const uint32_t lm = L.list ? filter_list<false, true>(F, fm, L, i, pi, P.cut2, p) : kListOff;
+    const uint32_t lm = L.list ? filter_list(F, fm, L, i, pi, P.cut2, p) : kListOff;
     if (L.list) {
         L.meta[i] = lm;
         if (lm == kListOff) note_particle(DN, i);
     }
     if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
-    else walk_list(F, i, fm, p, vis);
+    else walk_full(F, i, fm, p, vis);
     lambda[i] = vis.finish(S.rho0);
     if (aux) vis.store_aux(aux, P.N, i);
 }
@@ -1027,6 +1081,7 @@ struct DeltaVisitT {
     // FMAs, so every walker (cells, lists, cooperative warp) rounds them the same way
     struct Contrib { float coef, rx, ry, rz, rw, t; uint32_t flags; };   // flags: 1 delta part, 2 contact part
     static constexpr bool kKnow = kKnown != kDeltaAny;
+    static constexpr bool kTestsContacts = true;
     const DevParams& P;
     const float* __restrict__ lambda;
     const float* __restrict__ w;       // inverse masses, or null (all 1, the reference)
@@ -1092,6 +1147,18 @@ struct DeltaVisitT {
             pacc.x = __fmaf_rn(-c.rx, c.t, pacc.x); xacc.x = __fmaf_rn(-c.rx, c.t, xacc.x);
             pacc.y = __fmaf_rn(-c.ry, c.t, pacc.y); xacc.y = __fmaf_rn(-c.ry, c.t, xacc.y);
             pacc.z = __fmaf_rn(-c.rz, c.t, pacc.z); xacc.z = __fmaf_rn(-c.rz, c.t, xacc.z);
+        }
+    }
+    // the density part predicated (LambdaVisit::add_if); contacts are rare enough for a branch
+    __device__ __forceinline__ void add_if(bool live, const Contrib& c) {
+        asm("{ .reg .pred q; setp.ne.u32 q, %4, 0; @q fma.rn.f32 %0, %5, %6, %0; @q fma.rn.f32 %1, %5, %7, %1;"
+            " @q fma.rn.f32 %2, %5, %8, %2; @q fma.rn.f32 %3, %5, %9, %3; }"
+            : "+f"(ax), "+f"(ay), "+f"(az), "+f"(aw)
+            : "r"((live && (c.flags & 1u)) ? 1u : 0u), "f"(c.coef), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
+        if (live && (c.flags & 2u)) {
+            Contrib k = c;
+            k.flags = 2u;
+            add(k, true);
         }
     }
 };
@@ -1163,15 +1230,16 @@ __device__ __noinline__ void coop_delta(const DevParams& P, uint32_t mode, const
     if (lane_id() == 0) delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
-// delta pass 0 of an iteration over the near lists its lambda pass recorded (kB = kNearBatch), or
-// any delta pass over the frame's full list when there are no near lists (kB = kListBatch); the
+// delta pass 0 of an iteration over the near lists its lambda pass recorded (kFull = false), or
+// any delta pass over the frame's full list when there are no near lists (kFull = true); the
 // particles without one (the set C) walk the cells.  kMode != 0: the pass
 // mode fixed at compile time (the two passes of a fluid frame), kMode = 0: `mode` at run time; kKnown:
 // what else is fixed (DeltaKnown).
-// Blocks per SM by the list it walks (measured on GB300): 6 over the near lists (fluid_1m: 2%
-// faster than 5), 5 over the full lists of the density-active workload (6 was 15% slower).
-template <uint32_t kMode, uint32_t kB, uint32_t kKnown>
-__global__ void __launch_bounds__(256, kB == kNearBatch ? 6 : 5)
+// Blocks of 256 per SM by the list it walks (1M particles, GB300): 6 over the near lists (31.3 us;
+// 5 33.2), 4 over the full lists, whose groups of four entries take 64 registers (275 us; 5 360 with
+// spills, 3 282).
+template <uint32_t kMode, bool kFull, uint32_t kKnown>
+__global__ void __launch_bounds__(256, kFull ? 4 : 6)
 delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,
                   float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
                   const float* __restrict__ lambda, const float* __restrict__ w, float4* __restrict__ delta,
@@ -1192,7 +1260,8 @@ delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const f
     const float li = (mode & kDoDelta) ? lambda[i] : 0.f;
     const SceneCtx S = scene_ctx(P, i);
     DeltaVisitT<kKnown> vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
-    walk_list<false, kB>(L, i, meta, pin, vis);
+    if constexpr (kFull) walk_full(L, i, meta, pin, vis);
+    else walk_near(L, i, meta, pin, vis);
     delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
@@ -1249,6 +1318,12 @@ struct OmegaVisit {
         if (!c.near) return;
         ox = __fadd_rn(ox, c.ox); oy = __fadd_rn(oy, c.oy); oz = __fadd_rn(oz, c.oz);
     }
+    __device__ __forceinline__ void add_if(bool live, const Contrib& c) {   // LambdaVisit::add_if
+        asm("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q add.rn.f32 %0, %0, %4; @q add.rn.f32 %1, %1, %5;"
+            " @q add.rn.f32 %2, %2, %6; }"
+            : "+f"(ox), "+f"(oy), "+f"(oz)
+            : "r"((live && c.near) ? 1u : 0u), "f"(c.ox), "f"(c.oy), "f"(c.oz));
+    }
 };
 
 __global__ void __launch_bounds__(256)
@@ -1297,11 +1372,10 @@ __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __rest
 // omega over the full list (recording the near list when L.list, and noting the particles left
 // without one in DN when DN is given); the particles without a full list (the set C) are walked
 // by the leading blocks.
-// kNear: the pass filters the full list into omega's near list (the fluid workloads: 5 blocks
-// per SM, 2.5% faster than 6 on fluid_1m); else it walks the full list (the density-active
-// workload: 6, 5 was 3.8% slower).
+// kNear: the pass filters the full list into omega's near list (5 blocks of 256 per SM: 80 us with 1M
+// particles; 4 and 6 88); else it walks the full list (4: 211 us; 3 219, 5 230).
 template <bool kNear>
-__global__ void __launch_bounds__(256, kNear ? 5 : 6)
+__global__ void __launch_bounds__(256, kNear ? 5 : 4)
 omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
                   CoopSet C, DeferList DN, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
@@ -1327,7 +1401,7 @@ omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict_
         if (lm == kListOff) note_particle(DN, i);
     }
     if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
-    else walk_list<false, 2>(F, i, fm, p, vis);
+    else walk_full(F, i, fm, p, vis);
     omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
 }
 
@@ -1402,6 +1476,18 @@ struct VortViscVisitT {
     __device__ __forceinline__ void add(const Contrib& c, bool) {
         if (c.flags & 1u) { gx = __fadd_rn(gx, c.gx); gy = __fadd_rn(gy, c.gy); gz = __fadd_rn(gz, c.gz); }
         if (c.flags & 2u) { sx = __fadd_rn(sx, c.sx); sy = __fadd_rn(sy, c.sy); sz = __fadd_rn(sz, c.sz); sw = __fadd_rn(sw, c.sw); }
+    }
+    __device__ __forceinline__ void add_if(bool live, const Contrib& c) {   // LambdaVisit::add_if
+        if constexpr ((kTerms & 1u) != 0u)
+            asm("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q add.rn.f32 %0, %0, %4; @q add.rn.f32 %1, %1, %5;"
+                " @q add.rn.f32 %2, %2, %6; }"
+                : "+f"(gx), "+f"(gy), "+f"(gz)
+                : "r"((live && (c.flags & 1u)) ? 1u : 0u), "f"(c.gx), "f"(c.gy), "f"(c.gz));
+        if constexpr ((kTerms & 2u) != 0u)
+            asm("{ .reg .pred q; setp.ne.u32 q, %4, 0; @q add.rn.f32 %0, %0, %5; @q add.rn.f32 %1, %1, %6;"
+                " @q add.rn.f32 %2, %2, %7; @q add.rn.f32 %3, %3, %8; }"
+                : "+f"(sx), "+f"(sy), "+f"(sz), "+f"(sw)
+                : "r"((live && (c.flags & 2u)) ? 1u : 0u), "f"(c.sx), "f"(c.sy), "f"(c.sz), "f"(c.sw));
     }
 };
 
@@ -1478,11 +1564,11 @@ __device__ __noinline__ void coop_vort_visc(const DevParams& P, const float4* __
 // terms and the omega pass's near list Ln at hand, vorticity runs over the full list and
 // viscosity over the near list (its entries beyond the cut add exact zeros): the two sums keep
 // their own order.
-// kNear: viscosity over omega's near list (the fluid workloads: 6 blocks per SM, 6.6% faster
-// than 5 on fluid_1m); else both terms over the full list (the density-active workload's ~125
-// entries: 5 blocks per SM, 6 was 36% slower).
-template <bool kNear>
-__global__ void __launch_bounds__(256, kNear ? 6 : 5)
+// Blocks of 256 per SM: with viscosity over omega's near list 4 (113 us with 1M particles; 3 119, 5 141);
+// both terms over the full list's groups 3 (80 registers: 367 us; 2 400, 4 536 with spills).
+enum VortViscLists : uint32_t { kVortViscFull, kVortVisc, kViscNear };   // Lv, Ln: full, none; full, near; near, none
+template <uint32_t kLists>
+__global__ void __launch_bounds__(256, kLists == kVortViscFull ? 3 : 4)
 vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                       const float4* __restrict__ vin, float4* __restrict__ vout, const float4* __restrict__ omega,
                       float4* __restrict__ fext, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
@@ -1502,14 +1588,15 @@ vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restr
     const uint32_t nm = (do_vort && do_visc && Ln.list) ? Ln.meta[i] : kListOff;
     if (nm != kListOff) {
         VortViscVisitT<1u> vo(P, vin, omega, p[i], vin[i], oi, true, false);
-        walk_list<false, 2>(Lv, i, meta, p, vo);   // position + omega per entry: batches of 2 fit the registers
+        walk_full(Lv, i, meta, p, vo);
         VortViscVisitT<2u> vs(P, vin, omega, p[i], vin[i], oi, false, true);
         walk_near(Ln, i, nm, p, vs);
         vort_visc_finish(P, i, vo, vs, vout, fext, w, vhost);
         return;
     }
     VortViscVisit vis(P, vin, omega, p[i], vin[i], oi, do_vort != 0, do_visc != 0);
-    walk_list<false, 2>(Lv, i, meta, p, vis);
+    if constexpr (kLists == kVortVisc || kLists == kVortViscFull) walk_full(Lv, i, meta, p, vis);
+    else walk_near<false, 2>(Lv, i, meta, p, vis);
     vort_visc_finish(P, i, vis, vis, vout, fext, w, vhost);
 }
 

@@ -350,20 +350,20 @@ static void launch_delta_staged(uint32_t N, cudaStream_t st, const DevParams& P,
 
 // delta_list_kernel for `mode`: the fluid frame's two pass modes run code specialised on the mode
 // and, with config.txt's nSCorr and far pairs exactly zero, on those (DeltaKnown).
-template <uint32_t kB>
+template <bool kFull>
 static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevParams& P, uint32_t mode,
                               const float4* pin, const float4* pa, float4* pout, float4* x, float4* v, const float* lam,
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
                               const NbList& L, const NbList& F, const LongLists& LL) {
     constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply, kLast = kFluid | kDoUpdate;
     const bool known = P.n_scorr == 4 && P.far_pairs_zero != 0u;
-    auto k = delta_list_kernel<0, kB, kDeltaAny>;
+    auto k = delta_list_kernel<0, kFull, kDeltaAny>;
     if (mode == kFluid)
-        k = !known ? delta_list_kernel<kFluid, kB, kDeltaAny>
-                   : (w ? delta_list_kernel<kFluid, kB, kDeltaMass> : delta_list_kernel<kFluid, kB, kDeltaPlain>);
+        k = !known ? delta_list_kernel<kFluid, kFull, kDeltaAny>
+                   : (w ? delta_list_kernel<kFluid, kFull, kDeltaMass> : delta_list_kernel<kFluid, kFull, kDeltaPlain>);
     else if (mode == kLast)
-        k = !known ? delta_list_kernel<kLast, kB, kDeltaAny>
-                   : (w ? delta_list_kernel<kLast, kB, kDeltaMass> : delta_list_kernel<kLast, kB, kDeltaPlain>);
+        k = !known ? delta_list_kernel<kLast, kFull, kDeltaAny>
+                   : (w ? delta_list_kernel<kLast, kFull, kDeltaMass> : delta_list_kernel<kLast, kFull, kDeltaPlain>);
     k<<<gn + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
 }
 
@@ -518,7 +518,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 PROF_BEGIN(by_list ? "delta_list" : "delta");
                 const int pout = next_p(cur.p);
                 if (by_list) {
-                    (use_lists ? launch_delta_list<kNearBatch> : launch_delta_list<kListBatch>)(
+                    (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                         gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
                                       s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
                     nl += 1;
@@ -596,7 +596,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                                     s->delta, s->cell_start, s->cell_end, CF, F, s->ll);
                 nl += 1;
             } else if (by_list) {
-                (use_lists ? launch_delta_list<kNearBatch> : launch_delta_list<kListBatch>)(
+                (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                     gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
                                   s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
                 nl += 1;
@@ -666,14 +666,11 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
         PROF_BEGIN(Lv.list ? "vort_visc_list" : "vort_visc");
         if (Lv.list) {
             float4* const vh = (readback && visc) ? s->rb_dev + s->cap : nullptr;
-            if (Ln.list)
-                vort_visc_list_kernel<true><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega,
-                                                                   s->fext, s->cell_start, s->cell_end, vort, visc, wf,
-                                                                   vfull ? CF : CN, Lv, Ln, vh, F, s->ll);
-            else
-                vort_visc_list_kernel<false><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega,
-                                                                   s->fext, s->cell_start, s->cell_end, vort, visc, wf,
-                                                                   vfull ? CF : CN, Lv, Ln, vh, F, s->ll);
+            auto k = Ln.list ? vort_visc_list_kernel<kVortVisc>
+                             : (vfull ? vort_visc_list_kernel<kVortViscFull> : vort_visc_list_kernel<kViscNear>);
+            k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
+                                               s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, Ln, vh,
+                                               F, s->ll);
             v_read = v_read || vh != nullptr;
             nl += 1;
         } else {
@@ -874,7 +871,7 @@ int create_sim(const pbd_params* prm, uint32_t capacity, const std::vector<Scene
     // full-list slots: kFullMax when the parameters reach beyond the 27 cells (shells), else
     // kFullSlim; longer lists are walked by a warp per particle instead (correct, slower)
     s->fl_slots = ((prm->active & PBD_ACTIVE_FIND_NEIGHBOURS) && prm->kernel_width_neighbours >= 2) ? kFullMax : kFullSlim;
-    parts.push_back({(void**)&s->fl_list, (size_t)s->fl_slots * C * 4}); parts.push_back({(void**)&s->fl_meta, C * 4});
+    parts.push_back({(void**)&s->fl_list, (size_t)full_slots(s->fl_slots) * C * 4}); parts.push_back({(void**)&s->fl_meta, C * 4});
     s->ll.slots = std::min(capacity, kLongSlots);
     parts.push_back({(void**)&s->ll.list, (size_t)s->ll.slots * kLongMax * 4}); parts.push_back({(void**)&s->ll.meta, (size_t)s->ll.slots * 4});
     if (s->batched) {
@@ -1636,7 +1633,7 @@ int pbd_adjoint_forward(pbd_sim* s, int nsteps, int ckpt_every, void* stream) {
     const uint32_t S = s->prm.stabilization_iterations;
     const bool stab_tape = s->prm.collision_type == 0 && S > 1;   // contact passes after the first
     const size_t per_tape = N * (16 + 16 + 4 + 4 + ((visc || vort) ? 32 : 0) + (solids ? 4 : 0) + (vort ? 48 : 0)) +
-                            (tape_full ? N * (4 * (size_t)s->fl_slots + 4) : 0) +
+                            (tape_full ? N * (4 * (size_t)full_slots(s->fl_slots) + 4) : 0) +
                             (size_t)I * N * (16 + 4 + 32 + 4 * kListMax + 4) +
                             (stab_tape ? (size_t)I * (S - 1) * (N * 16 + 256) : 0) + 2048;
     const size_t acc_bytes = 16 * (size_t)div_up((uint32_t)N, 128);   // two doubles per reverse block
@@ -1688,7 +1685,7 @@ int pbd_adjoint_forward(pbd_sim* s, int nsteps, int ckpt_every, void* stream) {
         T.w = solids ? (float*)take(N * 4) : nullptr;
         T.omega = vort ? (float4*)take(N * 16) : nullptr;
         T.eta = vort ? (float4*)take(N * 16) : nullptr;
-        T.full = tape_full ? (uint32_t*)take(N * 4 * (size_t)s->fl_slots) : nullptr;
+        T.full = tape_full ? (uint32_t*)take(N * 4 * (size_t)full_slots(s->fl_slots)) : nullptr;
         T.full_meta = tape_full ? (uint32_t*)take(N * 4) : nullptr;
         T.fext = vort ? (float4*)take(N * 16) : nullptr;
     }

@@ -292,7 +292,7 @@ lambda_staged_kernel(const __grid_constant__ DevParams P, const float4* __restri
     const float4 pi = p[i];
     LambdaVisit vis(P, pi);
     if (staged) walk_staged(P, pa[i], own, sm, vis);
-    else walk_list(F, i, fm, p, vis);
+    else walk_full(F, i, fm, p, vis);
     lambda[i] = vis.finish(P.rho0);
 }
 
@@ -325,7 +325,7 @@ delta_staged_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const
     const float li = dd ? lambda[i] : 0.f;
     DeltaVisit vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, dd, (mode & kDoCollide) != 0, xi);
     if (staged) walk_staged(P, pa[i], own, sm, vis);
-    else walk_list<false, kListBatch>(F, i, fm, pin, vis);
+    else walk_full(F, i, fm, pin, vis);
     delta_finish(P, P.rho0, mode, i, vis, pout, x, v, delta);
 }
 
