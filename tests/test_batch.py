@@ -75,3 +75,34 @@ def test_batch_add_between_frames_and_autotune(need_gpu, pbd, scenes, tmp_path):
         b.step(3)
         b.sync()
         assert all(np.all(np.isfinite(b.state(k)["x"])) for k in range(len(sl)))
+
+
+def test_batch_state_with_interleaved_adds(need_gpu, pbd, scenes):
+    """a scene's state is its sorted run followed by what was added since: adds in turns, before the
+    first frame and after it, in the order they came"""
+    shared = _shared(pbd, scenes)
+    sl = _scene_list(scenes)
+    descs = [pbd.scene_desc(len(sc["pos"]), sc["rho"], sc["g"], sc["box"]) for sc in sl]
+    half = [len(sc["pos"]) // 2 for sc in sl]
+    with pbd.Batch(shared, descs) as b:
+        for k in (2, 0, 3):
+            b.add_particles(k, sl[k]["pos"][:half[k]], sl[k]["vel"][:half[k]])
+        b.add_particles(2, sl[2]["pos"][half[2]:-3], sl[2]["vel"][half[2]:-3])
+        assert len(b.state(1)["x"]) == 0
+        assert np.array_equal(b.state(2)["x"], sl[2]["pos"][:-3]) and np.array_equal(b.state(2)["v"], sl[2]["vel"][:-3])
+        assert np.array_equal(b.state(3)["x"], sl[3]["pos"][:half[3]])
+        b.step(2)
+        b.sync()
+        before = [b.state(k) for k in range(len(sl))]
+        b.add_particles(1, sl[1]["pos"], sl[1]["vel"])
+        b.add_particles(0, sl[0]["pos"][half[0]:], sl[0]["vel"][half[0]:])
+        after = [b.state(k) for k in range(len(sl))]
+    for k, tail in enumerate((sl[0]["pos"][half[0]:], sl[1]["pos"], sl[2]["pos"][:0], sl[3]["pos"][:0])):
+        assert np.array_equal(after[k]["x"], np.concatenate([before[k]["x"], tail])), k
+    for k, n in ((0, half[0]), (2, len(sl[2]["pos"]) - 3), (3, half[3])):
+        with pbd.Sim(_single(pbd, shared, sl[k]), n) as s:
+            s.add_particles(sl[k]["pos"][:n], sl[k]["vel"][:n])
+            s.step(2)
+            s.sync()
+            ref = s.state()
+        assert np.array_equal(before[k]["x"], ref["x"]) and np.array_equal(before[k]["v"], ref["v"]), k
