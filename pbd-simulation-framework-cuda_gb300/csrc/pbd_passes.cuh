@@ -18,7 +18,8 @@
 //    kLongRange -- in practice the range that SortReorder.h:183-184 extends to N (up to M
 //    entries) -- which would otherwise serialise a whole warp behind one thread;
 //  - walk_full, walk_near: one thread per particle over a stored list;
-//  - walk_row: one warp per particle over a stored list (the long lists, LongLists).
+//  - walk_group: G lanes per particle over a stored list (the long lists, LongLists, with a warp; small
+//    simulations with fewer lanes).
 #pragma once
 #include <type_traits>
 #include "pbd_device.cuh"
@@ -50,6 +51,9 @@ constexpr uint32_t kLongRange = 32;
 constexpr uint32_t kFullMask = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
+// a value of lane k of the caller's group of `width` lanes
+__device__ __forceinline__ float shfl_f(float v, int k, int width) { return __shfl_sync(kFullMask, v, k, width); }
+__device__ __forceinline__ uint32_t shfl_u(uint32_t v, int k, int width) { return __shfl_sync(kFullMask, v, k, width); }
 __device__ __forceinline__ uint32_t lanemask_lt_u() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -253,19 +257,29 @@ __device__ __forceinline__ void shell_cell(int sh, int t, int& a, int& b, int& c
     c = t - 2 * (side - 2) - sh;
 }
 
-// One warp stores particle i's list (the entries and order of for_each_range, without i, up to the
-// cap M) into `row`: a lane per cell for the table loads, then a lane per entry, which finds its
-// cell by a search over the lanes' offsets.  Returns the row's meta.
-__device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
-                                              const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
-                                              uint32_t* row) {
-    const uint32_t lane = lane_id();
-    const uint32_t cap = min(P.M, kLongMax + 1u);   // one past the row's room: too long
+// G lanes enumerate particle i's list (the entries and order of for_each_range, without i, up to
+// `cap`, the list cap M or one past the room of whatever takes the entries): a lane per cell for
+// the table loads, then a lane per entry, which finds its cell by a search over the group's
+// offsets.  emit(k, j) gets every entry once.  long_stop: a cell range longer than kLongRange ends the
+// walk (walk_seq's hand-over).  Every lane of the warp calls it; groups with on = false only take
+// part in the shuffles.
+struct GroupList {
+    uint32_t n, nc;      // entries, contact entries
+    bool handed_over;
+};
+template <int G, class Emit>
+__device__ __forceinline__ GroupList enumerate_group(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor, bool on,
+                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                                                     uint32_t cap, bool long_stop, Emit&& emit) {
+    const uint32_t lane = lane_id(), t = lane & (uint32_t)(G - 1);
+    const uint32_t shift = lane & ~(uint32_t)(G - 1), gmask = G == 32 ? kFullMask : (1u << G) - 1u;
     const bool quirk = (P.flags & PBD_FLAG_CELL_END_QUIRK) && S.n >= 2;
-    uint32_t n = 0, nc = 0;
+    GroupList R{0u, 0u, false};
+    bool done = !on || cap == 0u;
     auto cells = [&](bool in, int a, int b, int c) {
         uint32_t s = 0, len = 0, own = 0;
-        if (in) {
+        bool is_long = false;
+        if (in && !done) {
             const uint32_t h = (morton_axis(__fmaf_rn((float)a, P.d, anchor.x)) << 2) +
                                (morton_axis(__fmaf_rn((float)b, P.d, anchor.y)) << 1) +
                                morton_axis(__fmaf_rn((float)c, P.d, anchor.z));
@@ -275,6 +289,7 @@ __device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx
                 if (s < P.N) {
                     if ((quirk && h == S.n - 1) || e > S.end) e = S.end;
                     if (e > s) {
+                        is_long = e - s > kLongRange;
                         own = (s <= i && i < e) ? 1u : 0u;
                         len = min(e - s - own, cap);
                     }
@@ -283,84 +298,215 @@ __device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx
         }
         uint32_t off = len;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFullMask, off, o);
-            if (lane >= (uint32_t)o) off += v;
+        for (int o = 1; o < G; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFullMask, off, o, G);
+            if (t >= (uint32_t)o) off += v;
         }
-        const uint32_t total = __shfl_sync(kFullMask, off, 31);
+        const uint32_t total = __shfl_sync(kFullMask, off, G - 1, G);
         off -= len;
-        for (uint32_t o0 = 0; o0 < total && n + o0 < cap; o0 += 32u) {
-            const uint32_t o = o0 + lane;
+        if (long_stop) {
+            const uint32_t bad = __ballot_sync(kFullMask, is_long && R.n + off < cap);
+            if ((bad >> shift) & gmask) { R.handed_over = true; done = true; }
+        }
+        const uint32_t mine = done ? 0u : total;
+        for (uint32_t o0 = 0; __any_sync(kFullMask, o0 < mine && R.n + o0 < cap); o0 += (uint32_t)G) {
+            const uint32_t o = o0 + t;
             uint32_t q = 0;   // the last lane whose offset is not beyond o
 #pragma unroll
-            for (uint32_t step = 16; step > 0; step >>= 1) {
-                const uint32_t v = __shfl_sync(kFullMask, off, q + step);
+            for (uint32_t step = G / 2; step > 0; step >>= 1) {
+                const uint32_t v = __shfl_sync(kFullMask, off, q + step, G);
                 if (v <= o) q += step;
             }
-            const uint32_t qs = __shfl_sync(kFullMask, s, q), qo = __shfl_sync(kFullMask, off, q);
-            const uint32_t qi = __shfl_sync(kFullMask, own, q);
+            const uint32_t qs = __shfl_sync(kFullMask, s, q, G), qo = __shfl_sync(kFullMask, off, q, G);
+            const uint32_t qi = __shfl_sync(kFullMask, own, q, G);
             uint32_t j = qs + (o - qo);
             if (qi && j >= i) ++j;
-            if (o < total && n + o < P.M && n + o < kLongMax) row[n + o] = j;
+            if (o < mine && R.n + o < cap) emit(R.n + o, j);
         }
-        n = min(n + total, cap);
+        R.n = min(R.n + mine, cap);
+        done = done || R.n == cap;
     };
     if (P.active & PBD_ACTIVE_FIND_CONTACTS) {
-        const int t = (int)lane;
-        cells(t < 27, t / 9 - 1, (t / 3) % 3 - 1, t % 3 - 1);
-        nc = n;
+#pragma unroll 1
+        for (int t0 = 0; t0 < 27; t0 += G) {
+            const int k = t0 + (int)t;
+            cells(k < 27, k / 9 - 1, (k / 3) % 3 - 1, k % 3 - 1);
+        }
+        R.nc = R.n;
     }
     if (P.active & PBD_ACTIVE_FIND_NEIGHBOURS)
-        for (int sh = 2; sh <= (int)P.K && n < cap; ++sh) {
+        for (int sh = 2; sh <= (int)P.K; ++sh) {
             const int side = 2 * sh + 1, count = side * side * side - (side - 2) * (side - 2) * (side - 2);
-            for (int t0 = 0; t0 < count && n < cap; t0 += 32) {
-                const int t = t0 + (int)lane;
+            for (int t0 = 0; t0 < count && !__all_sync(kFullMask, done); t0 += G) {
+                const int k = t0 + (int)t;
                 int a = 0, b = 0, c = 0;
-                if (t < count) shell_cell(sh, t, a, b, c);
-                cells(t < count, a, b, c);
+                if (k < count) shell_cell(sh, k, a, b, c);
+                cells(k < count, a, b, c);
             }
         }
-    return n > kLongMax ? kListOff : (n | (nc << 16));
+    return R;
 }
 
-// One warp per particle over a stored list (entry k at entry(k)): lanes evaluate 32 entries at a
-// time, two such groups of position loads in flight, and the contributions that change a sum are
-// added in list order through shuffles, as in walk_coop.
-template <class E, class V>
-__device__ __forceinline__ void walk_row(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
-                                         V& vis) {
-    const uint32_t lane = lane_id();
-    auto part = [&](uint32_t k0, uint32_t k1, bool contact) {
-        for (uint32_t kb = k0; kb < k1; kb += 64u) {
-            uint32_t j[2];
-            float4 pj[2];
-            typename ExtraOf<V>::type ex[2];
+// One warp stores particle i's list into `row` (kLongMax entries at most).  Returns the row's meta.
+__device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
+                                              const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                                              uint32_t* row) {
+    const GroupList R = enumerate_group<32>(P, S, i, anchor, true, cs, ce, min(P.M, kLongMax + 1u), false,
+                                            [&](uint32_t k, uint32_t j) { if (k < kLongMax) row[k] = j; });
+    return R.n > kLongMax ? kListOff : (R.n | (R.nc << 16));
+}
+
+// G lanes per particle over a stored list (entry k at entry(k); n and nc the same in all lanes of a
+// group): each lane evaluates every G-th entry, two position loads in flight and the next indices
+// loaded meanwhile, and the contributions that change a sum are added in list order through
+// shuffles, as in walk_coop, so every lane of the group ends with the sums.  Every lane of the warp
+// calls it.
+template <int G, class E, class V>
+__device__ __forceinline__ void walk_group(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
+                                           V& vis) {
+    const uint32_t t = lane_id() & (uint32_t)(G - 1);
+    constexpr uint32_t kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
+    uint32_t jn[2];
 #pragma unroll
-            for (uint32_t b = 0; b < 2u; ++b) {
-                const uint32_t k = kb + b * 32u + lane;
-                j[b] = k < k1 ? *entry(k) : i;
-            }
+    for (uint32_t b = 0; b < 2u; ++b) jn[b] = b * G + t < n ? *entry(b * G + t) : i;
+    for (uint32_t kb = 0; __any_sync(kFullMask, kb < n); kb += 2u * G) {
+        uint32_t j[2];
+        float4 pj[2];
+        typename ExtraOf<V>::type ex[2];
 #pragma unroll
-            for (uint32_t b = 0; b < 2u; ++b) {
-                pj[b] = __ldg(p + j[b]);
-                ex[b] = fetch_extra(vis, j[b]);
-            }
+        for (uint32_t b = 0; b < 2u; ++b) {
+            j[b] = jn[b];
+            pj[b] = __ldg(p + j[b]);
+            ex[b] = fetch_extra(vis, j[b]);
+        }
 #pragma unroll
-            for (uint32_t b = 0; b < 2u; ++b) {
-                const bool valid = kb + b * 32u + lane < k1;
-                const typename V::Contrib c = valid ? contrib_of(vis, j[b], pj[b], ex[b], contact) : V::zero();
-                uint32_t take = __ballot_sync(kFullMask, valid && V::effective(c));
-                while (take) {
-                    const int k = __ffs(take) - 1;
-                    take &= take - 1u;
-                    vis.add(V::shfl(c, k), contact);
-                }
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = kb + (2u + b) * G + t;
+            jn[b] = k < n ? *entry(k) : i;
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = kb + b * G + t;
+            const typename V::Contrib c = k < n ? contrib_of(vis, j[b], pj[b], ex[b], k < nc) : V::zero();
+            uint32_t take = __ballot_sync(kFullMask, k < n && V::effective(c));
+#pragma unroll
+            for (int o = G; o < 32; o <<= 1) take |= take >> o;   // the entries any group of the warp adds
+            take &= kGroup;
+            while (take) {
+                const int q = __ffs(take) - 1;
+                take &= take - 1u;
+                vis.add(V::shfl(c, q, G), true);   // a contribution without effect leaves the sums alone
             }
         }
-    };
-    part(0u, nc, true);
+    }
     vis.end_contacts(nc);
-    part(nc, n, false);
+}
+
+// walk_group with the sums split over the group's lanes, for a pass whose main walk it is.  Every sum
+// of a visitor is a chain acc = fma(mul, val, acc) over the entries (mul = 1 where a contribution is
+// added as it is: the same rounding as an addition).  Each lane puts its entry's numbers (V::rows,
+// zeros where the entry has no effect, which leave a chain alone) into shared memory, a row per
+// number, and lane t of the group runs the chain of sum t (t + G, ...) over them: two loads and four
+// fused multiply-adds for four entries, where handing a contribution to every lane took seven
+// shuffles and seven adds per entry.
+constexpr uint32_t kSumStride = 68;   // two entries per lane, rows four banks apart
+template <int G, class E, class V>
+__device__ __forceinline__ void walk_group_sums(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
+                                                V& vis) {
+    constexpr int kRows = V::kRows, kSums = V::kSums, kPer = (kSums + G - 1) / G;
+    __shared__ float4 rows4[8][(kRows + 1) * kSumStride / 4];   // blocks of up to 256 threads
+    float* rows = reinterpret_cast<float*>(rows4[threadIdx.x >> 5]);
+    const uint32_t lane = lane_id(), t = lane & (uint32_t)(G - 1);
+    rows[kRows * kSumStride + lane] = 1.0f;
+    rows[kRows * kSumStride + 32u + lane] = 1.0f;
+    float acc[kPer];
+    const float4 *mul[kPer], *val[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        int m = kRows, v = kRows;
+        acc[u] = 0.0f;
+#pragma unroll
+        for (int s = u * G; s < kSums && s < (u + 1) * G; ++s)
+            if ((int)t == s - u * G) { acc[u] = vis.sum(s); m = V::mul_row(s); v = V::val_row(s); }
+        mul[u] = reinterpret_cast<const float4*>(rows + m * kSumStride + (lane - t));
+        val[u] = reinterpret_cast<const float4*>(rows + v * kSumStride + (lane - t));
+    }
+    uint32_t jn[2];
+#pragma unroll
+    for (uint32_t b = 0; b < 2u; ++b) jn[b] = b * G + t < n ? *entry(b * G + t) : i;
+    for (uint32_t kb = 0; __any_sync(kFullMask, kb < n); kb += 2u * G) {
+        uint32_t j[2];
+        float4 pj[2];
+        typename ExtraOf<V>::type ex[2];
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) {
+            j[b] = jn[b];
+            pj[b] = __ldg(p + j[b]);
+            ex[b] = fetch_extra(vis, j[b]);
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = kb + (2u + b) * G + t;
+            jn[b] = k < n ? *entry(k) : i;
+        }
+        __syncwarp();   // the last step's rows have been read
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = kb + b * G + t;
+            float r[kRows];
+            V::rows(contrib_of(vis, j[b], pj[b], ex[b], k < nc), k < n, r);
+#pragma unroll
+            for (int q = 0; q < kRows; ++q) rows[q * kSumStride + b * 32u + lane] = r[q];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b)
+#pragma unroll
+            for (int q = 0; q < G / 4; ++q)
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    const float4 m = mul[u][b * 8u + q], v = val[u][b * 8u + q];
+                    acc[u] = __fmaf_rn(m.x, v.x, acc[u]);
+                    acc[u] = __fmaf_rn(m.y, v.y, acc[u]);
+                    acc[u] = __fmaf_rn(m.z, v.z, acc[u]);
+                    acc[u] = __fmaf_rn(m.w, v.w, acc[u]);
+                }
+    }
+#pragma unroll
+    for (int s = 0; s < kSums; ++s) vis.sum(s) = __shfl_sync(kFullMask, acc[s / G], s % G, G);
+}
+
+// filter_list with G lanes per particle (entry k at entry(k), n entries, nc of them contacts; 0 for a
+// group that only takes part): each lane tests every G-th entry, its slot among the group's lanes
+// from a ballot.
+template <int G, class E>
+__device__ __forceinline__ uint32_t filter_group(E&& entry, uint32_t n, uint32_t nc, const NbList& L, uint32_t i,
+                                                 const float4& pi, float cut2, const float4* __restrict__ p) {
+    const uint32_t lane = lane_id(), t = lane & (uint32_t)(G - 1);
+    const uint32_t shift = lane & ~(uint32_t)(G - 1), gmask = G == 32 ? kFullMask : (1u << G) - 1u;
+    uint32_t m = 0, mc = 0;
+    for (uint32_t kb = 0; __any_sync(kFullMask, kb < n); kb += 4u * G) {
+        uint32_t j[4];
+        float4 pj[4];
+#pragma unroll
+        for (uint32_t b = 0; b < 4u; ++b) j[b] = kb + b * G + t < n ? *entry(kb + b * G + t) : i;
+#pragma unroll
+        for (uint32_t b = 0; b < 4u; ++b) pj[b] = __ldg(p + j[b]);
+#pragma unroll
+        for (uint32_t b = 0; b < 4u; ++b) {
+            const uint32_t k = kb + b * G + t;
+            const float rx = pi.x - pj[b].x, ry = pi.y - pj[b].y, rz = pi.z - pj[b].z;
+            const bool near = k < n && dist2(rx, ry, rz) < cut2;
+            const uint32_t all = (__ballot_sync(kFullMask, near) >> shift) & gmask;
+            const uint32_t con = (__ballot_sync(kFullMask, near && k < nc) >> shift) & gmask;
+            const uint32_t at = m + __popc(all & ((1u << t) - 1u));
+            if (near && at < L.kmax) L.list[(size_t)at * L.stride + i] = j[b];
+            m += __popc(all);
+            mc += __popc(con);
+        }
+    }
+    __syncwarp();
+    return m > L.kmax ? kListOff : (m | (mc << 8));
 }
 
 // One thread per particle over a stored list (meta not kListOff).
@@ -555,7 +701,7 @@ struct ListRecorder {
     __device__ ListRecorder(const NbList& F_, uint32_t i_) : F(F_), i(i_) {}
     __device__ static Contrib zero() { return Contrib{}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
     __device__ __forceinline__ void end_contacts(uint32_t) { nc = n; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) {
         if (n < F.kmax) *full_at(F, i, n) = j;
@@ -756,14 +902,12 @@ struct NullVisit {
     struct Contrib {};
     __device__ static Contrib zero() { return Contrib{}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4&, bool) const { return Contrib{}; }
     __device__ __forceinline__ void add(const Contrib&, bool) {}
 };
 
-__device__ __forceinline__ float shfl_f(float v, int k) { return __shfl_sync(kFullMask, v, k); }
-__device__ __forceinline__ uint32_t shfl_u(uint32_t v, int k) { return __shfl_sync(kFullMask, v, k); }
 
 // Hand particle i to the cooperative kernel; if the list is full, walk it here.
 __device__ __forceinline__ bool defer_particle(const DeferList& D, uint32_t i) {
@@ -830,21 +974,27 @@ __device__ __forceinline__ uint32_t note_particle(const DeferList& D, uint32_t i
     return k;
 }
 
-// One warp runs particle i's walk in a pass after the frame's first lambda pass: over its full
-// list, its long row or, without either, the cells.
+// Particle i's stored list as a warp reads it: its full list, else its long row; none: walk the cells.
+struct WarpList {
+    const uint32_t* row;   // null: no list
+    bool grouped;          // a full list (groups of four), else a row
+    uint32_t n, nc;
+};
+__device__ __forceinline__ WarpList warp_list(const LongLists& LL, const NbList& F, uint32_t i) {
+    const uint32_t fm = F.list ? F.meta[i] : kListOff;
+    if (!(fm & kListOff)) return WarpList{F.list, true, fm & 0xFFu, (fm >> 8) & 0xFFu};
+    const uint32_t q = fm & ~(kListOff | kListWalked);
+    const uint32_t m = (F.list && q < LL.slots) ? LL.meta[q] : kListOff;
+    if (m == kListOff) return WarpList{nullptr, false, 0u, 0u};
+    return WarpList{LL.list + (size_t)q * kLongMax, false, m & 0xFFFFu, m >> 16};
+}
+// One warp runs particle i's walk in a pass after the frame's first lambda pass.
 template <class V>
 __device__ __forceinline__ void walk_warp(const DevParams& P, const SceneCtx& S, uint32_t i, float4 anchor,
                                           const float4* __restrict__ p, const uint32_t* __restrict__ cs,
                                           const uint32_t* __restrict__ ce, const LongLists& LL, const NbList& F, V& vis) {
-    const uint32_t fm = F.list ? F.meta[i] : kListOff;
-    if (!(fm & kListOff)) {
-        walk_row([&](uint32_t k) { return full_at(F, i, k); }, fm & 0xFFu, (fm >> 8) & 0xFFu, i, p, vis);
-        return;
-    }
-    const uint32_t q = fm & ~(kListOff | kListWalked);
-    const uint32_t m = (F.list && q < LL.slots) ? LL.meta[q] : kListOff;
-    const uint32_t* row = LL.list + (size_t)q * kLongMax;
-    if (m != kListOff) walk_row([&](uint32_t k) { return row + k; }, m & 0xFFFFu, m >> 16, i, p, vis);
+    const WarpList W = warp_list(LL, F, i);
+    if (W.row) walk_group<32>([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, i, p, vis);
     else walk_coop(P, S, i, anchor, p, cs, ce, vis);
 }
 
@@ -862,9 +1012,9 @@ struct LambdaVisit {
     __device__ void reset() { A = B = Cx = Cy = Cz = Cw = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k) {
-        return Contrib{shfl_f(c.a, k), shfl_f(c.b, k), shfl_f(c.s, k), shfl_f(c.rx, k), shfl_f(c.ry, k),
-                       shfl_f(c.rz, k), shfl_f(c.rw, k), shfl_u(c.near, k)};
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
+        return Contrib{shfl_f(c.a, k, width), shfl_f(c.b, k, width), shfl_f(c.s, k, width), shfl_f(c.rx, k, width), shfl_f(c.ry, k, width),
+                       shfl_f(c.rz, k, width), shfl_f(c.rw, k, width), shfl_u(c.near, k, width)};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
@@ -890,6 +1040,18 @@ struct LambdaVisit {
             " @q fma.rn.f32 %5, %9, %13, %5; }"
             : "+f"(A), "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz), "+f"(Cw)
             : "r"((live && c.near) ? 1u : 0u), "f"(c.a), "f"(c.b), "f"(c.s), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
+    }
+    // walk_group_sums: A, B, C from the rows a, b, s, r
+    static constexpr int kRows = 7, kSums = 6;
+    __device__ static constexpr int mul_row(int s) { return s < 2 ? kRows : 2; }
+    __device__ static constexpr int val_row(int s) { return s < 2 ? s : s + 1; }
+    __device__ __forceinline__ float& sum(int s) {
+        return s == 0 ? A : (s == 1 ? B : (s == 2 ? Cx : (s == 3 ? Cy : (s == 4 ? Cz : Cw))));
+    }
+    __device__ __forceinline__ static void rows(const Contrib& c, bool live, float* r) {
+        const bool on = live && c.near;
+        r[0] = on ? c.a : 0.f; r[1] = on ? c.b : 0.f; r[2] = on ? c.s : 0.f;
+        r[3] = on ? c.rx : 0.f; r[4] = on ? c.ry : 0.f; r[5] = on ? c.rz : 0.f; r[6] = on ? c.rw : 0.f;
     }
     // the sums the reverse pass needs: aux[i] = (rho, B, S.x, S.y), aux[N + i] = (S.z, S.w, 0, 0)
     __device__ __forceinline__ void store_aux(float4* __restrict__ aux, uint32_t N, uint32_t i) const {
@@ -941,12 +1103,12 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         }
         F.meta[i] = fm;
         const bool listed = !(fm & kListOff);
+        if (!listed && !(fm & kListWalked)) return;
         const uint32_t lm = (L.list && listed) ? filter_list<true>(F, fm, L, i, pi, P.cut2, p) : kListOff;
         if (L.list) {
             L.meta[i] = lm;
             if (lm == kListOff) note_particle(DN, i);
         }
-        if (!listed && !(fm & kListWalked)) return;
         if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
         else if (listed) walk_full<true>(F, i, fm, p, vis);
         else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
@@ -979,14 +1141,27 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
     if (aux) vis.store_aux(aux, P.N, i);
 }
 
-// One warp computes lambda_i.
+// One warp computes lambda_i.  With L, it also leaves the particle's near list for the delta pass (and
+// sums over that), or notes the particle in DN: the cell-end range's 512 entries hold ~6 near ones, and
+// walked again in the delta pass they held it up (21 us against 13 for lambda_list with 33k particles).
 __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                                             float* __restrict__ lambda, float4* __restrict__ aux, uint32_t i,
-                                            const LongLists& LL, const NbList& F) {
+                                            const LongLists& LL, const NbList& F, const NbList& L, const DeferList& DN) {
     const SceneCtx S = scene_ctx(P, i);
-    LambdaVisit vis(P, p[i]);
-    walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
+    const float4 pi = p[i];
+    LambdaVisit vis(P, pi);
+    uint32_t lm = kListOff;
+    if (L.list) {
+        const WarpList W = warp_list(LL, F, i);
+        if (W.row) lm = filter_group<32>([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, L, i, pi, P.cut2, p);
+        if (lane_id() == 0) {
+            L.meta[i] = lm;
+            if (lm == kListOff) note_particle(DN, i);
+        }
+    }
+    if (lm != kListOff) walk_group<32>([&](uint32_t k) { return L.list + (size_t)k * L.stride + i; }, lm & 0xFFu, lm >> 8, i, p, vis);
+    else walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) {
         lambda[i] = vis.finish(S.rho0);
         if (aux) vis.store_aux(aux, P.N, i);
@@ -996,15 +1171,16 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
 __global__ void __launch_bounds__(128)
 lambda_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
                    const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux) {
-    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LongLists{}, NbList{}); });
+    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LongLists{}, NbList{}, NbList{}, DeferList{}); });
 }
 
 // After lambda_kernel stored the full lists: the particles left without one (the set DF), a warp
-// each.  Stores their long rows and computes their lambda.
+// each.  Stores their long rows, computes their lambda and leaves their near lists.
 __global__ void __launch_bounds__(128)
 lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
                    const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList DF, float4* __restrict__ aux,
-                   const __grid_constant__ LongLists LL, const __grid_constant__ NbList F) {
+                   const __grid_constant__ LongLists LL, const __grid_constant__ NbList F, const __grid_constant__ NbList L,
+                   const __grid_constant__ DeferList DN) {
     const uint32_t n = min(*DF.count, DF.cap);
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < n; q += warps) {
@@ -1015,7 +1191,7 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
             if (lane_id() == 0) LL.meta[q] = m;
             __syncwarp();
         }
-        coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F);
+        coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN);
     }
 }
 
@@ -1026,21 +1202,15 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
 __global__ void __launch_bounds__(256, 5)
 lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
-                   CoopSet C, DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+                   CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const uint32_t fm = F.meta[i];
-    if (fm & kListOff) {
-        if (L.list) {
-            L.meta[i] = kListOff;
-            note_particle(DN, i);
-        }
-        return;
-    }
+    if (fm & kListOff) return;   // in the set C
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
     LambdaVisit vis(P, pi);
@@ -1053,6 +1223,83 @@ lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict
     else walk_full(F, i, fm, p, vis);
     lambda[i] = vis.finish(S.rho0);
     if (aux) vis.store_aux(aux, P.N, i);
+}
+
+// The passes of a small simulation: G lanes per particle.  With a thread per particle a 4,275-particle
+// pass is 34 blocks on 152 SMs, each thread a serial chain of list loads, position loads and adds; a
+// group takes the loads of G entries at a time.  The sums are added in list order all the same.
+//
+// The frame's first lambda pass (lambda_kernel with full lists): the list enumerated, stored and
+// filtered by the group.  Particles without a full list go to lambda_long_kernel.
+template <int G>
+__global__ void __launch_bounds__(256)
+lambda_group_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
+                    float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F,
+                    DeferList DF, DeferList DN) {
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = tid / G < P.N, first = on && tid % G == 0u;
+    const uint32_t i = on ? tid / G : P.N - 1u;
+    const SceneCtx S = scene_ctx(P, i);
+    const float4 pi = p[i];
+    const GroupList R = enumerate_group<G>(P, S, i, pa[i], on, cs, ce, min(P.M, F.kmax + 1u), true,
+                                           [&](uint32_t k, uint32_t j) { if (k < F.kmax) *full_at(F, i, k) = j; });
+    __syncwarp();
+    const bool listed = on && !R.handed_over && R.n <= F.kmax;
+    if (first) F.meta[i] = listed ? (R.n | (R.nc << 8)) : (kListOff | note_particle(DF, i));
+    uint32_t lm = kListOff;
+    if (L.list) {
+        lm = filter_group<G>([&](uint32_t k) { return full_at(F, i, k); }, listed ? R.n : 0u, R.nc, L, i, pi, P.cut2, p);
+        if (!listed) lm = kListOff;
+        if (first && listed) {
+            L.meta[i] = lm;
+            if (lm == kListOff) note_particle(DN, i);
+        }
+    }
+    LambdaVisit vis(P, pi);
+    const bool near = lm != kListOff;
+    walk_group_sums<G>([&](uint32_t k) { return near ? L.list + (size_t)k * L.stride + i : full_at(F, i, k); },
+                  !listed ? 0u : (near ? lm & 0xFFu : R.n), 0u, i, p, vis);
+    if (first && listed) {
+        lambda[i] = vis.finish(S.rho0);
+        if (aux) vis.store_aux(aux, P.N, i);
+    }
+}
+
+// lambda_list_kernel with G lanes per particle.
+template <int G>
+__global__ void __launch_bounds__(256)
+lambda_list_group_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+                         const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
+                         CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L,
+                         const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+    if (blockIdx.x < C.blocks) {
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN); });
+        return;
+    }
+    const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
+    const bool on = tid / G < P.N, first = on && tid % G == 0u;
+    const uint32_t i = on ? tid / G : P.N - 1u;
+    const uint32_t fm = F.meta[i];
+    const bool listed = on && !(fm & kListOff);
+    const float4 pi = p[i];
+    uint32_t lm = kListOff;
+    if (L.list) {
+        lm = filter_group<G>([&](uint32_t k) { return full_at(F, i, k); }, listed ? fm & 0xFFu : 0u, (fm >> 8) & 0xFFu, L, i, pi, P.cut2, p);
+        if (!listed) lm = kListOff;
+        if (first && listed) {
+            L.meta[i] = lm;
+            if (lm == kListOff) note_particle(DN, i);
+        }
+    }
+    LambdaVisit vis(P, pi);
+    const bool near = lm != kListOff;
+    walk_group_sums<G>([&](uint32_t k) { return near ? L.list + (size_t)k * L.stride + i : full_at(F, i, k); },
+                  !listed ? 0u : (near ? lm & 0xFFu : fm & 0xFFu), 0u, i, p, vis);
+    if (first && listed) {
+        lambda[i] = vis.finish(scene_ctx(P, i).rho0);
+        if (aux) vis.store_aux(aux, P.N, i);
+    }
 }
 
 // ======================================================================================
@@ -1098,9 +1345,9 @@ struct DeltaVisitT {
     __device__ void reset() { ax = ay = az = aw = 0.f; pacc = pi; xacc = xi; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.flags != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k) {
-        return Contrib{shfl_f(c.coef, k), shfl_f(c.rx, k), shfl_f(c.ry, k), shfl_f(c.rz, k), shfl_f(c.rw, k),
-                       shfl_f(c.t, k), shfl_u(c.flags, k)};
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
+        return Contrib{shfl_f(c.coef, k, width), shfl_f(c.rx, k, width), shfl_f(c.ry, k, width), shfl_f(c.rz, k, width), shfl_f(c.rw, k, width),
+                       shfl_f(c.t, k, width), shfl_u(c.flags, k, width)};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float;   // lambda_j
@@ -1160,6 +1407,20 @@ struct DeltaVisitT {
             k.flags = 2u;
             add(k, true);
         }
+    }
+    // walk_group_sums: the density part's sums, then the contacts' on p* and x, from coef, -t and r
+    static constexpr int kRows = 6, kSums = 10;
+    __device__ static constexpr int mul_row(int s) { return s < 4 ? 0 : 1; }
+    __device__ static constexpr int val_row(int s) { return s < 4 ? 2 + s : (s < 7 ? s - 2 : s - 5); }
+    __device__ __forceinline__ float& sum(int s) {
+        return s == 0 ? ax : (s == 1 ? ay : (s == 2 ? az : (s == 3 ? aw : (s == 4 ? pacc.x : (s == 5 ? pacc.y : (s == 6 ? pacc.z
+               : (s == 7 ? xacc.x : (s == 8 ? xacc.y : xacc.z))))))));
+    }
+    __device__ __forceinline__ static void rows(const Contrib& c, bool live, float* r) {
+        const uint32_t f = live ? c.flags : 0u;
+        r[0] = (f & 1u) ? c.coef : 0.f;
+        r[1] = (f & 2u) ? -c.t : 0.f;
+        r[2] = f ? c.rx : 0.f; r[3] = f ? c.ry : 0.f; r[4] = f ? c.rz : 0.f; r[5] = f ? c.rw : 0.f;
     }
 };
 using DeltaVisit = DeltaVisitT<kDeltaAny>;
@@ -1265,6 +1526,34 @@ delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const f
     delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
+// delta_list_kernel with G lanes per particle (small simulations, see lambda_group_kernel).
+template <bool kFull, int G>
+__global__ void __launch_bounds__(256)
+delta_list_group_kernel(const __grid_constant__ DevParams P, uint32_t mode, const float4* __restrict__ pin,
+                        const float4* __restrict__ pa, float4* __restrict__ pout, float4* __restrict__ x,
+                        float4* __restrict__ v, const float* __restrict__ lambda, const float* __restrict__ w,
+                        float4* __restrict__ delta, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                        CoopSet C, const __grid_constant__ NbList L, const __grid_constant__ NbList F,
+                        const __grid_constant__ LongLists LL) {
+    if (blockIdx.x < C.blocks) {
+        run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i, LL, F); });
+        return;
+    }
+    const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
+    const bool on = tid / G < P.N;
+    const uint32_t i = on ? tid / G : P.N - 1u;
+    const uint32_t meta = L.meta[i];
+    const bool listed = on && !(meta & kListOff);
+    const float4 pi = pin[i];
+    const bool need_x = (mode & (kDoCollide | kDoUpdate)) != 0;
+    const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float li = (mode & kDoDelta) ? lambda[i] : 0.f;
+    DeltaVisit vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
+    walk_group_sums<G>([&](uint32_t k) { return kFull ? full_at(L, i, k) : L.list + (size_t)k * L.stride + i; },
+                  listed ? meta & 0xFFu : 0u, (meta >> 8) & 0xFFu, i, pin, vis);
+    if (listed && tid % G == 0u) delta_finish(P, scene_ctx(P, i).rho0, mode, i, vis, pout, x, v, delta);
+}
+
 __global__ void __launch_bounds__(128)
 delta_coop_kernel(const __grid_constant__ DevParams P, uint32_t mode, const float4* __restrict__ pin, const float4* __restrict__ pa, float4* __restrict__ pout,
                   float4* __restrict__ x, float4* __restrict__ v, const float* __restrict__ lambda, const float* __restrict__ w,
@@ -1299,8 +1588,8 @@ struct OmegaVisit {
     __device__ void reset() { ox = oy = oz = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k) {
-        return Contrib{shfl_f(c.ox, k), shfl_f(c.oy, k), shfl_f(c.oz, k), shfl_u(c.near, k)};
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
+        return Contrib{shfl_f(c.ox, k, width), shfl_f(c.oy, k, width), shfl_f(c.oz, k, width), shfl_u(c.near, k, width)};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float4;   // v_j
@@ -1323,6 +1612,14 @@ struct OmegaVisit {
             " @q add.rn.f32 %2, %2, %6; }"
             : "+f"(ox), "+f"(oy), "+f"(oz)
             : "r"((live && c.near) ? 1u : 0u), "f"(c.ox), "f"(c.oy), "f"(c.oz));
+    }
+    static constexpr int kRows = 3, kSums = 3;   // walk_group_sums
+    __device__ static constexpr int mul_row(int) { return kRows; }
+    __device__ static constexpr int val_row(int s) { return s; }
+    __device__ __forceinline__ float& sum(int s) { return s == 0 ? ox : (s == 1 ? oy : oz); }
+    __device__ __forceinline__ static void rows(const Contrib& c, bool live, float* r) {
+        const bool on = live && c.near;
+        r[0] = on ? c.ox : 0.f; r[1] = on ? c.oy : 0.f; r[2] = on ? c.oz : 0.f;
     }
 };
 
@@ -1405,6 +1702,39 @@ omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict_
     omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
 }
 
+// omega_list_kernel with G lanes per particle (small simulations, see lambda_group_kernel).
+template <int G>
+__global__ void __launch_bounds__(256)
+omega_list_group_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+                        const float4* __restrict__ v, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                        float4* __restrict__ omega, CoopSet C, DeferList DN, const __grid_constant__ NbList L,
+                        const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+    if (blockIdx.x < C.blocks) {
+        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F); });
+        return;
+    }
+    const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
+    const bool on = tid / G < P.N, first = on && tid % G == 0u;
+    const uint32_t i = on ? tid / G : P.N - 1u;
+    const uint32_t fm = F.meta[i];
+    const bool listed = on && !(fm & kListOff);
+    const float4 pi = p[i];
+    uint32_t lm = kListOff;
+    if (L.list) {
+        lm = filter_group<G>([&](uint32_t k) { return full_at(F, i, k); }, listed ? fm & 0xFFu : 0u, (fm >> 8) & 0xFFu, L, i, pi, P.cut2, p);
+        if (!listed) lm = kListOff;
+        if (first) {
+            L.meta[i] = lm;
+            if (lm == kListOff) note_particle(DN, i);
+        }
+    }
+    OmegaVisit vis(P, v, pi, v[i]);
+    const bool near = lm != kListOff;
+    walk_group_sums<G>([&](uint32_t k) { return near ? L.list + (size_t)k * L.stride + i : full_at(F, i, k); },
+                  !listed ? 0u : (near ? lm & 0xFFu : fm & 0xFFu), 0u, i, p, vis);
+    if (first && listed) omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
+}
+
 __global__ void __launch_bounds__(128)
 omega_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
@@ -1438,9 +1768,9 @@ struct VortViscVisitT {
     __device__ void reset() { gx = gy = gz = sx = sy = sz = sw = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.flags != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k) {
-        return Contrib{shfl_f(c.gx, k), shfl_f(c.gy, k), shfl_f(c.gz, k), shfl_f(c.sx, k),
-                       shfl_f(c.sy, k), shfl_f(c.sz, k), shfl_f(c.sw, k), shfl_u(c.flags, k)};
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
+        return Contrib{shfl_f(c.gx, k, width), shfl_f(c.gy, k, width), shfl_f(c.gz, k, width), shfl_f(c.sx, k, width),
+                       shfl_f(c.sy, k, width), shfl_f(c.sz, k, width), shfl_f(c.sw, k, width), shfl_u(c.flags, k, width)};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = VortViscExtra<kTerms>;
@@ -1488,6 +1818,17 @@ struct VortViscVisitT {
                 " @q add.rn.f32 %2, %2, %7; @q add.rn.f32 %3, %3, %8; }"
                 : "+f"(sx), "+f"(sy), "+f"(sz), "+f"(sw)
                 : "r"((live && (c.flags & 2u)) ? 1u : 0u), "f"(c.sx), "f"(c.sy), "f"(c.sz), "f"(c.sw));
+    }
+    static constexpr int kRows = 7, kSums = 7;   // walk_group_sums
+    __device__ static constexpr int mul_row(int) { return kRows; }
+    __device__ static constexpr int val_row(int s) { return s; }
+    __device__ __forceinline__ float& sum(int s) {
+        return s == 0 ? gx : (s == 1 ? gy : (s == 2 ? gz : (s == 3 ? sx : (s == 4 ? sy : (s == 5 ? sz : sw)))));
+    }
+    __device__ __forceinline__ static void rows(const Contrib& c, bool live, float* r) {
+        const bool vo = live && (c.flags & 1u), vs = live && (c.flags & 2u);
+        r[0] = vo ? c.gx : 0.f; r[1] = vo ? c.gy : 0.f; r[2] = vo ? c.gz : 0.f;
+        r[3] = vs ? c.sx : 0.f; r[4] = vs ? c.sy : 0.f; r[5] = vs ? c.sz : 0.f; r[6] = vs ? c.sw : 0.f;
     }
 };
 
@@ -1600,6 +1941,34 @@ vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restr
     vort_visc_finish(P, i, vis, vis, vout, fext, w, vhost);
 }
 
+// vort_visc_list_kernel with G lanes per particle (small simulations, see lambda_group_kernel); both
+// terms in one walk of Lv, the full list (kFull) or omega's near list.
+template <bool kFull, int G>
+__global__ void __launch_bounds__(256)
+vort_visc_list_group_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
+                            const float4* __restrict__ vin, float4* __restrict__ vout, const float4* __restrict__ omega,
+                            float4* __restrict__ fext, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                            int do_vort, int do_visc, const float* __restrict__ w, CoopSet C,
+                            const __grid_constant__ NbList Lv, float4* __restrict__ vhost,
+                            const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+    if (blockIdx.x < C.blocks) {
+        run_coop_set(C, [&](uint32_t i) {
+            coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, vhost, LL, F);
+        });
+        return;
+    }
+    const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
+    const bool on = tid / G < P.N;
+    const uint32_t i = on ? tid / G : P.N - 1u;
+    const uint32_t meta = Lv.meta[i];
+    const bool listed = on && !(meta & kListOff);
+    const float4 oi = do_vort ? omega[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    VortViscVisit vis(P, vin, omega, p[i], vin[i], oi, do_vort != 0, do_visc != 0);
+    walk_group_sums<G>([&](uint32_t k) { return kFull ? full_at(Lv, i, k) : Lv.list + (size_t)k * Lv.stride + i; },
+                  listed ? meta & 0xFFu : 0u, (meta >> 8) & 0xFFu, i, p, vis);
+    if (listed && tid % G == 0u) vort_visc_finish(P, i, vis, vis, vout, fext, w, vhost);
+}
+
 __global__ void __launch_bounds__(128)
 vort_visc_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ vin,
                       float4* __restrict__ vout, const float4* __restrict__ omega, float4* __restrict__ fext,
@@ -1622,7 +1991,7 @@ struct DensityVisit {
     __device__ DensityVisit(const DevParams& P_, float4 pi_) : P(P_), pi(pi_) {}
     __device__ static Contrib zero() { return Contrib{0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k) { return Contrib{shfl_f(c.a, k), shfl_u(c.near, k)}; }
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_f(c.a, k, width), shfl_u(c.near, k, width)}; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
@@ -1695,7 +2064,7 @@ struct ListVisit {
     __device__ ListVisit(uint32_t* o, uint32_t c) : out(o), cap(c) {}
     __device__ static Contrib zero() { return Contrib{0u}; }
     __device__ static bool effective(const Contrib&) { return true; }
-    __device__ static Contrib shfl(const Contrib& c, int k) { return Contrib{shfl_u(c.j, k)}; }
+    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_u(c.j, k, width)}; }
     __device__ __forceinline__ void end_contacts(uint32_t c) { contacts = c; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) const { return Contrib{j}; }
     __device__ __forceinline__ void add(const Contrib& c, bool) {

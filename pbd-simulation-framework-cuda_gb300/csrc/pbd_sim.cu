@@ -353,13 +353,30 @@ static void launch_delta_staged(uint32_t N, cudaStream_t st, const DevParams& P,
         delta_staged_kernel<0><<<g, kStageThreads, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, F, LL);
 }
 
+// Lanes per particle of the list passes: more than one while the particles alone leave most of the
+// GPU idle and a pass is one thread's chain of loads.  Measured (GB300, us a frame, 1 / 4 / 8 / 16
+// lanes): 4,275 particles 87 / 64 / 62 / 60; 15,525 (config.txt's 72 entries) 136 / 126 / 117 / 121;
+// 32,768 103 / 103 / 120 / 143; at 65,536 four lanes are 13% slower than one.
+int pass_lanes(uint32_t N) {
+    return N <= 8192u ? 16 : (N <= 16384u ? 8 : (N <= 24576u ? 4 : 1));
+}
+// A group pass's kernel for the lane count.
+#define BY_LANES(name, ...) \
+    (lanes == 4 ? name<__VA_ARGS__ 4> : (lanes == 8 ? name<__VA_ARGS__ 8> : name<__VA_ARGS__ 16>))
+#define COMMA ,
+
 // delta_list_kernel for `mode`: the fluid frame's two pass modes run code specialised on the mode
 // and, with config.txt's nSCorr and far pairs exactly zero, on those (DeltaKnown).
 template <bool kFull>
 static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevParams& P, uint32_t mode,
                               const float4* pin, const float4* pa, float4* pout, float4* x, float4* v, const float* lam,
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
-                              const NbList& L, const NbList& F, const LongLists& LL) {
+                              const NbList& L, const NbList& F, const LongLists& LL, int lanes, uint32_t N) {
+    if (lanes > 1) {
+        auto k = BY_LANES(delta_list_group_kernel, kFull COMMA);
+        k<<<div_up((uint64_t)N * lanes, tn) + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
+        return;
+    }
     constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply, kLast = kFluid | kDoUpdate;
     const bool known = P.n_scorr == 4 && P.far_pairs_zero != 0u;
     auto k = delta_list_kernel<0, kFull, kDeltaAny>;
@@ -438,6 +455,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     auto next_p = [&](int c) { return c == anchor ? (anchor + 1) % 3 : 3 - c - anchor; };
 
     const uint32_t gn = div_up(N, tn);
+    const int lanes = pass_lanes(N);
+    const uint32_t gl = div_up((uint64_t)N * lanes, tn);   // blocks of the group passes
     const DeferList D{s->defer_items, s->defer_count, s->defer_done, s->defer_cap};
     const uint32_t gc = (uint32_t)s->num_sms * 2u;   // cooperative kernels: grid-stride over the deferred
     // the list passes' own cooperative blocks: DF is read by every full-list pass of the frame,
@@ -496,16 +515,27 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 lambda_staged_kernel<<<kCoopBlocks + div_up(N, kStageThreads), kStageThreads, 0, st>>>(
                     P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF, F, s->ll);
                 nl += 1;
+            } else if (use_full && it > 0 && lanes > 1) {
+                auto k = BY_LANES(lambda_list_group_kernel, );
+                k<<<gl + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF,
+                                                   Lr.list ? DN : DX, aux, Lr, F, s->ll);
+                nl += 1;
             } else if (use_full && it > 0) {
                 lambda_list_kernel<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
                                                                     CF, Lr.list ? DN : DX, aux, Lr, F, s->ll);
                 nl += 1;
+            } else if (use_full && lanes > 1) {
+                auto k = BY_LANES(lambda_group_kernel, );
+                k<<<gl, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, aux, Lr, F, DF, Lr.list ? DN : DX);
+                lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, DF,
+                                                                aux, s->ll, F, Lr, Lr.list ? DN : DX);
+                nl += 2;
             } else {
                 lambda_kernel<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux, Lr,
                                                  use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots);
                 if (use_full)
                     lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
-                                                                    DF, aux, s->ll, F);
+                                                                    DF, aux, s->ll, F, Lr, Lr.list ? DN : DX);
                 else
                     lambda_coop_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux);
                 nl += 2;
@@ -525,7 +555,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 if (by_list) {
                     (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                         gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
+                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N);
                     nl += 1;
                 } else {
                     delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -603,7 +633,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             } else if (by_list) {
                 (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                     gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll);
+                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N);
                 nl += 1;
             } else {
                 delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -647,7 +677,11 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
         // viscosity alone walks them: the particles left without one go to its cooperative blocks
         const DeferList DNo = (Lo.list && !vort) ? DN : DX;
         if (use_full) {
-            if (Lo.list)
+            if (lanes > 1) {
+                auto k = BY_LANES(omega_list_group_kernel, );
+                k<<<gl + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end, s->omega, CF,
+                                                   DNo, Lo, F, s->ll);
+            } else if (Lo.list)
                 omega_list_kernel<true><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end,
                                                                s->omega, CF, DNo, Lo, F, s->ll);
             else
@@ -671,11 +705,18 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
         PROF_BEGIN(Lv.list ? "vort_visc_list" : "vort_visc");
         if (Lv.list) {
             float4* const vh = (readback && visc) ? s->rb_dev + s->cap : nullptr;
+            if (lanes > 1) {
+                auto kg = vfull ? BY_LANES(vort_visc_list_group_kernel, true COMMA)
+                                : BY_LANES(vort_visc_list_group_kernel, false COMMA);
+                kg<<<gl + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
+                                                    s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, vh, F, s->ll);
+            } else {
             auto k = Ln.list ? vort_visc_list_kernel<kVortVisc>
                              : (vfull ? vort_visc_list_kernel<kVortViscFull> : vort_visc_list_kernel<kViscNear>);
             k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
                                                s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, Ln, vh,
                                                F, s->ll);
+            }
             v_read = v_read || vh != nullptr;
             nl += 1;
         } else {

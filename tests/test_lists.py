@@ -252,3 +252,20 @@ def test_delta_pass_variants_bit_identical_to_full_walk(need_gpu, pbd, scenes, d
     a = _run(pbd, params, pos, vel, 3, inv_mass=w)
     b = _run(pbd, params, pos, vel, 3, inv_mass=w, full_walk=True)
     _same(a, b)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 1, 3), (3, 5, 7), (16, 32, 16), (19, 19, 23), (24, 25, 27), (16, 32, 32), (25, 27, 29), (24, 32, 32), (27, 29, 32)])
+def test_lanes_per_particle_bit_identical_to_full_walk(need_gpu, pbd, scenes, shape, dense):
+    """the list passes take 16, 8, 4 or 1 lanes per particle by the number of particles (16 up to 8,192,
+    8 up to 16,384, 4 up to 24,576): both sides of every change, partial warps, one particle"""
+    params = scenes.workload_params(pbd, 40, 1995.0 if dense else 1000.0, vorticity=0.0005, viscosity=0.00015 if dense else 0.01)
+    params.lambda_epsilon = 0.0001 if dense else 0.1
+    if dense:
+        params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 4.1, 3.5, 2
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(*shape, seed=24, spacing=0.95)
+    vel[:, :3] = np.random.default_rng(24).normal(0, 0.5, size=(len(vel), 3)).astype(np.float32)
+    a = _run(pbd, params, pos, vel, 2)
+    b = _run(pbd, params, pos, vel, 2, full_walk=True)
+    _same(a, b)
