@@ -9,8 +9,8 @@
 //
 // The working memory is the file-scope array below: kNoAllocMaxKeys keys at most
 // (1,048,576), kScratchWords * 4 = 9,441,536 bytes (9.0 MiB).  Every GPU that loads the library
-// keeps that array until the process exits.  All calls share it and it keeps the last call's
-// contents, so each call first zeroes the parts that must start at zero; calls whose GPU work
+// keeps that array until the process exits.  All calls share it: each call zeroes the parts that must
+// start at zero, the digit counts at its end and the rest at its start; calls whose GPU work
 // overlaps (different streams, or different host threads) race on it and must be serialised by
 // the caller.  Its error word holds the outcome of the last call on the device:
 // pbd_sort_noalloc_status reads it.
@@ -44,7 +44,8 @@ constexpr size_t kOffHist = kOffVals + kNoAllocMaxKeys;
 constexpr size_t kOffStatus = kOffHist + (size_t)kMaxPasses * kRadix;
 constexpr size_t kOffTiles = kOffStatus + (size_t)kMaxPasses * kNoAllocMaxTiles * kRadix;
 constexpr size_t kOffErr = kOffTiles + kMaxPasses;
-constexpr size_t kScratchWords = (kOffErr + 1 + 63) & ~size_t(63);
+constexpr size_t kOffDone = kOffErr + 1;   // finished tiles of a sort's last pass
+constexpr size_t kScratchWords = (kOffDone + 1 + 63) & ~size_t(63);
 
 static_assert(kScratchWords * 4 == 9441536, "the fixed array's size is stated in pbd.h");
 static __device__ __align__(256) uint32_t g_sort_scratch[kScratchWords];
@@ -56,28 +57,40 @@ uint32_t* g_scratch_ptr[kMaxDevices] = {};
 uint32_t g_spin_limit = kSpinLimit;
 uint32_t g_hold = 0;
 
-// Zero the histograms, the look-back rows the call will use, the tile counters and the error word.
-__global__ void noalloc_clear_kernel(uint32_t* base, uint32_t ntiles) {
+// Digit histograms of every pass (the sim counts them in its predict kernel), after zeroing the look-back
+// rows the call will use, the tile counters and the error word.  The histograms are zero when a call
+// starts: the array starts as zeros and every sort's last tile zeroes them (SortScratch::done).  Two
+// blocks of 512 per SM and keys four at a time where they are aligned: with 1,024 blocks of 256 the
+// flush of the blocks' histograms took most of the time (with the clearing kernel before it 16 us for
+// 1,048,576 keys).
+__global__ void __launch_bounds__(512)
+noalloc_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* base, uint32_t ntiles, int npasses,
+                    uint32_t key_bits) {
+    __shared__ uint32_t sh[kMaxPasses * kRadix];
+    for (int b = threadIdx.x; b < kMaxPasses * kRadix; b += blockDim.x) sh[b] = 0u;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    for (uint32_t k = t; k < kMaxPasses * kRadix; k += stride) base[kOffHist + k] = 0u;
-    for (uint32_t pass = 0; pass < kMaxPasses; ++pass)
+    for (int pass = 0; pass < npasses; ++pass)
         for (uint32_t k = t; k < ntiles * kRadix; k += stride)
             base[kOffStatus + (size_t)pass * kNoAllocMaxTiles * kRadix + k] = 0u;
     if (t < kMaxPasses) base[kOffTiles + t] = 0u;
     if (t == 0) base[kOffErr] = 0u;
-}
-
-// Digit histograms of every pass (the sim counts them in its predict kernel).
-__global__ void noalloc_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ hist,
-                                    int npasses, uint32_t key_bits) {
-    __shared__ uint32_t sh[kMaxPasses * kRadix];
-    for (int b = threadIdx.x; b < kMaxPasses * kRadix; b += blockDim.x) sh[b] = 0u;
     __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t key = keys[i];
-        for (int ps = 0; ps < npasses; ++ps) atomicAdd(&sh[ps * kRadix + sort_digit(key, ps, key_bits)], 1u);
+    const uint32_t n4 = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u ? n / 4u : 0u;
+    const uint32_t warp0 = t & ~31u;
+    for (uint32_t g = warp0; g < n4; g += stride) {   // whole warps: count_digits takes all lanes
+        const bool in = g + (t & 31u) < n4;
+        const uint4 k = in ? reinterpret_cast<const uint4*>(keys)[g + (t & 31u)] : make_uint4(0u, 0u, 0u, 0u);
+        count_digits<false>(sh, k.x, in, npasses, key_bits);
+        count_digits<false>(sh, k.y, in, npasses, key_bits);
+        count_digits<false>(sh, k.z, in, npasses, key_bits);
+        count_digits<false>(sh, k.w, in, npasses, key_bits);
+    }
+    for (uint32_t i = 4u * n4 + warp0; i < n; i += stride) {
+        const bool in = i + (t & 31u) < n;
+        count_digits<false>(sh, in ? keys[i + (t & 31u)] : 0u, in, npasses, key_bits);
     }
     __syncthreads();
+    uint32_t* hist = base + kOffHist;
     for (int b = threadIdx.x; b < npasses * kRadix; b += blockDim.x)
         if (sh[b]) atomicAdd(&hist[b], sh[b]);
 }
@@ -143,9 +156,8 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
     }
     S.key_bits = key_bits;
 
-    noalloc_clear_kernel<<<32, 256, 0, st>>>(base, plan.ntiles);
-    const uint32_t gh = std::min<uint32_t>((n + 255) / 256, 1024u);
-    noalloc_hist_kernel<<<gh, 256, 0, st>>>(d_keys_in, n, S.hist, npasses, key_bits);
+    const uint32_t gh = std::min<uint32_t>((n + 2047) / 2048, 2u * kSortSpread);
+    noalloc_hist_kernel<<<gh, 512, 0, st>>>(d_keys_in, n, base, plan.ntiles, npasses, key_bits);
     // Ping-pong between the caller's outputs and the fixed array so that the last pass
     // writes the outputs: pass p writes the outputs when (npasses - 1 - p) is even.
     uint32_t* tmp_k = base + kOffKeys;
@@ -156,6 +168,7 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
         const bool to_out = ((npasses - 1 - pass) % 2) == 0;
         uint32_t* dk = to_out ? d_keys_out : tmp_k;
         uint32_t* dv = to_out ? d_perm_out : tmp_v;
+        if (pass == npasses - 1) S.done = base + kOffDone;
         sort_pass(st, plan, src_k, src_v, dk, dv, n, pass, S);
         src_k = dk;
         src_v = dv;

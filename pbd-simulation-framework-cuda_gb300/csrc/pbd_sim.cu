@@ -407,7 +407,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
 
     // applyForces + initializeCellIds (+ histograms, + clearing last frame's cells)
     const uint32_t total = std::max(N, s->table_hint);
-    const uint32_t gpred = std::max(1u, std::min(div_up(total, kThreadsParticle), (uint32_t)s->num_sms * 8u));
+    const uint32_t gpred = std::max(1u, std::min(div_up(total, kPredictThreads), (uint32_t)s->num_sms * kPredictBlocksPerSm));
     if (tape) {
         cudaMemcpyAsync(tape->x_in, s->x[cur.x], (size_t)N * 16, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(tape->v_in, s->v[cur.v], (size_t)N * 16, cudaMemcpyDeviceToDevice, st);
@@ -415,7 +415,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     }
     PROF_BEGIN("predict_key");
     const float* wcur = s->mass_used ? s->w[cur.x] : nullptr;
-    predict_key_kernel<<<gpred, kThreadsParticle, 0, st>>>(P, s->x[cur.x], s->v[cur.v], s->p[cur.p], s->fext, wcur,
+    predict_key_kernel<<<gpred, kPredictThreads, 0, st>>>(P, s->x[cur.x], s->v[cur.v], s->p[cur.p], s->fext, wcur,
                                                            s->keys[0], s->keys[np % 2], s->table_n, s->cell_start,
                                                            s->hist, np, s->err, s->dfr_count);
     PROF_END();

@@ -76,6 +76,7 @@ struct SortScratch {
     uint32_t max_tiles;
     uint32_t spin_limit = kSpinLimit;   // polls of one look-back wait before it gives up
     uint32_t hold = 0;                  // 1: the first tile of each pass never publishes (tests)
+    uint32_t* done = nullptr;           // given to a sort's last pass: its last tile zeroes hist and this word
     uint32_t key_bits = 32;             // only bits [0, key_bits) order the keys
 };
 
@@ -99,6 +100,28 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
+}
+
+// Count a key's digits into the block's histograms sh[pass][digit].  All lanes of a warp call it; `valid`
+// lanes count.  kCoherent: neighbouring keys mostly share their upper digits (Morton keys of particles
+// in last frame's order), where 32 lanes adding to one word took 32 turns: the lanes that hold the first
+// lane's digit are counted with one add.
+template <bool kCoherent>
+__device__ __forceinline__ void count_digits(uint32_t* sh, uint32_t key, bool valid, int npasses, uint32_t key_bits) {
+    const uint32_t any = __ballot_sync(0xffffffffu, valid);
+    if (any == 0u) return;
+    const uint32_t lane = threadIdx.x & 31u, lead = (uint32_t)__ffs(any) - 1u;
+    for (int ps = 0; ps < npasses; ++ps) {
+        const uint32_t d = sort_digit(key, ps, key_bits);
+        if (kCoherent && ps > 0) {
+            const uint32_t d0 = __shfl_sync(0xffffffffu, d, lead);
+            const uint32_t same = __ballot_sync(0xffffffffu, valid && d == d0);
+            if (lane == lead) atomicAdd(&sh[ps * kRadix + d0], (uint32_t)__popc(same));
+            else if (valid && d != d0) atomicAdd(&sh[ps * kRadix + d], 1u);
+        } else if (valid) {
+            atomicAdd(&sh[ps * kRadix + d], 1u);
+        }
+    }
 }
 
 // One LSD pass over digit `pass` (bits 8*pass .. 8*pass+7).  kFirst: values are the
@@ -238,6 +261,15 @@ onesweep_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin
         if (o < n) {            // always true unless a look-back wait gave up (error word set)
             kout[o] = kk;
             vout[o] = s_vals[i];
+        }
+    }
+    if (S.done) {   // every tile has read its counts: the last one leaves them zero for the next sort
+        __syncthreads();
+        if (tid == 0) s_tile = atomicAdd(S.done, 1u);
+        __syncthreads();
+        if (s_tile == gridDim.x - 1) {
+            for (int b = tid; b < kMaxPasses * kRadix; b += kThreads) S.hist[b] = 0u;
+            if (tid == 0) *S.done = 0u;
         }
     }
 }

@@ -107,3 +107,18 @@ def test_noalloc_sort_at_the_edges_of_its_tile_sizes(need_gpu, pbd, n):
     k, p = _sort_noalloc(pbd, keys, key_bits=21)
     assert np.array_equal(p, order.astype(np.uint32)) and np.array_equal(k, keys[order])
     assert pbd.lib().pbd_sort_noalloc_status(None) == pbd.OK
+
+
+@pytest.mark.parametrize("offset,n", [(0, 4099), (1, 4099), (2, 7), (3, 300001)])
+def test_noalloc_sort_of_keys_at_any_word(need_gpu, pbd, offset, n):
+    # the counting pass reads four keys at a time only from a 16-byte boundary; two sorts in a row, the
+    # second finds the counts the first one's last tile left zero
+    import torch
+    keys = np.random.default_rng(offset).integers(0, 1 << 21, size=n + offset, dtype=np.uint64).astype(np.uint32)
+    d = torch.tensor(keys.view(np.int32), device="cuda")[offset:]
+    out, perm = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+    order = np.argsort(keys[offset:], kind="stable")
+    for _ in range(2):
+        pbd.check(pbd.lib().pbd_sort_keys_noalloc(d.data_ptr(), out.data_ptr(), perm.data_ptr(), n, 21, None))
+        assert pbd.lib().pbd_sort_noalloc_status(None) == pbd.OK
+        assert np.array_equal(perm.cpu().numpy().view(np.uint32), order.astype(np.uint32))
