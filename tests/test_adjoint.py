@@ -582,3 +582,30 @@ def test_gpu_adjoint_everything_at_once(need_gpu, pbd, scenes, adj):
     assert abs(gr - rr) <= 1e-2 * abs(rr) and abs(ge - re) <= 1e-2 * abs(re), (gr, rr, ge, re)
     for k in ("x", "v", "p", "ids"):
         assert np.array_equal(fin[k], after[k]), k
+
+
+@pytest.mark.gpu
+def test_gpu_recorded_segments_are_not_mixed_up(need_gpu, pbd, scenes):
+    """rollouts on one simulation with the particles set anew for each: the recorded segments are reused
+    only where the workspace is laid out the same (frames, checkpoint distance, particles, masses), so
+    every gradient has the bits a fresh simulation gives"""
+    prm, pos, vel, w = adjoint_scene(pbd, scenes, viscosity=0.01)
+    half = len(pos) // 2
+    m = np.where(np.arange(len(pos)) % 5 == 0, 0.0, 1.0).astype(np.float32)
+    g = np.zeros((len(pos), 4), np.float32)
+    g[:, :3] = w
+    sim = pbd.Sim(prm, len(pos))
+    for frames, every, n, mass in ((6, 2, len(pos), False), (4, 2, len(pos), False), (6, 2, len(pos), False), (6, 3, len(pos), False),
+                                   (4, 2, half, False), (4, 2, len(pos), False), (4, 2, len(pos), True), (4, 2, len(pos), True)):
+        got = []
+        for s in (sim, pbd.Sim(prm, len(pos))):
+            s.clear()
+            if mass:
+                s.add_particles_mass(pos[:n], vel[:n], m[:n])
+            else:
+                s.add_particles(pos[:n], vel[:n])
+            s.adjoint_forward(frames, every)
+            got.append(s.adjoint_backward(g[:n]))
+        for a, b in zip(*got):
+            assert np.array_equal(a, b), (frames, every, n, mass)
+    sim.close()
