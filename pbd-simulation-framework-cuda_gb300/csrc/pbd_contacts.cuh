@@ -23,7 +23,7 @@
 namespace pbd {
 
 struct ContactStore {
-    uint32_t* list;      // M x stride partner indices, slot-major
+    uint32_t* list;      // partner indices, four entries side by side as in a full list (full_at)
     uint32_t* count;     // entries per particle
     uint32_t* solved;    // ceil(M / 32) x stride words: bit k of particle i = constraint (i, k) solved
     unsigned long long* best;   // each particle's chosen constraint key in this batch (0: none)
@@ -34,12 +34,9 @@ struct ContactStore {
     uint32_t M;
 };
 
-// Lanes per particle in the claim pass: entry k of a list goes to lane k mod kClaimLanes.  Lists
-// longer than kClaimLong (up to M = 512 entries where the cell-end quirk stretches a cell's
-// range, against ~26 on average) go to a whole warp in the pass's leading blocks instead, so they
-// do not hold up the pass.
-constexpr uint32_t kClaimLanes = 1;
-constexpr uint32_t kClaimBatch = 4;    // entries per lane per step
+// Lists longer than kClaimLong (up to M = 512 entries where the cell-end quirk stretches a cell's
+// range, against ~26 on average) go to a whole warp in the claim pass's leading blocks, so they do not
+// hold up the pass.
 constexpr uint32_t kClaimLong = 64;
 constexpr uint32_t kClaimCoopBlocks = 4;
 
@@ -87,18 +84,32 @@ __device__ __forceinline__ bool contact_geometry(const DevParams& P, const float
     return true;
 }
 
+__device__ __forceinline__ NbList contact_entries(const ContactStore& C) { return NbList{C.list, nullptr, C.stride, C.M}; }
+
 // Every entry of particle i's list, in list order, up to the cap M.
 struct ContactListVisit {
     struct Contrib { uint32_t j; };
-    uint32_t* list;
-    uint32_t stride, i, n = 0;
-    __device__ ContactListVisit(uint32_t* l, uint32_t s, uint32_t i_) : list(l), stride(s), i(i_) {}
+    NbList L;
+    uint32_t i, n = 0;
+    __device__ ContactListVisit(const ContactStore& C, uint32_t i_) : L(contact_entries(C)), i(i_) {}
     __device__ static Contrib zero() { return Contrib{0u}; }
     __device__ static bool effective(const Contrib&) { return true; }
     __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_u(c.j, k, width)}; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) const { return Contrib{j}; }
-    __device__ __forceinline__ void add(const Contrib& c, bool) { list[(size_t)n * stride + i] = c.j; ++n; }
+    __device__ __forceinline__ void add(const Contrib& c, bool) { *full_at(L, i, n) = c.j; ++n; }
+};
+
+// The same by one thread, four entries a store.
+struct ContactWriteVisit {
+    struct Contrib { uint32_t j; };
+    FullWriter out;
+    __device__ ContactWriteVisit(const ContactStore& C, uint32_t i) : out(contact_entries(C), i) {}
+    __device__ static Contrib zero() { return Contrib{0u}; }
+    __device__ static bool effective(const Contrib&) { return true; }
+    __device__ __forceinline__ void end_contacts(uint32_t) {}
+    __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) const { return Contrib{j}; }
+    __device__ __forceinline__ void add(const Contrib& c, bool) { out.push(c.j); }
 };
 
 __device__ __forceinline__ void contact_list_done(const ContactStore& C, uint32_t i, uint32_t n) {
@@ -119,117 +130,144 @@ contact_list_kernel(DevParams P, const float4* __restrict__ pa, const uint32_t* 
     __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < P.N) {
-        ContactListVisit vis(C.list, C.stride, i);
+        ContactWriteVisit vis(C, i);
         bool deferred = false;
         walk_seq(P, scene_ctx(P, i), i, pa[i], pa, cs, ce, vis, true, &deferred);
         if (deferred) left[atomicAdd(&nleft, 1u)] = i;
-        else contact_list_done(C, i, vis.n);
+        else {
+            vis.out.flush();
+            contact_list_done(C, i, vis.out.n);
+        }
     }
     __syncthreads();
     const uint32_t nl = nleft;
     for (uint32_t k = threadIdx.x >> 5; k < nl; k += blockDim.x >> 5) {
         const uint32_t q = left[k];
-        ContactListVisit vis(C.list, C.stride, q);
+        ContactListVisit vis(C, q);
         walk_coop(P, scene_ctx(P, q), q, pa[q], pa, cs, ce, vis);
         if (lane_id() == 0) contact_list_done(C, q, vis.n);
     }
 }
 
-// Offer the keys of particle i's pending overlapping constraints k = t, t + L, t + 2L, ... (lane t
-// of L lanes) to both particles; returns the highest key offered to i itself.  Each lane takes B
-// entries per step (index loads, then position loads, in flight together, the next step's
-// indices loaded meanwhile); a cheap squared-distance test (a superset of the overlap test,
-// |r| < diameter) skips most entries before the exact one.
-template <uint32_t L, uint32_t B>
+// Offer constraint (i, k)'s key to its partner j and to `own`, i's own best, when the contact acts.
+__device__ __forceinline__ void offer(const DevParams& P, const ContactStore& C, const float* __restrict__ w, uint32_t i,
+                                      uint32_t k, uint32_t j, const float4& pi, const float4& pj, unsigned long long& own) {
+    if (!contact_acts(P, w, i, j, contact_len(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z))) return;
+    const uint32_t c = i * C.M + k;
+    const unsigned long long key = ((unsigned long long)lowbias32(c + 1u) << 32) | c;
+    own = key > own ? key : own;          // i's own offers: one atomic per particle
+    atomicMax(C.best + j, key);           // the partner's (no read first: fire and forget)
+}
+
+// One thread offers the keys of particle i's pending overlapping constraints (n of them at most) and
+// returns the highest.  32 entries at a time: first only the squared distances (a superset of the
+// overlap test, |r| < diameter), four entries per index load, into a mask without the solved ones;
+// then the exact test, key and atomic for the entries in the mask.  About 12% of the entries compete:
+// with the test of every entry followed by its offer, some lane of a warp took almost every offer
+// (2,400 warp instructions per 32 particles against 1,150).
 __device__ __forceinline__ unsigned long long claim_entries(const DevParams& P, const ContactStore& C,
                                                             const float4* __restrict__ p, const float* __restrict__ w,
-                                                            uint32_t i, uint32_t t, uint32_t n) {
-    constexpr uint32_t kStep = B * L;
-    static_assert((kStep <= 32u && (32u % kStep) == 0u) || (L == 32u && B == 2u), "a step's solved words");
+                                                            uint32_t i, uint32_t n) {
+    const NbList L = contact_entries(C);
     const float4 pi = p[i];
     const float reach2 = P.d * P.d * 1.0001f;
-    const uint32_t* __restrict__ e = C.list + i;
     unsigned long long own = 0ull;
-    uint32_t word[B];   // solved bits of the word holding each of this step's entries
-    uint32_t jn[B];     // the next step's entries, loaded while this step is tested
-#pragma unroll
-    for (uint32_t b = 0; b < B; ++b) {
-        word[b] = 0u;
-        jn[b] = (t + b * L < n) ? __ldcs(e + (size_t)(t + b * L) * C.stride) : i;
-    }
+    for (uint32_t k0 = 0; k0 < n; k0 += 32u) {
+        const uint32_t solved = C.solved[(size_t)(k0 >> 5) * C.stride + i];
+        const uint32_t m = min(n - k0, 32u);
+        const uint4* e = reinterpret_cast<const uint4*>(L.list) + (size_t)(k0 >> 2) * L.stride + i;
+        uint4 q = __ldg(e);
+        uint32_t mask = 0;
 #pragma unroll 1
-    for (uint32_t k0 = 0; k0 < n; k0 += kStep) {
-        if (kStep <= 32u) {                      // a step stays inside one 32-entry word
-            if ((k0 & 31u) == 0u) {
-                const uint32_t v = C.solved[(size_t)(k0 >> 5) * C.stride + i];
+        for (uint32_t kb = 0; kb < m; kb += 4u) {
+            const uint32_t j[4] = {q.x, kb + 1u < m ? q.y : i, kb + 2u < m ? q.z : i, kb + 3u < m ? q.w : i};
+            float4 pj[4];
 #pragma unroll
-                for (uint32_t b = 0; b < B; ++b) word[b] = v;
+            for (uint32_t b = 0; b < 4u; ++b) pj[b] = __ldg(p + j[b]);
+            e += L.stride;
+            if (kb + 4u < m) q = __ldg(e);
+            uint32_t four = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < 4u; ++b) {
+                const float dx = pj[b].x - pi.x, dy = pj[b].y - pi.y, dz = pj[b].z - pi.z;
+                if (kb + b < m && dist2(dx, dy, dz) < reach2) four |= 1u << b;
             }
-        } else {                                 // 64 entries a step: entry b of a lane is in word k0/32 + b
-#pragma unroll
-            for (uint32_t b = 0; b < B; ++b)
-                word[b] = (k0 + b * 32u < n) ? C.solved[(size_t)((k0 >> 5) + b) * C.stride + i] : 0u;
+            mask |= four << kb;
         }
-        uint32_t j[B];
-        float4 pj[B];
-#pragma unroll
-        for (uint32_t b = 0; b < B; ++b) j[b] = jn[b];
-#pragma unroll
-        for (uint32_t b = 0; b < B; ++b) pj[b] = (k0 + t + b * L < n) ? __ldg(p + j[b]) : pi;
-#pragma unroll
-        for (uint32_t b = 0; b < B; ++b) {
-            const uint32_t k = k0 + kStep + t + b * L;
-            jn[b] = (k < n) ? __ldcs(e + (size_t)k * C.stride) : i;
-        }
-#pragma unroll
-        for (uint32_t b = 0; b < B; ++b) {
-            const uint32_t k = k0 + t + b * L;
-            if (k >= n || ((word[b] >> (k & 31u)) & 1u)) continue;
-            const float dx = pj[b].x - pi.x, dy = pj[b].y - pi.y, dz = pj[b].z - pi.z;
-            if (!(dx * dx + dy * dy + dz * dz < reach2)) continue;
-            if (!contact_acts(P, w, i, j[b], contact_len(dx, dy, dz))) continue;
-            const uint32_t c = i * C.M + k;
-            const unsigned long long key = ((unsigned long long)lowbias32(c + 1u) << 32) | c;
-            own = key > own ? key : own;          // i's own offers: one atomic per particle
-            atomicMax(C.best + j[b], key);        // the partner's (no read first: fire and forget)
+        mask &= ~solved;
+        uint32_t k = k0 + (uint32_t)__ffs(mask) - 1u;
+        uint32_t j = mask ? __ldg(full_at(L, i, k)) : i;
+        while (mask) {   // the next entry's index in flight
+            mask &= mask - 1u;
+            const uint32_t kn = k0 + (uint32_t)__ffs(mask) - 1u;
+            const float4 pj = __ldg(p + j);
+            const uint32_t jn = mask ? __ldg(full_at(L, i, kn)) : i;
+            offer(P, C, w, i, k, j, pi, pj, own);
+            k = kn;
+            j = jn;
         }
     }
     return own;
 }
 
-// Maximum over groups of L lanes (L a power of two dividing 32); every lane of the warp calls it.
-template <uint32_t L>
-__device__ __forceinline__ unsigned long long group_max(unsigned long long v) {
+// The same for a long list by the 32 lanes of a warp (lane t takes entries t, t + 32, ...): a lane's
+// highest own offer.
+__device__ __forceinline__ unsigned long long claim_entries_warp(const DevParams& P, const ContactStore& C,
+                                                                 const float4* __restrict__ p, const float* __restrict__ w,
+                                                                 uint32_t i, uint32_t t, uint32_t n) {
+    const NbList L = contact_entries(C);
+    const float4 pi = p[i];
+    const float reach2 = P.d * P.d * 1.0001f;
+    unsigned long long own = 0ull;
+    for (uint32_t k0 = 0; k0 < n; k0 += 64u) {
+        uint32_t j[2], solved[2];
+        float4 pj[2];
 #pragma unroll
-    for (uint32_t s = 1; s < L; s <<= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, s);
-        v = o > v ? o : v;
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = k0 + b * 32u + t;
+            j[b] = k < n ? __ldg(full_at(L, i, k)) : i;
+            solved[b] = k < n ? C.solved[(size_t)(k >> 5) * C.stride + i] : kFullMask;
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) pj[b] = __ldg(p + j[b]);
+#pragma unroll
+        for (uint32_t b = 0; b < 2u; ++b) {
+            const uint32_t k = k0 + b * 32u + t;
+            if ((solved[b] >> t) & 1u) continue;
+            if (dist2(pj[b].x - pi.x, pj[b].y - pi.y, pj[b].z - pi.z) < reach2) offer(P, C, w, i, k, j[b], pi, pj[b], own);
+        }
     }
-    return v;
+    return own;
 }
 
-// Each pending overlapping constraint offers its key to both of its particles; the particle's
-// own offers are reduced over its lanes into one atomic.  The first kClaimCoopBlocks blocks take
-// the long lists, a warp each; the others take every other particle, kClaimLanes lanes each.
-__global__ void __launch_bounds__(256, 6)
+// Each pending overlapping constraint offers its key to both of its particles.  The first
+// kClaimCoopBlocks blocks take the long lists, a warp each; the others take every other particle, a
+// thread each.  Four blocks of 256 per SM, whose positions and lists the L1 holds better than more
+// blocks' (a stabilization pass of 16 batches with 262,144 particles: 467 us; 5 and 6 blocks 500, 8 524;
+// eight entries per step instead of four 488).
+__global__ void __launch_bounds__(256, 4)
 contact_claim_kernel(DevParams P, ContactStore C, const float4* __restrict__ p, const float* __restrict__ w) {
     if (blockIdx.x < kClaimCoopBlocks) {
         const uint32_t nl = *C.long_count;
         const uint32_t wpb = blockDim.x >> 5, lane = threadIdx.x & 31u;
         for (uint32_t q = blockIdx.x * wpb + (threadIdx.x >> 5); q < nl; q += kClaimCoopBlocks * wpb) {
             const uint32_t i = C.long_items[q];
-            const unsigned long long own = group_max<32>(claim_entries<32, 2>(P, C, p, w, i, lane, C.count[i]));
+            unsigned long long own = claim_entries_warp(P, C, p, w, i, lane, C.count[i]);
+#pragma unroll
+            for (uint32_t s = 1; s < 32u; s <<= 1) {
+                const unsigned long long o = __shfl_xor_sync(kFullMask, own, s);
+                own = o > own ? o : own;
+            }
             if (lane == 0 && own) atomicMax(C.best + i, own);
         }
         return;
     }
-    constexpr uint32_t L = kClaimLanes;
-    const uint32_t i = (blockIdx.x - kClaimCoopBlocks) * (blockDim.x / L) + threadIdx.x / L, t = threadIdx.x % L;
-    uint32_t n = i < P.N ? C.count[i] : 0u;
-    if (n > kClaimLong) n = 0u;                  // a long list: a leading block's warp takes it
-    // no early exit: the lanes meet in the shuffles below
-    const unsigned long long own = group_max<L>(n ? claim_entries<L, kClaimBatch>(P, C, p, w, i, t, n) : 0ull);
-    if (t == 0 && own) atomicMax(C.best + i, own);
+    const uint32_t i = (blockIdx.x - kClaimCoopBlocks) * blockDim.x + threadIdx.x;
+    if (i >= P.N) return;
+    const uint32_t n = C.count[i];
+    if (n > kClaimLong) return;                  // a long list: a leading block's warp takes it
+    const unsigned long long own = claim_entries(P, C, p, w, i, n);
+    if (own) atomicMax(C.best + i, own);
 }
 
 // A constraint both of whose particles took it is solved by its partner's thread: the key holds

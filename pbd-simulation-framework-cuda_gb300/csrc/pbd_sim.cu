@@ -579,7 +579,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 for (uint32_t b = 0; b < prm.max_collision_batches; ++b, ++nbatch) {
                     C.best = keys[nbatch & 1u];
                     C.best_next = keys[(nbatch + 1u) & 1u];
-                    contact_claim_kernel<<<kClaimCoopBlocks + div_up(N, kThreadsParticle / kClaimLanes), kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], wf);
+                    contact_claim_kernel<<<kClaimCoopBlocks + div_up(N, kThreadsParticle), kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], wf);
                     contact_solve_kernel<<<div_up(N, kThreadsParticle), kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], s->x[cur.x], wf);
                     nl += 2;
                 }
@@ -850,7 +850,8 @@ int ensure_contacts(pbd_sim* s) {
         set_error("collisionType 1: capacity x maxNeighboursPerParticle must stay below 2^32");
         return PBD_ERR_UNSUPPORTED;
     }
-    const size_t need = ((C * M * 4 + 255) & ~size_t(255)) + ((C * 4 + 255) & ~size_t(255)) +
+    const size_t slots = full_slots((uint32_t)M);
+    const size_t need = ((C * slots * 4 + 255) & ~size_t(255)) + ((C * 4 + 255) & ~size_t(255)) +
                         ((C * W * 4 + 255) & ~size_t(255)) + C * 16 + ((C * 4 + 255) & ~size_t(255)) + 256 + 256;
     if (s->ct_arena && s->ct_bytes >= need && s->ct.M == M) return PBD_OK;
     if (s->ct_arena) {
@@ -864,7 +865,7 @@ int ensure_contacts(pbd_sim* s) {
     s->ct_bytes = need;
     char* c = static_cast<char*>(s->ct_arena);
     auto take = [&](size_t b) { char* r = c; c += (b + 255) & ~size_t(255); return r; };
-    s->ct.list = (uint32_t*)take(C * M * 4);
+    s->ct.list = (uint32_t*)take(C * slots * 4);
     s->ct.count = (uint32_t*)take(C * 4);
     s->ct.solved = (uint32_t*)take(C * W * 4);
     s->ct.best = (unsigned long long*)take(C * 16);   // two buffers of C keys
