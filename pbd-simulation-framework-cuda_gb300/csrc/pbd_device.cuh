@@ -63,6 +63,9 @@ struct DevParams {
     // an adjoint's taped frame: the vorticity pass also stores each particle's eta (its
     // sum_j |omega_j - omega_i| / (p_j - p_i + 1e-8)) here; null in every other frame
     float4* eta_tape;
+    // every predicted position's w is 1 for the whole frame: applyForces sets it (Forces.h:94), and with
+    // collisionType 0 nothing but a 0 is ever added to it (collisionType 1 writes 0 there)
+    uint32_t unit_w;
 };
 
 // The scene a particle belongs to, as the walk and the per-scene constants see it.

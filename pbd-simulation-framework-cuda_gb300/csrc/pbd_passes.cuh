@@ -1001,14 +1001,17 @@ __device__ __forceinline__ void walk_warp(const DevParams& P, const SceneCtx& S,
 // ======================================================================================
 // computeLambda (Density.h:48-93)
 // ======================================================================================
-struct LambdaVisit {
+// kUnitW: every p.w is 1 (DevParams::unit_w), so the entries' w difference is 0: it adds nothing to |r|_4
+// and nothing to the gradient sum's w, and is left out.
+template <bool kUnitW>
+struct LambdaVisitT {
     // a = W, b = |grad|^2 = s^2 |r|^2; the gradient sum takes s * r by explicit FMAs, so every
     // walker rounds it the same way
     struct Contrib { float a, b, s, rx, ry, rz, rw; uint32_t near; };
     const DevParams& P;
     float4 pi;
     float A = 0.f, B = 0.f, Cx = 0.f, Cy = 0.f, Cz = 0.f, Cw = 0.f;
-    __device__ LambdaVisit(const DevParams& P_, float4 pi_) : P(P_), pi(pi_) {}
+    __device__ LambdaVisitT(const DevParams& P_, float4 pi_) : P(P_), pi(pi_) {}
     __device__ void reset() { A = B = Cx = Cy = Cz = Cw = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
@@ -1018,10 +1021,10 @@ struct LambdaVisit {
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
+        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = kUnitW ? 0.0f : pi.w - pj.w;
         const float r2 = dist2(rx, ry, rz);
         const float dist = sqrt_fast(r2);
-        const float r2w = __fmaf_rn(rw, rw, r2);
+        const float r2w = kUnitW ? r2 : __fmaf_rn(rw, rw, r2);
         const float s = spiky_scale(P, dist, r2w);
         // beyond the cut every kernel is exactly 0: add() leaves the sums alone
         return Contrib{poly6(P, dist), __fmul_rn(__fmul_rn(s, s), r2w), s, rx, ry, rz, rw, r2 >= P.cut2 ? 0u : 1u};
@@ -1030,16 +1033,19 @@ struct LambdaVisit {
         if (!c.near) return;
         A = __fadd_rn(A, c.a); B = __fadd_rn(B, c.b);
         Cx = __fmaf_rn(c.s, c.rx, Cx); Cy = __fmaf_rn(c.s, c.ry, Cy);
-        Cz = __fmaf_rn(c.s, c.rz, Cz); Cw = __fmaf_rn(c.s, c.rw, Cw);
+        Cz = __fmaf_rn(c.s, c.rz, Cz);
+        if constexpr (!kUnitW) Cw = __fmaf_rn(c.s, c.rw, Cw);
     }
     // add() when `live`, as predicated instructions: as a branch the compiler moves the contribution's
     // arithmetic into it, and the entries of a group run one after the other
     __device__ __forceinline__ void add_if(bool live, const Contrib& c) {
-        asm("{ .reg .pred q; setp.ne.u32 q, %6, 0; @q add.rn.f32 %0, %0, %7; @q add.rn.f32 %1, %1, %8;"
-            " @q fma.rn.f32 %2, %9, %10, %2; @q fma.rn.f32 %3, %9, %11, %3; @q fma.rn.f32 %4, %9, %12, %4;"
-            " @q fma.rn.f32 %5, %9, %13, %5; }"
-            : "+f"(A), "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz), "+f"(Cw)
-            : "r"((live && c.near) ? 1u : 0u), "f"(c.a), "f"(c.b), "f"(c.s), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
+        asm("{ .reg .pred q; setp.ne.u32 q, %5, 0; @q add.rn.f32 %0, %0, %6; @q add.rn.f32 %1, %1, %7;"
+            " @q fma.rn.f32 %2, %8, %9, %2; @q fma.rn.f32 %3, %8, %10, %3; @q fma.rn.f32 %4, %8, %11, %4; }"
+            : "+f"(A), "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz)
+            : "r"((live && c.near) ? 1u : 0u), "f"(c.a), "f"(c.b), "f"(c.s), "f"(c.rx), "f"(c.ry), "f"(c.rz));
+        if constexpr (!kUnitW)
+            asm("{ .reg .pred q; setp.ne.u32 q, %1, 0; @q fma.rn.f32 %0, %2, %3, %0; }"
+                : "+f"(Cw) : "r"((live && c.near) ? 1u : 0u), "f"(c.s), "f"(c.rw));
     }
     // walk_group_sums: A, B, C from the rows a, b, s, r
     static constexpr int kRows = 7, kSums = 6;
@@ -1067,20 +1073,22 @@ struct LambdaVisit {
         return __fdiv_rn(-a, __fadd_rn(__fadd_rn(b, c), P.lambda_eps));
     }
 };
+using LambdaVisit = LambdaVisitT<false>;
 
+template <bool kUnitW>
 __global__ void __launch_bounds__(256, 4)   // 5 (48 registers) spills: 622 -> 649 us on the 1M dense frame
 lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
               const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux,
-              NbList L, NbList F, DeferList DF, DeferList DN, uint32_t long_slots) {
+              NbList L, NbList F, DeferList DF, DeferList DN, uint32_t long_slots, float4* __restrict__ pl) {
     // walks the cells; L.list: record the near lists for the delta pass that follows (the
-    // particles left without one noted in DN); F.list: store the full lists (the frame's first
+    // particles left without one noted in DN); pl: also leave (p, lambda) there; F.list: store the full lists (the frame's first
     // lambda pass; the particles left without one noted in DF and finished by lambda_long_kernel,
     // which stores the lists of the first long_slots of them)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
-    LambdaVisit vis(P, pi);
+    LambdaVisitT<kUnitW> vis(P, pi);
     bool deferred = false;
     if (F.list) {
         // the walk stores the full list (indices only), the filter the near list; the sums then
@@ -1112,7 +1120,9 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
         else if (listed) walk_full<true>(F, i, fm, p, vis);
         else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
-        lambda[i] = vis.finish(S.rho0);
+        const float li = vis.finish(S.rho0);
+            lambda[i] = li;
+            if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
         if (aux) vis.store_aux(aux, P.N, i);
         return;
     } else if (L.list) {
@@ -1125,7 +1135,9 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         if (!deferred) {
             if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
             else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
-            lambda[i] = vis.finish(S.rho0);
+            const float li = vis.finish(S.rho0);
+            lambda[i] = li;
+            if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
             if (aux) vis.store_aux(aux, P.N, i);
             return;
         }
@@ -1137,7 +1149,9 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         vis.reset();
         walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
     }
-    lambda[i] = vis.finish(S.rho0);
+    const float li = vis.finish(S.rho0);
+            lambda[i] = li;
+            if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
     if (aux) vis.store_aux(aux, P.N, i);
 }
 
@@ -1147,7 +1161,8 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
 __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                                             float* __restrict__ lambda, float4* __restrict__ aux, uint32_t i,
-                                            const LongLists& LL, const NbList& F, const NbList& L, const DeferList& DN) {
+                                            const LongLists& LL, const NbList& F, const NbList& L, const DeferList& DN,
+                                            float4* __restrict__ pl) {
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
     LambdaVisit vis(P, pi);
@@ -1163,7 +1178,9 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
     if (lm != kListOff) walk_group<32>([&](uint32_t k) { return L.list + (size_t)k * L.stride + i; }, lm & 0xFFu, lm >> 8, i, p, vis);
     else walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) {
-        lambda[i] = vis.finish(S.rho0);
+        const float li = vis.finish(S.rho0);
+        lambda[i] = li;
+        if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
         if (aux) vis.store_aux(aux, P.N, i);
     }
 }
@@ -1171,7 +1188,7 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
 __global__ void __launch_bounds__(128)
 lambda_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
                    const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux) {
-    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LongLists{}, NbList{}, NbList{}, DeferList{}); });
+    for_each_deferred(D, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LongLists{}, NbList{}, NbList{}, DeferList{}, nullptr); });
 }
 
 // After lambda_kernel stored the full lists: the particles left without one (the set DF), a warp
@@ -1180,7 +1197,7 @@ __global__ void __launch_bounds__(128)
 lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
                    const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList DF, float4* __restrict__ aux,
                    const __grid_constant__ LongLists LL, const __grid_constant__ NbList F, const __grid_constant__ NbList L,
-                   const __grid_constant__ DeferList DN) {
+                   const __grid_constant__ DeferList DN, float4* __restrict__ pl) {
     const uint32_t n = min(*DF.count, DF.cap);
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < n; q += warps) {
@@ -1191,7 +1208,7 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
             if (lane_id() == 0) LL.meta[q] = m;
             __syncwarp();
         }
-        coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN);
+        coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN, pl);
     }
 }
 
@@ -1199,12 +1216,14 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
 // The particles without a full list (the set C) are walked by the leading blocks; the ones left
 // without a near list are noted in DN for the delta pass.  Kept apart from lambda_kernel so that
 // its register budget is the list walk's alone.
+template <bool kUnitW>
 __global__ void __launch_bounds__(256, 5)
 lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
-                   CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+                   CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL,
+                   float4* __restrict__ pl) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN, pl); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
@@ -1213,7 +1232,7 @@ lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict
     if (fm & kListOff) return;   // in the set C
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
-    LambdaVisit vis(P, pi);
+    LambdaVisitT<kUnitW> vis(P, pi);
     const uint32_t lm = L.list ? filter_list(F, fm, L, i, pi, P.cut2, p) : kListOff;
     if (L.list) {
         L.meta[i] = lm;
@@ -1221,7 +1240,9 @@ lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict
     }
     if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
     else walk_full(F, i, fm, p, vis);
-    lambda[i] = vis.finish(S.rho0);
+    const float li = vis.finish(S.rho0);
+    lambda[i] = li;
+    if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
     if (aux) vis.store_aux(aux, P.N, i);
 }
 
@@ -1274,7 +1295,7 @@ lambda_list_group_kernel(const __grid_constant__ DevParams P, const float4* __re
                          CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L,
                          const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, aux, i, LL, F, L, DN, nullptr); });
         return;
     }
     const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
@@ -1318,8 +1339,10 @@ enum DeltaMode : uint32_t {
 
 // What a delta visitor knows at compile time: kDeltaAny nothing (the mode, the inverse masses, the
 // exponent and far_pairs_zero are looked at for every entry); kDeltaPlain a pass with the density
-// part, the contacts, config.txt's nSCorr = 4, far pairs exactly zero and no inverse masses;
-// kDeltaMass the same with inverse masses.  The arithmetic is the same.
+// part, the contacts, config.txt's nSCorr = 4, far pairs exactly zero, every p.w 1 (LambdaVisitT's
+// kUnitW) and no inverse masses; kDeltaMass the same with inverse masses.  These two take a neighbour's
+// lambda from the w of its position (the lambda pass's pl), one gather per entry instead of two.  The
+// arithmetic is the same.
 enum DeltaKnown : uint32_t { kDeltaAny = 0, kDeltaPlain = 1, kDeltaMass = 2 };
 
 template <uint32_t kKnown>
@@ -1351,16 +1374,17 @@ struct DeltaVisitT {
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float;   // lambda_j
-    __device__ __forceinline__ float fetch(uint32_t j) const { return do_delta ? __ldg(lambda + j) : 0.f; }
+    __device__ __forceinline__ float fetch(uint32_t j) const { return (!kKnow && do_delta) ? __ldg(lambda + j) : 0.f; }
     __device__ __forceinline__ bool masses() const { return kKnown == kDeltaPlain ? false : (kKnown == kDeltaMass ? true : w != nullptr); }
-    __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, float lj, bool contact) const {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
+    __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, float lj_, bool contact) const {
+        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = kKnow ? 0.0f : pi.w - pj.w;
+        const float lj = kKnow ? pj.w : lj_;
         const float r2 = dist2(rx, ry, rz);
         const float dist = sqrt_fast(r2);
         const bool near = all_pairs || !(r2 >= P.cut2);
         Contrib c{0.f, rx, ry, rz, rw, 0.f, 0u};
         if (do_delta) {
-            const float s = spiky_scale(P, dist, __fmaf_rn(rw, rw, r2));
+            const float s = spiky_scale(P, dist, kKnow ? r2 : __fmaf_rn(rw, rw, r2));
             const float q = __fmul_rn(poly6(P, dist), P.inv_wq);
             const float sc = __fmul_rn(-P.k_scorr, kKnow ? ((q * q) * q) * q : powi(q, P.n_scorr));
             c.coef = __fmul_rn(__fadd_rn(__fadd_rn(li, lj), sc), s);
@@ -1388,7 +1412,8 @@ struct DeltaVisitT {
     __device__ __forceinline__ void add(const Contrib& c, bool) {
         if (c.flags & 1u) {
             ax = __fmaf_rn(c.coef, c.rx, ax); ay = __fmaf_rn(c.coef, c.ry, ay);
-            az = __fmaf_rn(c.coef, c.rz, az); aw = __fmaf_rn(c.coef, c.rw, aw);
+            az = __fmaf_rn(c.coef, c.rz, az);
+            if constexpr (!kKnow) aw = __fmaf_rn(c.coef, c.rw, aw);
         }
         if (c.flags & 2u) {
             pacc.x = __fmaf_rn(-c.rx, c.t, pacc.x); xacc.x = __fmaf_rn(-c.rx, c.t, xacc.x);
@@ -1398,10 +1423,12 @@ struct DeltaVisitT {
     }
     // the density part predicated (LambdaVisit::add_if); contacts are rare enough for a branch
     __device__ __forceinline__ void add_if(bool live, const Contrib& c) {
-        asm("{ .reg .pred q; setp.ne.u32 q, %4, 0; @q fma.rn.f32 %0, %5, %6, %0; @q fma.rn.f32 %1, %5, %7, %1;"
-            " @q fma.rn.f32 %2, %5, %8, %2; @q fma.rn.f32 %3, %5, %9, %3; }"
-            : "+f"(ax), "+f"(ay), "+f"(az), "+f"(aw)
-            : "r"((live && (c.flags & 1u)) ? 1u : 0u), "f"(c.coef), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
+        const uint32_t on = (live && (c.flags & 1u)) ? 1u : 0u;
+        asm("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q fma.rn.f32 %0, %4, %5, %0; @q fma.rn.f32 %1, %4, %6, %1;"
+            " @q fma.rn.f32 %2, %4, %7, %2; }"
+            : "+f"(ax), "+f"(ay), "+f"(az) : "r"(on), "f"(c.coef), "f"(c.rx), "f"(c.ry), "f"(c.rz));
+        if constexpr (!kKnow)
+            asm("{ .reg .pred q; setp.ne.u32 q, %1, 0; @q fma.rn.f32 %0, %2, %3, %0; }" : "+f"(aw) : "r"(on), "f"(c.coef), "f"(c.rw));
         if (live && (c.flags & 2u)) {
             Contrib k = c;
             k.flags = 2u;
@@ -1505,7 +1532,7 @@ delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const f
                   float4* __restrict__ pout, float4* __restrict__ x, float4* __restrict__ v,
                   const float* __restrict__ lambda, const float* __restrict__ w, float4* __restrict__ delta,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, CoopSet C, const __grid_constant__ NbList L, const __grid_constant__ NbList F,
-                  const __grid_constant__ LongLists LL) {
+                  const __grid_constant__ LongLists LL, const float4* __restrict__ pl) {
     const uint32_t mode = kMode ? kMode : mode_rt;
     if (blockIdx.x < C.blocks) {
         run_coop_set(C, [&](uint32_t i) { coop_delta(P, mode, pin, pa, pout, x, v, lambda, w, delta, cs, ce, i, LL, F); });
@@ -1515,14 +1542,25 @@ delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const f
     if (i >= P.N) return;
     const uint32_t meta = L.meta[i];
     if (meta & kListOff) return;
-    const float4 pi = pin[i];
+    float4 pi;
+    float li;
+    if constexpr (kKnown != kDeltaAny) {   // p.w is 1
+        pi = pl[i];
+        li = pi.w;
+        pi.w = 1.0f;
+    } else {
+        pi = pin[i];
+        li = (mode & kDoDelta) ? lambda[i] : 0.f;
+    }
     const bool need_x = (mode & (kDoCollide | kDoUpdate)) != 0;
     const float4 xi = need_x ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float li = (mode & kDoDelta) ? lambda[i] : 0.f;
     const SceneCtx S = scene_ctx(P, i);
     DeltaVisitT<kKnown> vis(P, lambda, w, pi, li, w ? w[i] : 1.0f, (mode & kDoDelta) != 0, (mode & kDoCollide) != 0, xi);
-    if constexpr (kFull) walk_full(L, i, meta, pin, vis);
-    else walk_near(L, i, meta, pin, vis);
+    const float4* pj = kKnown != kDeltaAny ? pl : pin;
+    if constexpr (kFull) walk_full(L, i, meta, pj, vis);
+    else walk_near(L, i, meta, pj, vis);
+    // the w of the sums: 0 times each coefficient, which is 0 until a coefficient is not finite
+    if constexpr (kKnown != kDeltaAny) vis.aw = 0.0f * vis.ax + 0.0f * vis.ay + 0.0f * vis.az;
     delta_finish(P, S.rho0, mode, i, vis, pout, x, v, delta);
 }
 
@@ -1578,13 +1616,14 @@ update_kernel(DevParams P, const float4* __restrict__ p, float4* __restrict__ x,
 // ======================================================================================
 // computeOmega (Density.h:232-269): omega_i = sum_j (v_j - v_i) x spiky(p_i, p_j)
 // ======================================================================================
-struct OmegaVisit {
+template <bool kUnitW>   // LambdaVisitT
+struct OmegaVisitT {
     struct Contrib { float ox, oy, oz; uint32_t near; };
     const DevParams& P;
     const float4* __restrict__ v;
     float4 pi, vi;
     float ox = 0.f, oy = 0.f, oz = 0.f;
-    __device__ OmegaVisit(const DevParams& P_, const float4* v_, float4 pi_, float4 vi_) : P(P_), v(v_), pi(pi_), vi(vi_) {}
+    __device__ OmegaVisitT(const DevParams& P_, const float4* v_, float4 pi_, float4 vi_) : P(P_), v(v_), pi(pi_), vi(vi_) {}
     __device__ void reset() { ox = oy = oz = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
@@ -1595,9 +1634,9 @@ struct OmegaVisit {
     using Extra = float4;   // v_j
     __device__ __forceinline__ float4 fetch(uint32_t j) const { return __ldg(v + j); }
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, const float4& vj, bool) const {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = pi.w - pj.w;
+        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = kUnitW ? 0.0f : pi.w - pj.w;
         const float r2 = dist2(rx, ry, rz);
-        const float s = spiky_scale(P, sqrt_fast(r2), __fmaf_rn(rw, rw, r2));
+        const float s = spiky_scale(P, sqrt_fast(r2), kUnitW ? r2 : __fmaf_rn(rw, rw, r2));
         const float wx = vj.x - vi.x, wy = vj.y - vi.y, wz = vj.z - vi.z;
         const float gx = s * rx, gy = s * ry, gz = s * rz;
         return Contrib{__fsub_rn(__fmul_rn(wy, gz), __fmul_rn(wz, gy)), __fsub_rn(__fmul_rn(wz, gx), __fmul_rn(wx, gz)),
@@ -1622,6 +1661,7 @@ struct OmegaVisit {
         r[0] = on ? c.ox : 0.f; r[1] = on ? c.oy : 0.f; r[2] = on ? c.oz : 0.f;
     }
 };
+using OmegaVisit = OmegaVisitT<false>;
 
 __global__ void __launch_bounds__(256)
 omega_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
@@ -1671,7 +1711,7 @@ __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __rest
 // by the leading blocks.
 // kNear: the pass filters the full list into omega's near list (5 blocks of 256 per SM: 80 us with 1M
 // particles; 4 and 6 88); else it walks the full list (4: 211 us; 3 219, 5 230).
-template <bool kNear>
+template <bool kNear, bool kUnitW>
 __global__ void __launch_bounds__(256, kNear ? 5 : 4)
 omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
@@ -1691,7 +1731,7 @@ omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict_
         return;
     }
     const float4 pi = p[i];
-    OmegaVisit vis(P, v, pi, v[i]);
+    OmegaVisitT<kUnitW> vis(P, v, pi, v[i]);
     const uint32_t lm = L.list ? filter_list(F, fm, L, i, pi, P.cut2, p) : kListOff;
     if (L.list) {
         L.meta[i] = lm;

@@ -163,6 +163,7 @@ struct pbd_sim {
     std::vector<SceneParams> h_scenes;
     float4 *fext = nullptr, *omega = nullptr, *delta = nullptr;
     float* lambda = nullptr;
+    float4* pl = nullptr;          // (p, lambda) of the last lambda pass, for the delta pass after it
     uint32_t *keys[2]{}, *vals[2]{};
     uint32_t *cell_start = nullptr, *cell_end = nullptr;
     uint32_t *hist = nullptr, *status = nullptr, *tile_counter = nullptr, *err = nullptr, *table_n = nullptr;
@@ -295,6 +296,7 @@ DevParams make_dev_params(const pbd_sim* s) {
     P.scene_of = s->scene_of;
     P.scene_range = s->scene_range;
     P.eta_tape = nullptr;
+    P.unit_w = ((p.active & PBD_ACTIVE_APPLY_FORCES) && p.collision_type == 0) ? 1u : 0u;
     const float c = std::max(P.hp, std::max(P.hs, P.d));
     P.cut2 = c * c * 1.0001f;
     return P;
@@ -373,14 +375,15 @@ template <bool kFull>
 static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevParams& P, uint32_t mode,
                               const float4* pin, const float4* pa, float4* pout, float4* x, float4* v, const float* lam,
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
-                              const NbList& L, const NbList& F, const LongLists& LL, int lanes, uint32_t N) {
+                              const NbList& L, const NbList& F, const LongLists& LL, int lanes, uint32_t N,
+                              const float4* pl) {
     if (lanes > 1) {
         auto k = BY_LANES(delta_list_group_kernel, kFull COMMA);
         k<<<div_up((uint64_t)N * lanes, tn) + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
         return;
     }
     constexpr uint32_t kFluid = kDoDelta | kDoCollide | kDoApply, kLast = kFluid | kDoUpdate;
-    const bool known = P.n_scorr == 4 && P.far_pairs_zero != 0u;
+    const bool known = pl && P.n_scorr == 4 && P.far_pairs_zero != 0u;
     auto k = delta_list_kernel<0, kFull, kDeltaAny>;
     if (mode == kFluid)
         k = !known ? delta_list_kernel<kFluid, kFull, kDeltaAny>
@@ -388,7 +391,7 @@ static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevPar
     else if (mode == kLast)
         k = !known ? delta_list_kernel<kLast, kFull, kDeltaAny>
                    : (w ? delta_list_kernel<kLast, kFull, kDeltaMass> : delta_list_kernel<kLast, kFull, kDeltaPlain>);
-    k<<<gn + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
+    k<<<gn + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL, pl);
 }
 
 // Record (or run) one frame of Fluid::compute (Fluid.cu:14-97) on `st`.
@@ -509,6 +512,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
         float4* aux = taped ? tape->aux[it] : nullptr;
         // a taped frame records the iteration's near lists into the tape (the delta pass reads them there)
         const NbList L = (taped && use_lists) ? NbList{tape->near[it], tape->near_meta[it], N, kListMax} : Lf;
+        // (p, lambda) side by side for a delta pass over lists at the lambda pass's positions
+        float4* const pl = (P.unit_w && lanes == 1 && use_full && (act & PBD_ACTIVE_COMPUTE_LAMBDA) && do_delta && !batched_contacts) ? s->pl : nullptr;
         if (act & PBD_ACTIVE_COMPUTE_LAMBDA) {
             const bool lstaged = staged_ok && it > 0 && !aux;
             PROF_BEGIN(lstaged ? "lambda_staged" : ((use_full && it > 0) ? "lambda_list" : "lambda"));
@@ -523,21 +528,23 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                                                    Lr.list ? DN : DX, aux, Lr, F, s->ll);
                 nl += 1;
             } else if (use_full && it > 0) {
-                lambda_list_kernel<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
-                                                                    CF, Lr.list ? DN : DX, aux, Lr, F, s->ll);
+                auto k = P.unit_w ? lambda_list_kernel<true> : lambda_list_kernel<false>;
+                k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF,
+                                                   Lr.list ? DN : DX, aux, Lr, F, s->ll, pl);
                 nl += 1;
             } else if (use_full && lanes > 1) {
                 auto k = BY_LANES(lambda_group_kernel, );
                 k<<<gl, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, aux, Lr, F, DF, Lr.list ? DN : DX);
                 lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, DF,
-                                                                aux, s->ll, F, Lr, Lr.list ? DN : DX);
+                                                                aux, s->ll, F, Lr, Lr.list ? DN : DX, pl);
                 nl += 2;
             } else {
-                lambda_kernel<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux, Lr,
-                                                 use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots);
+                auto k = P.unit_w ? lambda_kernel<true> : lambda_kernel<false>;
+                k<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux, Lr,
+                                                 use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots, pl);
                 if (use_full)
                     lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
-                                                                    DF, aux, s->ll, F, Lr, Lr.list ? DN : DX);
+                                                                    DF, aux, s->ll, F, Lr, Lr.list ? DN : DX, pl);
                 else
                     lambda_coop_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux);
                 nl += 2;
@@ -557,7 +564,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 if (by_list) {
                     (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                         gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N);
+                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, nullptr);
                     nl += 1;
                 } else {
                     delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -635,7 +642,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             } else if (by_list) {
                 (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
                     gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N);
+                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, pl);
                 nl += 1;
             } else {
                 delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -683,12 +690,12 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 auto k = BY_LANES(omega_list_group_kernel, );
                 k<<<gl + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end, s->omega, CF,
                                                    DNo, Lo, F, s->ll);
-            } else if (Lo.list)
-                omega_list_kernel<true><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end,
-                                                               s->omega, CF, DNo, Lo, F, s->ll);
-            else
-                omega_list_kernel<false><<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end,
-                                                               s->omega, CF, DNo, Lo, F, s->ll);
+            } else {
+                auto k = Lo.list ? (P.unit_w ? omega_list_kernel<true, true> : omega_list_kernel<true, false>)
+                                 : (P.unit_w ? omega_list_kernel<false, true> : omega_list_kernel<false, false>);
+                k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end, s->omega, CF, DNo,
+                                                   Lo, F, s->ll);
+            }
             nl += 1;
         } else {
             omega_kernel<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->cell_start, s->cell_end, s->omega, D, Lo, DNo);
@@ -914,6 +921,7 @@ int create_sim(const pbd_params* prm, uint32_t capacity, const std::vector<Scene
     for (int b = 0; b < 3; ++b) parts.push_back({(void**)&s->p[b], C * 16});
     parts.push_back({(void**)&s->fext, C * 16}); parts.push_back({(void**)&s->omega, C * 16});
     parts.push_back({(void**)&s->delta, C * 16}); parts.push_back({(void**)&s->lambda, C * 4});
+    parts.push_back({(void**)&s->pl, C * 16});
     parts.push_back({(void**)&s->cell_start, T * 4}); parts.push_back({(void**)&s->cell_end, T * 4});
     parts.push_back({(void**)&s->hist, (size_t)kMaxPasses * kRadix * 4});
     parts.push_back({(void**)&s->status, (size_t)kMaxPasses * s->max_tiles * kRadix * 4});

@@ -279,7 +279,7 @@ lambda_staged_kernel(const __grid_constant__ DevParams P, const float4* __restri
                      CoopSet C, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     __shared__ StageSmem<NoExtra> sm;
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, nullptr, i, LL, F, NbList{}, DeferList{}); });
+        run_coop_set(C, [&](uint32_t i) { coop_lambda(P, p, pa, cs, ce, lambda, nullptr, i, LL, F, NbList{}, DeferList{}, nullptr); });
         return;
     }
     const uint32_t i0 = (blockIdx.x - C.blocks) * kStageThreads;
