@@ -47,6 +47,15 @@ __device__ __forceinline__ typename V::Contrib contrib_of(V& vis, uint32_t j, co
     else return vis.contrib(j, pj, contact);
 }
 
+// Two float4 side by side (32-byte aligned), in one load.
+struct alignas(32) Pair4 { float4 a, b; };
+__device__ __forceinline__ Pair4 load_pair(const Pair4* p) {
+    Pair4 r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w) : "l"(p));
+    return r;
+}
+
 constexpr uint32_t kLongRange = 32;
 constexpr uint32_t kFullMask = 0xffffffffu;
 
@@ -526,6 +535,9 @@ __device__ __forceinline__ uint32_t filter_group(E&& entry, uint32_t n, uint32_t
 // visited entry by entry.
 template <class V, class = void> struct AddIf : std::false_type {};
 template <class V> struct AddIf<V, std::void_t<decltype(&V::add_if)>> : std::true_type {};
+// A visitor with load(j, pj, ex) takes an entry's position and extra data from an array of its own.
+template <class V, class = void> struct OwnLoad : std::false_type {};
+template <class V> struct OwnLoad<V, std::void_t<decltype(&V::load)>> : std::true_type {};
 template <class V, class = void> struct TestsContacts : std::false_type {};
 template <class V> struct TestsContacts<V, std::void_t<decltype(V::kTestsContacts)>> : std::true_type {};
 
@@ -545,8 +557,12 @@ __device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t 
         typename ExtraOf<V>::type ex[4];
 #pragma unroll
         for (uint32_t b = 0; b < 4u; ++b) {
-            pj[b] = __ldg(p + j[b]);
-            ex[b] = fetch_extra(vis, j[b]);
+            if constexpr (OwnLoad<V>::value) {
+                vis.load(j[b], pj[b], ex[b]);
+            } else {
+                pj[b] = __ldg(p + j[b]);
+                ex[b] = fetch_extra(vis, j[b]);
+            }
         }
         e += F.stride;
         if (kb + 4u < n) q = kOwn ? *e : __ldcs(e);
@@ -1699,11 +1715,16 @@ omega_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict
 __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                            const float4* __restrict__ v, const uint32_t* __restrict__ cs,
                                            const uint32_t* __restrict__ ce, float4* __restrict__ omega, uint32_t i,
-                                           const LongLists& LL, const NbList& F) {
+                                           const LongLists& LL, const NbList& F, Pair4* __restrict__ pairs) {
     const SceneCtx S = scene_ctx(P, i);
-    OmegaVisit vis(P, v, p[i], v[i]);
+    const float4 pi = p[i];
+    OmegaVisit vis(P, v, pi, v[i]);
     walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
-    if (lane_id() == 0) omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
+    if (lane_id() == 0) {
+        const float4 o = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
+        omega[i] = o;
+        if (pairs) pairs[i] = Pair4{pi, o};
+    }
 }
 
 // omega over the full list (recording the near list when L.list, and noting the particles left
@@ -1715,9 +1736,10 @@ template <bool kNear, bool kUnitW>
 __global__ void __launch_bounds__(256, kNear ? 5 : 4)
 omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
-                  CoopSet C, DeferList DN, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+                  CoopSet C, DeferList DN, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL,
+                  Pair4* __restrict__ pairs) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F); });
+        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F, pairs); });
         return;
     }
     const uint32_t i = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
@@ -1739,7 +1761,9 @@ omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict_
     }
     if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
     else walk_full(F, i, fm, p, vis);
-    omega[i] = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
+    const float4 o = make_float4(vis.ox, vis.oy, vis.oz, 0.f);
+    omega[i] = o;
+    if (pairs) pairs[i] = Pair4{pi, o};
 }
 
 // omega_list_kernel with G lanes per particle (small simulations, see lambda_group_kernel).
@@ -1750,7 +1774,7 @@ omega_list_group_kernel(const __grid_constant__ DevParams P, const float4* __res
                         float4* __restrict__ omega, CoopSet C, DeferList DN, const __grid_constant__ NbList L,
                         const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
     if (blockIdx.x < C.blocks) {
-        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F); });
+        run_coop_set(C, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LL, F, nullptr); });
         return;
     }
     const uint32_t tid = (blockIdx.x - C.blocks) * blockDim.x + threadIdx.x;
@@ -1779,7 +1803,7 @@ __global__ void __launch_bounds__(128)
 omega_coop_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float4* __restrict__ omega,
                   DeferList D) {
-    for_each_deferred(D, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LongLists{}, NbList{}); });
+    for_each_deferred(D, [&](uint32_t i) { coop_omega(P, p, pa, v, cs, ce, omega, i, LongLists{}, NbList{}, nullptr); });
 }
 
 // ======================================================================================
@@ -1874,6 +1898,22 @@ struct VortViscVisitT {
 
 using VortViscVisit = VortViscVisitT<3u>;
 
+// The same with an entry's position and omega from the omega pass's pairs: one 32-byte gather instead
+// of two of 16 (vorticity on).
+template <uint32_t kTerms>
+struct VortPairVisitT : VortViscVisitT<kTerms> {
+    using Base = VortViscVisitT<kTerms>;
+    using Extra = typename Base::Extra;
+    const Pair4* __restrict__ pairs;
+    __device__ VortPairVisitT(const Base& b, const Pair4* q) : Base(b), pairs(q) {}
+    __device__ __forceinline__ void load(uint32_t j, float4& pj, Extra& ex) const {
+        const Pair4 q = load_pair(pairs + j);
+        pj = q.a;
+        ex.oj = q.b;
+        if constexpr ((kTerms & 2u) != 0u) ex.vj = this->visc ? __ldg(this->v + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+};
+
 // The vorticity force from the vorticity sums of `vo` and the viscosity update from the sums of
 // `vs` (the same visitor when one walk summed both terms).  Explicitly rounded, so every kernel
 // that finishes a particle stores the same bits.  `vhost` (mapped pinned host memory, or null)
@@ -1954,7 +1994,8 @@ vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restr
                       const float4* __restrict__ vin, float4* __restrict__ vout, const float4* __restrict__ omega,
                       float4* __restrict__ fext, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                       int do_vort, int do_visc, const float* __restrict__ w, CoopSet C, const __grid_constant__ NbList Lv, const __grid_constant__ NbList Ln,
-                      float4* __restrict__ vhost, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL) {
+                      float4* __restrict__ vhost, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL,
+                      const Pair4* __restrict__ pairs) {
     if (blockIdx.x < C.blocks) {
         run_coop_set(C, [&](uint32_t i) {
             coop_vort_visc(P, p, pa, vin, vout, omega, fext, cs, ce, do_vort, do_visc, w, i, vhost, LL, F);
@@ -1976,8 +2017,16 @@ vort_visc_list_kernel(const __grid_constant__ DevParams P, const float4* __restr
         return;
     }
     VortViscVisit vis(P, vin, omega, p[i], vin[i], oi, do_vort != 0, do_visc != 0);
-    if constexpr (kLists == kVortVisc || kLists == kVortViscFull) walk_full(Lv, i, meta, p, vis);
-    else walk_near<false, 2>(Lv, i, meta, p, vis);
+    if constexpr (kLists == kVortViscFull) {
+        if (pairs) {
+            VortPairVisitT<3u> vp(vis, pairs);
+            walk_full(Lv, i, meta, p, vp);
+            vort_visc_finish(P, i, vp, vp, vout, fext, w, vhost);
+            return;
+        }
+    }
+    if constexpr (kLists == kViscNear) walk_near<false, 2>(Lv, i, meta, p, vis);
+    else walk_full(Lv, i, meta, p, vis);
     vort_visc_finish(P, i, vis, vis, vout, fext, w, vhost);
 }
 
