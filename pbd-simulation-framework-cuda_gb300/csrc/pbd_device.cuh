@@ -66,7 +66,29 @@ struct DevParams {
     // every predicted position's w is 1 for the whole frame: applyForces sets it (Forces.h:94), and with
     // collisionType 0 nothing but a 0 is ever added to it (collisionType 1 writes 0 there)
     uint32_t unit_w;
+    // the predicted positions in steps of 1/512 cell (coarse_pos), kept by every kernel that writes them
+    // in a frame whose passes filter lists by them, else null; near_coarse: coarse_near's limit
+    uint2* coarse;
+    uint32_t near_coarse;
 };
+
+// A position in steps of 1/512 cell, clamped to the 128 cells the enclosure's limits leave (x | y << 16,
+// z); a position that is not a number goes to the far corner, away from every wall.  Two positions
+// closer than the cut are also near by coarse_near: rounding moves a difference by at most 1.01 steps
+// per axis (clamping by none), coarse_near's packed subtraction another one in x, together 2.5 steps.
+__device__ __forceinline__ uint32_t coarse_axis(float c) {
+    const float q = c * 512.0f;
+    return __float2uint_rn(q == q ? fminf(fmaxf(q, 0.0f), 65535.0f) : 65535.0f);
+}
+__device__ __forceinline__ uint2 coarse_pos(float4 p) {
+    return make_uint2(coarse_axis(p.x) | (coarse_axis(p.y) << 16), coarse_axis(p.z));
+}
+// Whether two coarse positions may be within the cut (limit = near_coarse; 0: never).
+__device__ __forceinline__ bool coarse_near(uint2 a, uint2 b, uint32_t limit) {
+    const uint32_t d = a.x - b.x;
+    const int dx = (int)d >> 16, dy = (int)(int16_t)(d & 0xFFFFu), dz = (int)(a.y - b.y);
+    return (uint32_t)(dx * dx) + (uint32_t)(dy * dy) + (uint32_t)(dz * dz) < limit;
+}
 
 // The scene a particle belongs to, as the walk and the per-scene constants see it.
 struct SceneCtx {

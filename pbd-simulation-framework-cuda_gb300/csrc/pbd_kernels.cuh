@@ -156,7 +156,9 @@ reorder_cells_kernel(DevParams P, ReorderArgs A, SortScratch S, int npasses, uin
         uint32_t o = A.perm[i];
         if (o >= N) { atomicOr(S.err, kErrSortTimeout); o = i; }   // only after a failed sort
         A.xo[i] = A.xi[o];
-        A.po[i] = A.pi[o];
+        const float4 pp = A.pi[o];
+        A.po[i] = pp;
+        if (P.coarse) P.coarse[i] = coarse_pos(pp);
         A.vo[i] = A.vi[o];
         if (A.co) A.co[i] = A.ci[o];
         if (A.ido) A.ido[i] = A.idi[o];

@@ -627,11 +627,29 @@ __device__ __forceinline__ void walk_near(const NbList& L, uint32_t i, uint32_t 
 // list alone (every entry left out adds an exact zero to every sum of a lambda, omega or delta
 // pass), so the warp runs the kernel arithmetic for ~6 entries per particle instead of ~32.
 // Returns the near list's meta (kListOff when it does not fit).
-template <bool kOwn = false>
-__device__ __forceinline__ uint32_t filter_list(const NbList& F, uint32_t fm, const NbList& L, uint32_t i,
-                                                const float4& pi, float cut2, const float4* __restrict__ p) {
+// kCoarse: by the coarse positions, which let in at most the entries within 0.006 cells of the cut
+// besides (they add the same exact zeros).  The filter is bound by the L1, which takes a turn for every
+// line a gather touches: 8-byte positions touch half as many as 16-byte ones.  A position of i that is
+// not finite has no near entry, as its r^2 is not below the cut.
+template <bool kOwn, bool kCoarse>
+__device__ __forceinline__ uint32_t filter_list(const DevParams& P, const NbList& F, uint32_t fm, const NbList& L, uint32_t i,
+                                                const float4& pi, const float4* __restrict__ p) {
+    using Pos = typename std::conditional<kCoarse, uint2, float4>::type;
     const uint32_t n = fm & 0xFFu, nc = (fm >> 8) & 0xFFu;
     const uint4* e = reinterpret_cast<const uint4*>(F.list) + i;
+    const Pos* __restrict__ pos;
+    Pos own;
+    float cut2 = 0.0f;
+    uint32_t limit = 0u;
+    if constexpr (kCoarse) {
+        pos = P.coarse;
+        own = coarse_pos(pi);
+        limit = (fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z) < __int_as_float(0x7f800000)) ? P.near_coarse : 0u;
+    } else {
+        pos = p;
+        own = pi;
+        cut2 = P.cut2;
+    }
     uint32_t* o = L.list + i;
     const size_t ost = L.stride;
     uint32_t m = 0, mc = 0;
@@ -640,16 +658,18 @@ __device__ __forceinline__ uint32_t filter_list(const NbList& F, uint32_t fm, co
 #pragma unroll 1
     for (uint32_t kb = 0; kb < n; kb += 4u) {
         const uint32_t j[4] = {q.x, kb + 1u < n ? q.y : i, kb + 2u < n ? q.z : i, kb + 3u < n ? q.w : i};
-        float4 pj[4];
+        Pos pj[4];
 #pragma unroll
-        for (uint32_t b = 0; b < 4u; ++b) pj[b] = __ldg(p + j[b]);
+        for (uint32_t b = 0; b < 4u; ++b) pj[b] = __ldg(pos + j[b]);
         e += F.stride;
         if (kb + 4u < n) q = kOwn ? *e : __ldcs(e);
 #pragma unroll
         for (uint32_t b = 0; b < 4u; ++b) {
             if (kb + b == nc) mc = m;
-            const float rx = pi.x - pj[b].x, ry = pi.y - pj[b].y, rz = pi.z - pj[b].z;
-            if (kb + b < n && dist2(rx, ry, rz) < cut2) {
+            bool near;
+            if constexpr (kCoarse) near = coarse_near(own, pj[b], limit);
+            else near = dist2(own.x - pj[b].x, own.y - pj[b].y, own.z - pj[b].z) < cut2;
+            if (kb + b < n && near) {
                 if (m < L.kmax) {
                     *o = j[b];
                     o += ost;
@@ -1128,7 +1148,7 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         F.meta[i] = fm;
         const bool listed = !(fm & kListOff);
         if (!listed && !(fm & kListWalked)) return;
-        const uint32_t lm = (L.list && listed) ? filter_list<true>(F, fm, L, i, pi, P.cut2, p) : kListOff;
+        const uint32_t lm = (L.list && listed) ? filter_list<true, kUnitW>(P, F, fm, L, i, pi, p) : kListOff;
         if (L.list) {
             L.meta[i] = lm;
             if (lm == kListOff) note_particle(DN, i);
@@ -1232,8 +1252,10 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
 // The particles without a full list (the set C) are walked by the leading blocks; the ones left
 // without a near list are noted in DN for the delta pass.  Kept apart from lambda_kernel so that
 // its register budget is the list walk's alone.
-template <bool kUnitW>
-__global__ void __launch_bounds__(256, 5)
+// kNear: with near lists (L).  Blocks of 256 per SM: 6 with them (62 us with 1M particles; 5 66, 4 74), 5
+// over full lists (183 us with 1M dense particles; 6 201).
+template <bool kUnitW, bool kNear>
+__global__ void __launch_bounds__(256, kNear ? 6 : 5)
 lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce, float* __restrict__ lambda,
                    CoopSet C, const __grid_constant__ DeferList DN, float4* __restrict__ aux, const __grid_constant__ NbList L, const __grid_constant__ NbList F, const __grid_constant__ LongLists LL,
@@ -1249,13 +1271,14 @@ lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict
     const SceneCtx S = scene_ctx(P, i);
     const float4 pi = p[i];
     LambdaVisitT<kUnitW> vis(P, pi);
-    const uint32_t lm = L.list ? filter_list(F, fm, L, i, pi, P.cut2, p) : kListOff;
-    if (L.list) {
+    uint32_t lm = kListOff;
+    if constexpr (kNear) {
+        lm = filter_list<false, kUnitW>(P, F, fm, L, i, pi, p);
         L.meta[i] = lm;
         if (lm == kListOff) note_particle(DN, i);
+        if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
     }
-    if (lm != kListOff) walk_near<true>(L, i, lm, p, vis);
-    else walk_full(F, i, fm, p, vis);
+    if (lm == kListOff) walk_full(F, i, fm, p, vis);
     const float li = vis.finish(S.rho0);
     lambda[i] = li;
     if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
@@ -1489,6 +1512,7 @@ __device__ __forceinline__ void delta_finish(const DevParams& P, float rho0, uin
         xn = pn;
     }
     pout[i] = pn;
+    if (P.coarse) P.coarse[i] = coarse_pos(pn);
     if (mode & (kDoCollide | kDoUpdate)) x[i] = xn;
 }
 
@@ -1754,7 +1778,7 @@ omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict_
     }
     const float4 pi = p[i];
     OmegaVisitT<kUnitW> vis(P, v, pi, v[i]);
-    const uint32_t lm = L.list ? filter_list(F, fm, L, i, pi, P.cut2, p) : kListOff;
+    const uint32_t lm = L.list ? filter_list<false, kUnitW>(P, F, fm, L, i, pi, p) : kListOff;
     if (L.list) {
         L.meta[i] = lm;
         if (lm == kListOff) note_particle(DN, i);

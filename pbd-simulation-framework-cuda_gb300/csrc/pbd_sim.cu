@@ -163,6 +163,7 @@ struct pbd_sim {
     std::vector<SceneParams> h_scenes;
     float4 *fext = nullptr, *omega = nullptr, *delta = nullptr;
     float* lambda = nullptr;
+    uint2* coarse = nullptr;       // DevParams::coarse
     Pair4* po = nullptr;           // (p, omega) of the omega pass, for the vorticity pass after it
     float4* pl = nullptr;          // (p, lambda) of the last lambda pass, for the delta pass after it
     uint32_t *keys[2]{}, *vals[2]{};
@@ -300,6 +301,9 @@ DevParams make_dev_params(const pbd_sim* s) {
     P.unit_w = ((p.active & PBD_ACTIVE_APPLY_FORCES) && p.collision_type == 0) ? 1u : 0u;
     const float c = std::max(P.hp, std::max(P.hs, P.d));
     P.cut2 = c * c * 1.0001f;
+    P.coarse = nullptr;
+    const double steps = 512.0 * std::sqrt((double)P.cut2) + 3.0;   // coarse_near: 2.5 steps, rounded up
+    P.near_coarse = (uint32_t)std::min(steps * steps + 1.0, 4294967295.0);
     return P;
 }
 
@@ -408,6 +412,9 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     const uint32_t N = s->N;
     const int np = sort_passes(s);
     const int tn = s->tpb_nbr;
+    // the thread-per-particle passes filter their lists by the coarse positions where p.w needs no look
+    if (P.unit_w && pass_lanes(N) == 1 && use_full_list(s) && near_lists_on(s, P) && !(prm.flags & PBD_FLAG_STAGED_PASSES))
+        P.coarse = s->coarse;
     SortScratch S{s->hist, s->status, s->tile_counter, s->err, s->max_tiles, s->sort_spin_limit, s->sort_hold};
     nl = 0;
 
@@ -529,7 +536,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                                                    Lr.list ? DN : DX, aux, Lr, F, s->ll);
                 nl += 1;
             } else if (use_full && it > 0) {
-                auto k = P.unit_w ? lambda_list_kernel<true> : lambda_list_kernel<false>;
+                auto k = Lr.list ? (P.unit_w ? lambda_list_kernel<true, true> : lambda_list_kernel<false, true>)
+                                 : (P.unit_w ? lambda_list_kernel<true, false> : lambda_list_kernel<false, false>);
                 k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, CF,
                                                    Lr.list ? DN : DX, aux, Lr, F, s->ll, pl);
                 nl += 1;
@@ -926,6 +934,7 @@ int create_sim(const pbd_params* prm, uint32_t capacity, const std::vector<Scene
     parts.push_back({(void**)&s->fext, C * 16}); parts.push_back({(void**)&s->omega, C * 16});
     parts.push_back({(void**)&s->delta, C * 16}); parts.push_back({(void**)&s->lambda, C * 4});
     parts.push_back({(void**)&s->pl, C * 16}); parts.push_back({(void**)&s->po, C * 32});
+    parts.push_back({(void**)&s->coarse, C * 8});
     parts.push_back({(void**)&s->cell_start, T * 4}); parts.push_back({(void**)&s->cell_end, T * 4});
     parts.push_back({(void**)&s->hist, (size_t)kMaxPasses * kRadix * 4});
     parts.push_back({(void**)&s->status, (size_t)kMaxPasses * s->max_tiles * kRadix * 4});

@@ -269,3 +269,20 @@ def test_lanes_per_particle_bit_identical_to_full_walk(need_gpu, pbd, scenes, sh
     a = _run(pbd, params, pos, vel, 2)
     b = _run(pbd, params, pos, vel, 2, full_walk=True)
     _same(a, b)
+
+
+@pytest.mark.parametrize("where", ["inside", "walls", "touching"])
+def test_coarse_filter_keeps_every_near_pair(need_gpu, pbd, scenes, where):
+    """the near lists are filtered by positions in steps of 1/512 cell: pairs at the cut to the last bits,
+    positions at the enclosure's limits (1.5 and 126.5, where the coarse position is near its end) and
+    particles pressed through one another, against the walk of every cell"""
+    params = scenes.workload_params(pbd, 128, 1000.0, vorticity=0.0005, viscosity=0.01)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    rng = np.random.default_rng(25)
+    origin = {"inside": (60.0, 60.0, 60.0), "walls": (98.0, 1.6, 98.0), "touching": (30.0, 30.0, 30.0)}[where]
+    pos, vel = scenes.lattice(30, 30, 30, origin=origin, spacing={"inside": 1.00005, "walls": 0.98, "touching": 0.7}[where], jitter=1e-6 if where == "inside" else 0.1, seed=25)
+    vel[:, :3] = rng.normal(0, 0.0 if where == "inside" else 20.0, size=(len(vel), 3)).astype(np.float32)
+    a = _run(pbd, params, pos, vel, 4)
+    b = _run(pbd, params, pos, vel, 4, full_walk=True)
+    _same(a, b)
