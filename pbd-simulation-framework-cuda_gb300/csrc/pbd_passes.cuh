@@ -773,106 +773,23 @@ struct FullWriter {
     }
 };
 
-// The frame's full list of particle i for a 27-cell neighbourhood (kernelWidthNeighbours 1,
-// findContacts on), indices only: the entries, order, cap M, self-skip and long-range hand-over
-// of walk_seq over for_each_range, with the three cells of a column stored by one loop.
-// Returns the list's meta (kListOff when it does not fit or the particle is handed over; then
-// *deferred tells which).
-__device__ __forceinline__ uint32_t store_full_list(const DevParams& P, const SceneCtx& S, uint32_t i, float4 pa,
-                                                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
-                                                    const NbList& F, bool* deferred) {
-    const uint32_t N = P.N, M = P.M;
-    if (M == 0) return 0u;
-    const bool quirk = (P.flags & PBD_FLAG_CELL_END_QUIRK) && S.n >= 2;
-    uint32_t mx[3], my[3], mz[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        mx[c] = morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.x)) << 2;
-        my[c] = morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.y)) << 1;
-        mz[c] = morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.z));
-    }
-    FullWriter out(F, i);
-    uint32_t n = 0;
-    bool full = false;   // the cap is reached
-#pragma unroll 1
-    for (int col = 0; col < 9 && !full; ++col) {
-        const int a = col / 3, b = col - 3 * (col / 3);
-        const uint32_t hxy = (a == 0 ? mx[0] : (a == 1 ? mx[1] : mx[2])) + (b == 0 ? my[0] : (b == 1 ? my[1] : my[2]));
-        uint32_t h[3], s3[3], e3[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            h[c] = hxy + mz[c];
-            s3[c] = h[c] < S.cells ? __ldg(cs + S.base + h[c]) : kEmptyCell;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) e3[c] = h[c] < S.cells ? __ldg(ce + S.base + h[c]) : 0u;
-        uint32_t len[3];
-        uint32_t reach = n;   // entries stored before the cell: the walk reaches it while below the cap
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const bool valid = s3[c] < N;
-            const uint32_t e = ((quirk && h[c] == S.n - 1) || e3[c] > S.end) ? S.end : e3[c];
-            len[c] = valid ? e - s3[c] : 0u;
-            if (valid && reach < M && len[c] > kLongRange) { *deferred = true; return kListOff; }
-            reach += len[c] - ((valid && s3[c] <= i && i < e) ? 1u : 0u);
-        }
-        const uint32_t l01 = len[0] + len[1], T = l01 + len[2];
-        if (reach < M && reach <= F.kmax) {   // the column fits below the cap and the list's room
-#pragma unroll 1
-            for (uint32_t t = 0; t < T; ++t) {
-                const uint32_t j = t < len[0] ? s3[0] + t : (t < l01 ? s3[1] + (t - len[0]) : s3[2] + (t - l01));
-                if (j != i) out.push(j);
-            }
-            n = reach;
-            continue;
-        }
-#pragma unroll 1
-        for (uint32_t t = 0; t < T && !full; ++t) {
-            const uint32_t j = t < len[0] ? s3[0] + t : (t < l01 ? s3[1] + (t - len[0]) : s3[2] + (t - l01));
-            if (j == i) continue;
-            if (n < F.kmax) out.push(j);
-            full = ++n == M;
-        }
-    }
-    out.flush();
-    return n > F.kmax ? kListOff : (n | (n << 8));
-}
-
-// The cells of one group of particle i's list (the 3 cells of a findContacts column, or the cells
-// of a findNeighbours column: 2 sh + 1 on an edge column, 2 otherwise), stored into the full list:
-// all table loads in flight first, then the entries in list order, skipping self, with the cap M,
-// the list's room and the long-range hand-over of walk_seq.  Returns true when the walk ends here
+// The cells of one group of particle i's list (store_column's), cell by cell: the entries in list
+// order, skipping self, with the cap M, the list's room and the long-range hand-over of walk_seq.  Returns true when the walk ends here
 // (cap reached or handed over).
 template <int kMax>
-__device__ __forceinline__ bool store_cell_group(const DevParams& P, const SceneCtx& S, uint32_t i, const uint32_t* h,
-                                                 int ncell, const uint32_t* __restrict__ cs,
-                                                 const uint32_t* __restrict__ ce, const NbList& F, bool quirk,
-                                                 FullWriter& out, uint32_t& n, bool* deferred) {
+__device__ __forceinline__ bool store_cells(const DevParams& P, const SceneCtx& S, uint32_t i, const uint32_t* h,
+                                            const uint32_t* s, const uint32_t* e, const NbList& F, bool quirk,
+                                            FullWriter& out, uint32_t& n, bool* deferred) {
     const uint32_t N = P.N, M = P.M;
-    uint32_t s[kMax], e[kMax], len[kMax];
-#pragma unroll
-    for (int c = 0; c < kMax; ++c) s[c] = (c < ncell && h[c] < S.cells) ? __ldg(cs + S.base + h[c]) : kEmptyCell;
-#pragma unroll
-    for (int c = 0; c < kMax; ++c) e[c] = (c < ncell && h[c] < S.cells) ? __ldg(ce + S.base + h[c]) : 0u;
+    uint32_t len[kMax];
     uint32_t reach = n;   // entries stored before the cell: the walk reaches it while below the cap
 #pragma unroll
     for (int c = 0; c < kMax; ++c) {
-        const bool valid = c < ncell && s[c] < N;
+        const bool valid = s[c] < N;
         const uint32_t ec = ((quirk && h[c] == S.n - 1) || e[c] > S.end) ? S.end : e[c];
         len[c] = valid ? ec - s[c] : 0u;
         if (valid && reach < M && len[c] > kLongRange) { *deferred = true; return true; }
         reach += len[c] - ((valid && s[c] <= i && i < ec) ? 1u : 0u);
-    }
-    if (reach < M && reach <= F.kmax) {   // the group fits below the cap and the list's room
-#pragma unroll
-        for (int c = 0; c < kMax; ++c)
-#pragma unroll 1
-            for (uint32_t t = 0; t < len[c]; ++t) {
-                const uint32_t j = s[c] + t;
-                if (j != i) out.push(j);
-            }
-        n = reach;
-        return false;
     }
 #pragma unroll
     for (int c = 0; c < kMax; ++c)
@@ -886,17 +803,106 @@ __device__ __forceinline__ bool store_cell_group(const DevParams& P, const Scene
     return false;
 }
 
-// The frame's full list of particle i with findNeighbours' shells (kernelWidthNeighbours 2 or 3,
-// findContacts on): the 27 cells, then each shell, by cell groups (store_cell_group).  Returns the
-// list's meta (kListOff when it does not fit or the particle is handed over; *deferred tells which).
-__device__ __forceinline__ uint32_t store_full_list_shells(const DevParams& P, const SceneCtx& S, uint32_t i, float4 pa,
-                                                           const uint32_t* __restrict__ cs,
-                                                           const uint32_t* __restrict__ ce, const NbList& F,
-                                                           bool* deferred) {
-    const uint32_t M = P.M;
-    if (M == 0) return 0u;
+// Append the entries of kRuns runs of particles without i, by one loop without a check per entry, where
+// no run is longer than kLongRange and the cap and the list's room are out of reach; false otherwise.
+template <int kRuns>
+__device__ __forceinline__ bool push_runs(const DevParams& P, uint32_t i, const uint32_t* rs, const uint32_t* len, const NbList& F,
+                                          FullWriter& out, uint32_t& n) {
+    uint32_t end[kRuns], off[kRuns];   // run r: entries [end[r - 1], end[r]) of the column; entry t is particle off[r] + t
+    uint32_t T = 0, longest = 0;
+#pragma unroll
+    for (int r = 0; r < kRuns; ++r) {
+        longest = max(longest, len[r]);
+        off[r] = rs[r] - T;
+        T += len[r];
+        end[r] = T;
+    }
+    if (!(longest <= kLongRange && n + T < P.M && n + T <= F.kmax)) return false;
+#pragma unroll 1
+    for (uint32_t t = 0; t < T; ++t) {
+        uint32_t o = off[kRuns - 1];
+#pragma unroll
+        for (int r = kRuns - 2; r >= 0; --r) o = t < end[r] ? off[r] : o;
+        const uint32_t j = o + t;
+        if (j != i) out.push(j);
+    }
+    n = out.n;
+    return true;
+}
+
+// One column of particle i's list: the 3 cells of a findContacts column or the cells of a
+// findNeighbours column (2 sh + 1 on an edge column, 2 otherwise), keys h in list order; the table
+// loads are all in flight first.  Cells z, z + 1 with z even have consecutive Morton keys, so their
+// particles lie side by side: where the cells' z follow each other (`consecutive`; rounding or a diameter
+// other than 1 can break it) each such pair is one run and the column has 2 to 4, else a run per cell.
+// A column with a range longer than kLongRange, the cell-end range, or near the cap or the list's room
+// goes cell by cell.  (One loop per cell, each with its checks, was 604 us for 1M dense particles, this
+// is 451; for 27 cells 154 -> 143.)  Returns true when the walk ends here (cap reached or handed over).
+template <int kCells>
+__device__ __forceinline__ bool store_column(const DevParams& P, const SceneCtx& S, uint32_t i, const uint32_t* h,
+                                             bool odd, bool consecutive, const uint32_t* __restrict__ cs,
+                                             const uint32_t* __restrict__ ce, const NbList& F, bool quirk,
+                                             FullWriter& out, uint32_t& n, bool* deferred) {
+    constexpr int kRuns = kCells == 2 ? 2 : (kCells + 1) / 2;
+    uint32_t s[kCells], e[kCells];
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) s[c] = h[c] < S.cells ? __ldg(cs + S.base + h[c]) : kEmptyCell;
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) e[c] = h[c] < S.cells ? __ldg(ce + S.base + h[c]) : 0u;
+    bool cell_end = false;
+    if (quirk) {
+#pragma unroll
+        for (int c = 0; c < kCells; ++c) cell_end = cell_end || h[c] == S.n - 1u;
+    }
+    if (!cell_end) {
+        if (kCells == 2 || !consecutive) {
+            uint32_t len[kCells];
+#pragma unroll
+            for (int c = 0; c < kCells; ++c) len[c] = s[c] < P.N ? e[c] - s[c] : 0u;
+            if (push_runs<kCells>(P, i, s, len, F, out, n)) return false;
+        } else {
+            const bool even_first = odd == (((kCells - 1) / 2) & 1);   // the column's first cell has an even z
+            uint32_t rs[kRuns], len[kRuns];
+#pragma unroll
+            for (int r = 0; r < kRuns; ++r) {   // cells (2 r, 2 r + 1) or (2 r - 1, 2 r), those that exist
+                const uint32_t s0 = r > 0 ? s[2 * r - 1] : kEmptyCell, e0 = r > 0 ? e[2 * r - 1] : 0u;
+                const uint32_t s2 = 2 * r + 1 < kCells ? s[2 * r + 1] : kEmptyCell, e2 = 2 * r + 1 < kCells ? e[2 * r + 1] : 0u;
+                const uint32_t slo = even_first ? s[2 * r] : s0, elo = even_first ? e[2 * r] : e0;
+                const uint32_t shi = even_first ? s2 : s[2 * r], ehi = even_first ? e2 : e[2 * r];
+                const bool lo = slo < P.N, hi = shi < P.N;
+                rs[r] = lo ? slo : shi;
+                len[r] = (lo || hi) ? (hi ? ehi : elo) - rs[r] : 0u;
+            }
+            if (push_runs<kRuns>(P, i, rs, len, F, out, n)) return false;
+        }
+    }
+    return store_cells<kCells>(P, S, i, h, s, e, F, quirk, out, n, deferred);
+}
+
+// The frame's full list of particle i, indices only (findContacts on; kShells: with findNeighbours'
+// shells, kernelWidthNeighbours 2 or 3): the entries, order, cap M, self-skip and long-range hand-over
+// of walk_seq over for_each_range, column by column.  Returns the list's meta (kListOff when it does not
+// fit or the particle is handed over; *deferred tells which).
+template <bool kShells>
+__device__ __forceinline__ uint32_t store_full_list(const DevParams& P, const SceneCtx& S, uint32_t i, float4 pa,
+                                                    const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
+                                                    const NbList& F, bool* deferred) {
+    if (P.M == 0) return 0u;
+    constexpr int R = kShells ? 3 : 1;
     const bool quirk = (P.flags & PBD_FLAG_CELL_END_QUIRK) && S.n >= 2;
-    const int K = (int)P.K;
+    const int K = kShells ? (int)P.K : 1;
+    uint32_t mz[2 * R + 1];
+    int zc = 0;
+    bool consecutive = true;
+#pragma unroll
+    for (int c = -R; c <= R; ++c) {
+        const float z = fminf(fmaxf(__fmaf_rn((float)c, P.d, pa.z), 0.0f), 1023.0f);   // morton_axis
+        const int cell = (int)(uint32_t)z;
+        mz[c + R] = expand_bits((uint32_t)cell);
+        if (c > -R && c > -K && c <= K) consecutive = consecutive && cell == zc + 1;
+        zc = cell;
+    }
+    const bool odd = (mz[R] & 1u) != 0u;
     uint32_t n = 0, nc = 0xFFFFFFFFu;
     FullWriter out(F, i);
     auto meta = [&]() -> uint32_t {
@@ -905,31 +911,46 @@ __device__ __forceinline__ uint32_t store_full_list_shells(const DevParams& P, c
         return n > F.kmax ? kListOff : (n | (c << 8));
     };
     uint32_t h[7];
+#pragma unroll 1
     for (int a = -1; a <= 1; ++a) {
         const uint32_t hx = morton_axis(__fmaf_rn((float)a, P.d, pa.x)) << 2;
+#pragma unroll 1
         for (int b = -1; b <= 1; ++b) {
             const uint32_t hxy = hx + (morton_axis(__fmaf_rn((float)b, P.d, pa.y)) << 1);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) h[c] = hxy + morton_axis(__fmaf_rn((float)(c - 1), P.d, pa.z));
-            if (store_cell_group<3>(P, S, i, h, 3, cs, ce, F, quirk, out, n, deferred)) return *deferred ? kListOff : meta();
+            for (int c = 0; c < 3; ++c) h[c] = hxy + mz[R - 1 + c];
+            if (store_column<3>(P, S, i, h, odd, consecutive, cs, ce, F, quirk, out, n, deferred)) return *deferred ? kListOff : meta();
         }
     }
-    nc = n;
-    for (int sh = 2; sh <= K; ++sh)
-        for (int a = -sh; a <= sh; ++a) {
-            const uint32_t hx = morton_axis(__fmaf_rn((float)a, P.d, pa.x)) << 2;
-            for (int b = -sh; b <= sh; ++b) {
-                const uint32_t hxy = hx + (morton_axis(__fmaf_rn((float)b, P.d, pa.y)) << 1);
-                const bool edge = (a == sh || a == -sh || b == sh || b == -sh);
-                const int m = edge ? 2 * sh + 1 : 2;   // interior columns: only c = -sh and c = +sh
+    if constexpr (kShells) {
+        nc = n;
+#pragma unroll 1
+        for (int sh = 2; sh <= K; ++sh)
+#pragma unroll 1
+            for (int a = -sh; a <= sh; ++a) {
+                const uint32_t hx = morton_axis(__fmaf_rn((float)a, P.d, pa.x)) << 2;
+#pragma unroll 1
+                for (int b = -sh; b <= sh; ++b) {
+                    const uint32_t hxy = hx + (morton_axis(__fmaf_rn((float)b, P.d, pa.y)) << 1);
+                    const bool edge = a == sh || a == -sh || b == sh || b == -sh;
+                    bool ends;
+                    if (!edge) {   // interior columns: only c = -sh and c = +sh
+                        h[0] = hxy + (sh == 2 ? mz[1] : mz[0]);
+                        h[1] = hxy + (sh == 2 ? mz[5] : mz[6]);
+                        ends = store_column<2>(P, S, i, h, odd, consecutive, cs, ce, F, quirk, out, n, deferred);
+                    } else if (sh == 2) {
 #pragma unroll
-                for (int t = 0; t < 7; ++t) {
-                    const int c = edge ? t - sh : (t == 0 ? -sh : sh);
-                    h[t] = hxy + morton_axis(__fmaf_rn((float)c, P.d, pa.z));
+                        for (int c = 0; c < 5; ++c) h[c] = hxy + mz[1 + c];
+                        ends = store_column<5>(P, S, i, h, odd, consecutive, cs, ce, F, quirk, out, n, deferred);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 7; ++c) h[c] = hxy + mz[c];
+                        ends = store_column<7>(P, S, i, h, odd, consecutive, cs, ce, F, quirk, out, n, deferred);
+                    }
+                    if (ends) return *deferred ? kListOff : meta();
                 }
-                if (store_cell_group<7>(P, S, i, h, m, cs, ce, F, quirk, out, n, deferred)) return *deferred ? kListOff : meta();
             }
-        }
+    }
     return meta();
 }
 
@@ -1132,9 +1153,9 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         uint32_t fm;
         const bool shells = (P.active & PBD_ACTIVE_FIND_NEIGHBOURS) && P.K >= 2;
         if (!shells && (P.active & PBD_ACTIVE_FIND_CONTACTS)) {
-            fm = store_full_list(P, S, i, pa[i], cs, ce, F, &deferred);
+            fm = store_full_list<false>(P, S, i, pa[i], cs, ce, F, &deferred);
         } else if (shells && P.K <= 3 && (P.active & PBD_ACTIVE_FIND_CONTACTS)) {
-            fm = store_full_list_shells(P, S, i, pa[i], cs, ce, F, &deferred);
+            fm = store_full_list<true>(P, S, i, pa[i], cs, ce, F, &deferred);
         } else {
             ListRecorder rec(F, i);
             walk_seq(P, S, i, pa[i], p, cs, ce, rec, true, &deferred);

@@ -286,3 +286,20 @@ def test_coarse_filter_keeps_every_near_pair(need_gpu, pbd, scenes, where):
     a = _run(pbd, params, pos, vel, 4)
     b = _run(pbd, params, pos, vel, 4, full_walk=True)
     _same(a, b)
+
+
+@pytest.mark.parametrize("radius,shells", [(0.4, 1), (0.4, 2), (0.63, 2), (0.5, 3), (0.3, 3)])
+def test_list_columns_bit_identical_to_full_walk(need_gpu, pbd, scenes, radius, shells):
+    """the first lambda pass stores a column's cells as runs of two where their z follow each other; a
+    diameter other than 1 repeats or skips cells, positions a rounding below a whole number make
+    p + 1 the cell after the next"""
+    params = scenes.workload_params(pbd, 64, 1995.0, vorticity=0.0005, viscosity=0.00015)
+    params.particle_radius = radius
+    params.lambda_epsilon = 0.1
+    params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 2.1, 2.0, shells
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(31, 29, 33, origin=(1.6, 1.6, 1.6), spacing=0.9, seed=26)
+    pos[::3, :3] = np.nextafter(np.ceil(pos[::3, :3]), np.float32(0), dtype=np.float32)
+    a = _run(pbd, params, pos, vel, 2)
+    b = _run(pbd, params, pos, vel, 2, full_walk=True)
+    _same(a, b)
