@@ -162,6 +162,19 @@ __device__ __forceinline__ float rcp_fast(float x) {
     return r;
 }
 
+// Two floats as one operand: an instruction does the arithmetic of two pairs of particles, each half
+// rounded as the scalar instruction rounds it.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void f2_split(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {   // a - b = b * (-1) + a, rounded once
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(f2(-1.0f, -1.0f).v), "l"(a.v));
+    return r;
+}
+
 // ---------------------------------------------------------- pair kernels (Density.h) --
 // poly6Viscosity: W = 315 t^3 t^3 / den, t = hp^2 - d^2, for 0.001 < d < hp - 0.001.  Selected, not
 // branched: the lanes of a warp disagree on the range.
@@ -178,6 +191,17 @@ __device__ __forceinline__ float spiky_scale(const DevParams& P, float dist, flo
     const float a = P.hs - dist;
     const float s = 15.0f * (a * a * P.inv_spiky_den) * rsqrt_fast(r2w);
     return (dist > 0.0001f && a > 0.0001f) ? s : 0.0f;
+}
+
+// poly6 and spiky_scale of two pairs without their ranges (the caller tests them), the same products in
+// the same order.
+__device__ __forceinline__ F2 poly6_open(const DevParams& P, F2 dist) {
+    const F2 t = sub2(f2(P.hp2, P.hp2), mul2(dist, dist));
+    const F2 t3 = mul2(mul2(t, t), t);
+    return mul2(mul2(mul2(f2(315.0f, 315.0f), t3), t3), f2(P.poly_inv_den, P.poly_inv_den));
+}
+__device__ __forceinline__ F2 spiky_open(const DevParams& P, F2 a, F2 inv_r) {   // a = hs - |r|
+    return mul2(mul2(f2(15.0f, 15.0f), mul2(mul2(a, a), f2(P.inv_spiky_den, P.inv_spiky_den))), inv_r);
 }
 
 // Integer power by repeated multiplication (the reference's pow(float, int)): r = 1, then

@@ -535,6 +535,14 @@ __device__ __forceinline__ uint32_t filter_group(E&& entry, uint32_t n, uint32_t
 // visited entry by entry.
 template <class V, class = void> struct AddIf : std::false_type {};
 template <class V> struct AddIf<V, std::void_t<decltype(&V::add_if)>> : std::true_type {};
+// A visitor with kAddTwo adds two entries, one after the other, by one call: the arithmetic of both in
+// two-float instructions, each kernel's range tested only where its term is added.  Over full lists the
+// passes are bound by instruction issue and the gathers together: 54 -> 43 instructions per entry for
+// delta and 43 -> 31 for lambda made them 211 -> 185 and 169 -> 147 us (1M particles, ~124 entries;
+// positions loaded a group ahead instead: 210 and 180, the registers cost warps).  i itself as an entry
+// must add nothing to its sums.
+template <class V, class = void> struct AddTwo : std::false_type {};
+template <class V> struct AddTwo<V, std::void_t<decltype(V::kAddTwo)>> : std::bool_constant<V::kAddTwo> {};
 // A visitor with load(j, pj, ex) takes an entry's position and extra data from an array of its own.
 template <class V, class = void> struct OwnLoad : std::false_type {};
 template <class V> struct OwnLoad<V, std::void_t<decltype(&V::load)>> : std::true_type {};
@@ -566,6 +574,13 @@ __device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t 
         }
         e += F.stride;
         if (kb + 4u < n) q = kOwn ? *e : __ldcs(e);
+        if constexpr (AddTwo<V>::value) {
+            constexpr bool kC = decltype(contacts)::value;
+            vis.template add_two<kC>(j[0], pj[0], kb < nc, j[1], pj[1], kb + 1u < nc);
+            vis.template add_two<kC>(j[2], pj[2], kb + 2u < nc, j[3], pj[3], kb + 3u < nc);
+            kb += 4u;
+            return;
+        }
 #pragma unroll
         for (uint32_t b = 0; b < 4u; ++b) {
             const bool contact = decltype(contacts)::value && kb + b < nc;
@@ -1107,6 +1122,45 @@ struct LambdaVisitT {
             asm("{ .reg .pred q; setp.lt.u32 q, %1, %2; setp.ltu.and.f32 q, %3, %4, q; @q fma.rn.f32 %0, %5, %6, %0; }"
                 : "+f"(Cw) : "r"(k), "r"(n), "f"(c.r2), "f"(P.cut2), "f"(c.s), "f"(c.rw));
     }
+    // The kernels are tested where they are added: within spiky's range (or NaN, which add() passes on)
+    // r^2 < cut2 holds, and i itself (r = 0) is in neither range.
+    static constexpr bool kAddTwo = true;
+    template <bool>
+    __device__ __forceinline__ void add_two(uint32_t, const float4& p0, bool, uint32_t, const float4& p1, bool) {
+        float x[2], y[2], z[2], w[2], d[2], a[2], W[2], s[2], B2[2];
+        f2_split(sub2(f2(pi.x, pi.y), f2(p0.x, p0.y)), x[0], y[0]);
+        f2_split(sub2(f2(pi.x, pi.y), f2(p1.x, p1.y)), x[1], y[1]);
+        z[0] = pi.z - p0.z; z[1] = pi.z - p1.z;
+        const float r0 = dist2(x[0], y[0], z[0]), r1 = dist2(x[1], y[1], z[1]);
+        float q0 = r0, q1 = r1;
+        if constexpr (!kUnitW) {
+            w[0] = pi.w - p0.w; w[1] = pi.w - p1.w;
+            q0 = __fmaf_rn(w[0], w[0], r0); q1 = __fmaf_rn(w[1], w[1], r1);
+        }
+        d[0] = sqrt_fast(r0); d[1] = sqrt_fast(r1);
+        const F2 dd = f2(d[0], d[1]), aa = sub2(f2(P.hs, P.hs), dd);
+        f2_split(poly6_open(P, dd), W[0], W[1]);
+        const F2 ss = spiky_open(P, aa, f2(rsqrt_fast(q0), rsqrt_fast(q1)));
+        f2_split(mul2(mul2(ss, ss), f2(q0, q1)), B2[0], B2[1]);
+        f2_split(aa, a[0], a[1]);
+        f2_split(ss, s[0], s[1]);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            asm("{ .reg .pred q; setp.gt.f32 q, %1, %2; setp.lt.and.f32 q, %1, %3, q; @q add.rn.f32 %0, %0, %4; }"
+                : "+f"(A) : "f"(d[b]), "f"(0.001f), "f"(P.hp_lim), "f"(W[b]));
+            if constexpr (kUnitW)
+                asm("{ .reg .pred q; setp.gtu.f32 q, %4, %6; setp.gtu.and.f32 q, %5, %6, q; @q add.rn.f32 %0, %0, %7;"
+                    " @q fma.rn.f32 %1, %8, %9, %1; @q fma.rn.f32 %2, %8, %10, %2; @q fma.rn.f32 %3, %8, %11, %3; }"
+                    : "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz)
+                    : "f"(d[b]), "f"(a[b]), "f"(0.0001f), "f"(B2[b]), "f"(s[b]), "f"(x[b]), "f"(y[b]), "f"(z[b]));
+            else
+                asm("{ .reg .pred q; setp.gtu.f32 q, %5, %7; setp.gtu.and.f32 q, %6, %7, q; @q add.rn.f32 %0, %0, %8;"
+                    " @q fma.rn.f32 %1, %9, %10, %1; @q fma.rn.f32 %2, %9, %11, %2; @q fma.rn.f32 %3, %9, %12, %3;"
+                    " @q fma.rn.f32 %4, %9, %13, %4; }"
+                    : "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz), "+f"(Cw)
+                    : "f"(d[b]), "f"(a[b]), "f"(0.0001f), "f"(B2[b]), "f"(s[b]), "f"(x[b]), "f"(y[b]), "f"(z[b]), "f"(w[b]));
+        }
+    }
     // walk_group_sums: A, B, C from the rows a, b, s, r
     static constexpr int kRows = 7, kSums = 6;
     __device__ static constexpr int mul_row(int s) { return s < 2 ? kRows : 2; }
@@ -1440,6 +1494,26 @@ struct DeltaVisitT {
     using Extra = float;   // lambda_j
     __device__ __forceinline__ float fetch(uint32_t j) const { return (!kKnow && do_delta) ? __ldg(lambda + j) : 0.f; }
     __device__ __forceinline__ bool masses() const { return kKnown == kDeltaPlain ? false : (kKnown == kDeltaMass ? true : w != nullptr); }
+    // the contact part's t of an entry at distance dist; false when they do not touch
+    __device__ __forceinline__ bool contact_t(uint32_t j, float dist, float& t) const {
+        const float overlap = P.d - dist;
+        if (!(overlap > 0.0f && dist > 0.00001f)) return false;
+        // share of the overlap this particle takes: inverseMass1 / (inverseMass1 + inverseMass2)
+        // (Collision.h:223-225, where both are forced to 1); solids have inverse mass 0
+        float share = 0.5f;
+        if (masses()) {
+            const float wj = __ldg(w + j);
+            share = (wi + wj) > 0.0f ? wi / (wi + wj) : 0.0f;
+        }
+        // -share * overlap * (1 - stiffness) along -r / |r|
+        t = __fmul_rn(__fmul_rn(-share * overlap, rcp_fast(dist)), P.one_minus_stiffness);
+        return share != 0.0f;
+    }
+    __device__ __forceinline__ void add_contact(float rx, float ry, float rz, float t) {
+        pacc.x = __fmaf_rn(-rx, t, pacc.x); xacc.x = __fmaf_rn(-rx, t, xacc.x);
+        pacc.y = __fmaf_rn(-ry, t, pacc.y); xacc.y = __fmaf_rn(-ry, t, xacc.y);
+        pacc.z = __fmaf_rn(-rz, t, pacc.z); xacc.z = __fmaf_rn(-rz, t, xacc.z);
+    }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, float lj_, bool contact) const {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z, rw = kKnow ? 0.0f : pi.w - pj.w;
         const float lj = kKnow ? pj.w : lj_;
@@ -1455,23 +1529,7 @@ struct DeltaVisitT {
             c.s = s;
             c.d = near && (s != 0.0f || all_pairs);
         }
-        if (contact && do_collide) {
-            const float overlap = P.d - dist;
-            if (near && overlap > 0.0f && dist > 0.00001f) {
-                // share of the overlap this particle takes: inverseMass1 / (inverseMass1 + inverseMass2)
-                // (Collision.h:223-225, where both are forced to 1); solids have inverse mass 0
-                float share = 0.5f;
-                if (masses()) {
-                    const float wj = __ldg(w + j);
-                    share = (wi + wj) > 0.0f ? wi / (wi + wj) : 0.0f;
-                }
-                if (share != 0.0f) {
-                    // -share * overlap * (1 - stiffness) along -r / |r|
-                    c.t = __fmul_rn(__fmul_rn(-share * overlap, rcp_fast(dist)), P.one_minus_stiffness);
-                    c.c = true;
-                }
-            }
-        }
+        if (contact && do_collide && near) c.c = contact_t(j, dist, c.t);
         return c;
     }
     __device__ __forceinline__ void add(const Contrib& c, bool) {
@@ -1480,11 +1538,7 @@ struct DeltaVisitT {
             az = __fmaf_rn(c.coef, c.rz, az);
             if constexpr (!kKnow) aw = __fmaf_rn(c.coef, c.rw, aw);
         }
-        if (c.c) {
-            pacc.x = __fmaf_rn(-c.rx, c.t, pacc.x); xacc.x = __fmaf_rn(-c.rx, c.t, xacc.x);
-            pacc.y = __fmaf_rn(-c.ry, c.t, pacc.y); xacc.y = __fmaf_rn(-c.ry, c.t, xacc.y);
-            pacc.z = __fmaf_rn(-c.rz, c.t, pacc.z); xacc.z = __fmaf_rn(-c.rz, c.t, xacc.z);
-        }
+        if (c.c) add_contact(c.rx, c.ry, c.rz, c.t);
     }
     // the density part predicated (LambdaVisitT::add_if); contacts are rare enough for a branch
     __device__ __forceinline__ void add_if(uint32_t k, uint32_t n, const Contrib& c) {
@@ -1499,10 +1553,40 @@ struct DeltaVisitT {
                 : "+f"(ax), "+f"(ay), "+f"(az), "+f"(aw)
                 : "r"((k < n && c.d) ? 1u : 0u), "f"(c.coef), "f"(c.rx), "f"(c.ry), "f"(c.rz), "f"(c.rw));
         }
-        if (c.c && k < n) {
-            Contrib o = c;
-            o.d = false;
-            add(o, true);
+        if (c.c && k < n) add_contact(c.rx, c.ry, c.rz, c.t);
+    }
+    // LambdaVisitT::add_two; a pass of unknown kind (kDeltaAny) adds every entry by itself
+    static constexpr bool kAddTwo = kKnow;
+    template <bool kContacts>   // some entry of the group is a contact (k0, k1: this one)
+    __device__ __forceinline__ void add_two(uint32_t j0, const float4& p0, bool k0, uint32_t j1, const float4& p1, bool k1) {
+        float x[2], y[2], z[2], d[2], a[2], c[2], s[2], l[2];
+        f2_split(sub2(f2(pi.x, pi.y), f2(p0.x, p0.y)), x[0], y[0]);
+        f2_split(sub2(f2(pi.x, pi.y), f2(p1.x, p1.y)), x[1], y[1]);
+        z[0] = pi.z - p0.z; z[1] = pi.z - p1.z;
+        const float r0 = dist2(x[0], y[0], z[0]), r1 = dist2(x[1], y[1], z[1]);
+        d[0] = sqrt_fast(r0); d[1] = sqrt_fast(r1);
+        const F2 dd = f2(d[0], d[1]), aa = sub2(f2(P.hs, P.hs), dd);
+        const F2 ss = spiky_open(P, aa, f2(rsqrt_fast(r0), rsqrt_fast(r1)));
+        const F2 q = mul2(poly6_open(P, dd), f2(P.inv_wq, P.inv_wq));
+        f2_split(mul2(f2(-P.k_scorr, -P.k_scorr), mul2(mul2(mul2(q, q), q), q)), c[0], c[1]);
+        f2_split(aa, a[0], a[1]);
+        l[0] = __fadd_rn(li, p0.w); l[1] = __fadd_rn(li, p1.w);   // w: the entry's lambda
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+            asm("{ .reg .pred q; setp.gt.f32 q, %1, %2; setp.lt.and.f32 q, %1, %3, q; @q add.rn.f32 %0, %0, %4; }"
+                : "+f"(l[b]) : "f"(d[b]), "f"(0.001f), "f"(P.hp_lim), "f"(c[b]));
+        f2_split(mul2(f2(l[0], l[1]), ss), c[0], c[1]);
+        f2_split(ss, s[0], s[1]);
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+            asm("{ .reg .pred q; setp.gt.f32 q, %3, %5; setp.gt.and.f32 q, %4, %5, q; setp.neu.and.f32 q, %6, 0f00000000, q;"
+                " @q fma.rn.f32 %0, %7, %8, %0; @q fma.rn.f32 %1, %7, %9, %1; @q fma.rn.f32 %2, %7, %10, %2; }"
+                : "+f"(ax), "+f"(ay), "+f"(az)
+                : "f"(d[b]), "f"(a[b]), "f"(0.0001f), "f"(s[b]), "f"(c[b]), "f"(x[b]), "f"(y[b]), "f"(z[b]));
+        if constexpr (kContacts) {
+            float t;
+            if (k0 && contact_t(j0, d[0], t)) add_contact(x[0], y[0], z[0], t);
+            if (k1 && contact_t(j1, d[1], t)) add_contact(x[1], y[1], z[1], t);
         }
     }
     // walk_group_sums: the density part's sums, then the contacts' on p* and x, from coef, -t and r
@@ -1595,8 +1679,8 @@ __device__ __noinline__ void coop_delta(const DevParams& P, uint32_t mode, const
 // mode fixed at compile time (the two passes of a fluid frame), kMode = 0: `mode` at run time; kKnown:
 // what else is fixed (DeltaKnown).
 // Blocks of 256 per SM by the list it walks (1M particles, GB300): 6 over the near lists (31.3 us;
-// 5 33.2), 4 over the full lists, whose groups of four entries take 64 registers (275 us; 5 360 with
-// spills, 3 282).
+// 5 33.2), 4 over the full lists, whose groups of four entries take 64 registers (185 us; 5 210 with
+// spills, 3 186).
 template <uint32_t kMode, bool kFull, uint32_t kKnown>
 __global__ void __launch_bounds__(256, kFull ? 4 : 6)
 delta_list_kernel(const __grid_constant__ DevParams P, uint32_t mode_rt, const float4* __restrict__ pin, const float4* __restrict__ pa,

@@ -303,3 +303,20 @@ def test_list_columns_bit_identical_to_full_walk(need_gpu, pbd, scenes, radius, 
     a = _run(pbd, params, pos, vel, 2)
     b = _run(pbd, params, pos, vel, 2, full_walk=True)
     _same(a, b)
+
+
+@pytest.mark.parametrize("collision_type", [0, 1])
+def test_two_entries_at_a_time_bit_identical_to_full_walk(need_gpu, pbd, scenes, collision_type):
+    """lambda and delta over full lists take two entries per call and test each kernel's range where its
+    term is added: pairs on both sides of every limit, pairs at one place, rows of every remainder"""
+    params = scenes.workload_params(pbd, 64, 1995.0, vorticity=0.0005, viscosity=0.00015)
+    params.lambda_epsilon = 0.1
+    params.collision_type = collision_type
+    params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 2.1, 2.0, 2
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(29, 31, 30, origin=(8.0, 8.0, 8.0), spacing=0.93, seed=27)
+    gaps = np.array([0.0, 1e-5, 2e-5, 9.99e-5, 1e-4, 1.01e-4, 9.99e-4, 1e-3, 1.01e-3, 0.5, 1.0, 1.9998, 1.9999, 2.0, 2.0989, 2.099, 2.1, 2.1002], np.float32)
+    a = np.arange(0, len(pos) - 1, 3)
+    pos[a + 1, :3] = pos[a, :3]
+    pos[a + 1, a % 3] += gaps[a // 3 % len(gaps)]
+    _same(_run(pbd, params, pos, vel, 2), _run(pbd, params, pos, vel, 2, full_walk=True))
