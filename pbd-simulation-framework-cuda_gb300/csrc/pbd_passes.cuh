@@ -578,14 +578,13 @@ __device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t 
             constexpr bool kC = decltype(contacts)::value;
             vis.template add_two<kC>(j[0], pj[0], kb < nc, j[1], pj[1], kb + 1u < nc);
             vis.template add_two<kC>(j[2], pj[2], kb + 2u < nc, j[3], pj[3], kb + 3u < nc);
-            kb += 4u;
-            return;
-        }
+        } else {
 #pragma unroll
-        for (uint32_t b = 0; b < 4u; ++b) {
-            const bool contact = decltype(contacts)::value && kb + b < nc;
-            if constexpr (AddIf<V>::value) vis.add_if(kb + b, n, contrib_of(vis, j[b], pj[b], ex[b], contact));
-            else if (kb + b < n) vis.add(contrib_of(vis, j[b], pj[b], ex[b], contact), contact);
+            for (uint32_t b = 0; b < 4u; ++b) {
+                const bool contact = decltype(contacts)::value && kb + b < nc;
+                if constexpr (AddIf<V>::value) vis.add_if(kb + b, n, contrib_of(vis, j[b], pj[b], ex[b], contact));
+                else if (kb + b < n) vis.add(contrib_of(vis, j[b], pj[b], ex[b], contact), contact);
+            }
         }
         kb += 4u;
     };
