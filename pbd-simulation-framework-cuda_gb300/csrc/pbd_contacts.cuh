@@ -242,10 +242,9 @@ __device__ __forceinline__ unsigned long long claim_entries_warp(const DevParams
 
 // Each pending overlapping constraint offers its key to both of its particles.  The first
 // kClaimCoopBlocks blocks take the long lists, a warp each; the others take every other particle, a
-// thread each.  Four blocks of 256 per SM, whose positions and lists the L1 holds better than more
-// blocks' (a stabilization pass of 16 batches with 262,144 particles: 467 us; 5 and 6 blocks 500, 8 524;
-// eight entries per step instead of four 488).
-__global__ void __launch_bounds__(256, 4)
+// thread each.  kPerSm blocks of 256 per SM (claim_blocks_per_sm).
+template <int kPerSm>
+__global__ void __launch_bounds__(256, kPerSm)
 contact_claim_kernel(DevParams P, ContactStore C, const float4* __restrict__ p, const float* __restrict__ w) {
     if (blockIdx.x < kClaimCoopBlocks) {
         const uint32_t nl = *C.long_count;
@@ -268,6 +267,16 @@ contact_claim_kernel(DevParams P, ContactStore C, const float4* __restrict__ p, 
     if (n > kClaimLong) return;                  // a long list: a leading block's warp takes it
     const unsigned long long own = claim_entries(P, C, p, w, i, n);
     if (own) atomicMax(C.best + i, own);
+}
+
+// Four blocks per SM have the L1 to themselves, whose hits the pass lives on; six run it in fewer waves and
+// hide the L2's and memory's latency.  So four where they need at most two waves, and no more than six
+// would.  Ten frames of 16 batches, ms per frame, four / six: 130,000 particles (1 wave each) 1.28 / 1.31,
+// 175,616 (2, 1) 1.94 / 1.64, 262,144 (2, 2) 2.17 / 2.37, 323,680 (3, 2) 2.69 / 2.63, 512,000 (4, 3)
+// 4.22 / 3.98, 1,000,000 (7, 5) 7.63 / 6.94.
+inline int claim_blocks_per_sm(uint32_t blocks, uint32_t sms) {
+    const uint32_t w4 = (blocks + 4u * sms - 1u) / (4u * sms), w6 = (blocks + 6u * sms - 1u) / (6u * sms);
+    return (w4 <= 2u && w4 <= w6) ? 4 : 6;
 }
 
 // A constraint both of whose particles took it is solved by its partner's thread: the key holds

@@ -589,13 +589,15 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             ContactStore C = s->ct;
             unsigned long long* const keys[2] = {s->ct.best, s->ct.best + s->ct.stride};
             const size_t words = (C.M + 31) / 32;
+            const uint32_t claim_blocks = kClaimCoopBlocks + div_up(N, kThreadsParticle);
+            const auto claim = claim_blocks_per_sm(claim_blocks, (uint32_t)s->num_sms) == 4 ? contact_claim_kernel<4> : contact_claim_kernel<6>;
             for (uint32_t k = 0; k < Sx; ++k) {
                 PROF_BEGIN("contact_batches");
                 cudaMemsetAsync(C.solved, 0, words * C.stride * 4, st);
                 for (uint32_t b = 0; b < prm.max_collision_batches; ++b, ++nbatch) {
                     C.best = keys[nbatch & 1u];
                     C.best_next = keys[(nbatch + 1u) & 1u];
-                    contact_claim_kernel<<<kClaimCoopBlocks + div_up(N, kThreadsParticle), kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], wf);
+                    claim<<<claim_blocks, kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], wf);
                     contact_solve_kernel<<<div_up(N, kThreadsParticle), kThreadsParticle, 0, st>>>(P, C, s->p[cur.p], s->x[cur.x], wf);
                     nl += 2;
                 }

@@ -145,3 +145,22 @@ def test_gpu_contact_batches_lists_match_cell_walk(need_gpu, pbd, scenes):
     assert np.array_equal(out[0]["ids"], out[1]["ids"])
     for k in ("x", "v"):
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_side", [42, 43])
+def test_gpu_contact_batches_both_claim_variants(need_gpu, pbd, scenes, n_side):
+    """the claim pass runs with 4 blocks per SM while one wave holds them, with 6 from 155,000 particles
+    on: 148,176 and 159,014 particles in isolated pairs.  Tolerance: coordinates up to 126 round by at
+    most 3.9e-6 per particle, axis and batch; four batches of two particles, sqrt(3): 5.4e-5"""
+    p, _, _ = pair_scene(pbd, scenes)
+    q = scenes.workload_params(pbd, 128, 1000.0, iterations=1)
+    q.collision_type, q.max_collision_batches, q.gravity = 1, 4, 0.0
+    q.flags, q.active = p.flags, p.active
+    _, pos, vel = pair_scene(pbd, scenes, n_side=n_side, spacing=2.8)
+    with pbd.Sim(q, len(pos)) as sim:
+        sim.add_particles(pos, vel)
+        sim.step(1)
+        x = by_id(sim.state())["x"]
+    r = np.linalg.norm(x[0::2, :3].astype(np.float64) - x[1::2, :3], axis=1)
+    assert np.allclose(r, 0.964, atol=6e-5)
