@@ -851,7 +851,7 @@ __device__ __forceinline__ bool push_runs(const DevParams& P, uint32_t i, const 
 // other than 1 can break it) each such pair is one run and the column has 2 to 4, else a run per cell.
 // A column with a range longer than kLongRange, the cell-end range, or near the cap or the list's room
 // goes cell by cell.  (One loop per cell, each with its checks, was 604 us for 1M dense particles, this
-// is 451; for 27 cells 154 -> 143.)  Returns true when the walk ends here (cap reached or handed over).
+// 451; for 27 cells 154 -> 143.  With the sums' two-float arithmetic the pass takes 409 and 138.)  Returns true when the walk ends here (cap reached or handed over).
 template <int kCells>
 __device__ __forceinline__ bool store_column(const DevParams& P, const SceneCtx& S, uint32_t i, const uint32_t* h,
                                              bool odd, bool consecutive, const uint32_t* __restrict__ cs,
@@ -1189,7 +1189,7 @@ struct LambdaVisitT {
 using LambdaVisit = LambdaVisitT<false>;
 
 template <bool kUnitW>
-__global__ void __launch_bounds__(256, 4)   // 5 (48 registers) spills: 622 -> 649 us on the 1M dense frame
+__global__ void __launch_bounds__(256, 4)   // 5 (48 registers) spills: 4% slower on 1M dense particles
 lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const uint32_t* __restrict__ cs,
               const uint32_t* __restrict__ ce, float* __restrict__ lambda, DeferList D, float4* __restrict__ aux,
               NbList L, NbList F, DeferList DF, DeferList DN, uint32_t long_slots, float4* __restrict__ pl) {
@@ -1234,8 +1234,8 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         else if (listed) walk_full<true>(F, i, fm, p, vis);
         else walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
         const float li = vis.finish(S.rho0);
-            lambda[i] = li;
-            if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
+        lambda[i] = li;
+        if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
         if (aux) vis.store_aux(aux, P.N, i);
         return;
     } else if (L.list) {
@@ -1263,8 +1263,8 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         walk_seq(P, S, i, pa[i], p, cs, ce, vis, false, &deferred);
     }
     const float li = vis.finish(S.rho0);
-            lambda[i] = li;
-            if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
+    lambda[i] = li;
+    if (pl) pl[i] = make_float4(pi.x, pi.y, pi.z, li);
     if (aux) vis.store_aux(aux, P.N, i);
 }
 
@@ -1330,7 +1330,7 @@ lambda_long_kernel(const __grid_constant__ DevParams P, const float4* __restrict
 // without a near list are noted in DN for the delta pass.  Kept apart from lambda_kernel so that
 // its register budget is the list walk's alone.
 // kNear: with near lists (L).  Blocks of 256 per SM: 6 with them (62 us with 1M particles; 5 66, 4 74), 5
-// over full lists (183 us with 1M dense particles; 6 201).
+// over full lists (147 us with 1M dense particles; 4 155, 6 167).
 template <bool kUnitW, bool kNear>
 __global__ void __launch_bounds__(256, kNear ? 6 : 5)
 lambda_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa,
@@ -1868,8 +1868,8 @@ __device__ __noinline__ void coop_omega(const DevParams& P, const float4* __rest
 // omega over the full list (recording the near list when L.list, and noting the particles left
 // without one in DN when DN is given); the particles without a full list (the set C) are walked
 // by the leading blocks.
-// kNear: the pass filters the full list into omega's near list (5 blocks of 256 per SM: 80 us with 1M
-// particles; 4 and 6 88); else it walks the full list (4: 211 us; 3 219, 5 230).
+// kNear: the pass filters the full list into omega's near list (5 blocks of 256 per SM: 69 us with 1M
+// particles; 4 76, 6 71); else it walks the full list (4: 205 us; 3 and 5 4 to 9% slower).
 template <bool kNear, bool kUnitW>
 __global__ void __launch_bounds__(256, kNear ? 5 : 4)
 omega_list_kernel(const __grid_constant__ DevParams P, const float4* __restrict__ p, const float4* __restrict__ pa, const float4* __restrict__ v,
@@ -2125,7 +2125,7 @@ __device__ __noinline__ void coop_vort_visc(const DevParams& P, const float4* __
 // viscosity over the near list (its entries beyond the cut add exact zeros): the two sums keep
 // their own order.
 // Blocks of 256 per SM: with viscosity over omega's near list 4 (113 us with 1M particles; 3 119, 5 141);
-// both terms over the full list's groups 3 (80 registers: 367 us; 2 400, 4 536 with spills).
+// both terms over the full list's groups 3 (80 registers: 340 us; 2 9% slower, 4 46% with spills).
 enum VortViscLists : uint32_t { kVortViscFull, kVortVisc, kViscNear };   // Lv, Ln: full, none; full, near; near, none
 template <uint32_t kLists>
 __global__ void __launch_bounds__(256, kLists == kVortViscFull ? 3 : 4)

@@ -61,7 +61,7 @@ struct Cur {
     bool operator==(const Cur& o) const { return x == o.x && p == o.p && v == o.v; }
 };
 constexpr int kMaxGraphs = 8;
-// Stored list capacities (slot-major, only the used slots are touched).  A particle whose list
+// Stored list capacities (only the used slots are touched).  A particle whose list
 // is longer goes to the warp-cooperative cell walk.
 constexpr uint32_t kListMax = 64;    // near list: entries within the cut
 constexpr uint32_t kFullMax = 255;   // full list: every entry of the frame's list (meta holds 8-bit counts)
