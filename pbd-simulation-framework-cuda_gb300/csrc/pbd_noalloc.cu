@@ -156,6 +156,15 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
     }
     S.key_bits = key_bits;
 
+    if (n <= kSortSmall && !S.hold) {
+        sort_small(st, d_keys_in, d_keys_out, d_perm_out, n, npasses, key_bits, S.err);
+        if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
+            set_error(std::string("pbd_sort_keys_noalloc: launch: ") + cudaGetErrorString(e));
+            return PBD_ERR_CUDA;
+        }
+        return PBD_OK;
+    }
+
     const uint32_t gh = std::min<uint32_t>((n + 2047) / 2048, 2u * kSortSpread);
     noalloc_hist_kernel<<<gh, 512, 0, st>>>(d_keys_in, n, base, plan.ntiles, npasses, key_bits);
     // Ping-pong between the caller's outputs and the fixed array so that the last pass

@@ -436,7 +436,12 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     // sortIds
     const SortPlan plan = sort_plan(N);
     const uint32_t ntiles = plan.ntiles;
-    for (int pass = 0; pass < np; ++pass) {
+    if (N <= kSortSmallFrame && !s->sort_hold) {
+        PROF_BEGIN("sort_small");
+        sort_small(st, s->keys[0], s->keys[np % 2], s->vals[np % 2], N, np, S.key_bits, nullptr);
+        PROF_END();
+        ++nl;
+    } else for (int pass = 0; pass < np; ++pass) {
         const int in = pass % 2, out = (pass + 1) % 2;
         PROF_BEGIN("onesweep_pass");
         sort_pass(st, plan, s->keys[in], s->vals[in], s->keys[out], s->vals[out], N, pass, S);

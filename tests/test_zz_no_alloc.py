@@ -122,3 +122,49 @@ def test_noalloc_sort_of_keys_at_any_word(need_gpu, pbd, offset, n):
         pbd.check(pbd.lib().pbd_sort_keys_noalloc(d.data_ptr(), out.data_ptr(), perm.data_ptr(), n, 21, None))
         assert pbd.lib().pbd_sort_noalloc_status(None) == pbd.OK
         assert np.array_equal(perm.cpu().numpy().view(np.uint32), order.astype(np.uint32))
+
+
+@pytest.mark.parametrize("key_bits", [1, 9, 21, 32])
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025, 2048, 2049, 4095, 4096, 4097])
+def test_noalloc_sort_of_few_keys_by_one_block(need_gpu, pbd, n, key_bits):
+    # up to 4,096 keys one block runs all passes, with 1, 2 or 4 keys per thread; bits above key_bits stay out
+    rng = np.random.default_rng(n + key_bits)
+    keys = (rng.integers(0, 1 << 32, size=n, dtype=np.uint64) & 0xFFFF00FF).astype(np.uint32)
+    order = np.argsort(keys & np.uint32((1 << key_bits) - 1), kind="stable")
+    k, p = _sort_noalloc(pbd, keys, key_bits=key_bits)
+    assert np.array_equal(p, order.astype(np.uint32)) and np.array_equal(k, keys[order])
+
+
+def test_noalloc_status_is_of_the_last_call_also_for_few_keys(need_gpu, pbd):
+    L = pbd.lib()
+    many, few = (np.random.default_rng(s).integers(0, 1 << 24, size=s, dtype=np.uint64).astype(np.uint32) for s in (50000, 500))
+    try:
+        pbd.check(L.pbd_debug_set_wait_limit(None, 2000, 1))
+        _sort_noalloc(pbd, many)
+        assert L.pbd_sort_noalloc_status(None) == pbd.ERR_TIMEOUT
+    finally:
+        pbd.check(L.pbd_debug_set_wait_limit(None, 0, 0))
+    for keys in (few, many):
+        k, _ = _sort_noalloc(pbd, keys)
+        assert L.pbd_sort_noalloc_status(None) == pbd.OK
+        assert np.array_equal(k, np.sort(keys))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (8, 8, 16), (5, 5, 41), (16, 16, 8), (3, 683, 1)])
+@pytest.mark.parametrize("forces", [True, False])
+def test_step_sort_of_few_particles_by_one_block(need_gpu, pbd, scenes, shape, forces):
+    # 1, 1,024, 1,025, 2,048 and 2,049 particles (the last by the tiles' passes), 3 and 4 passes
+    params = scenes.workload_params(pbd, 128, 1000.0)
+    if not forces:
+        params.active &= ~pbd.ACTIVE["applyForces"]
+    pos, vel = scenes.lattice(*shape, spacing=0.15 if max(shape) > 100 else 0.9, seed=28)
+    pos, vel = pos[::-1].copy(), vel[::-1].copy()
+    with pbd.Sim(params, len(pos)) as sim:
+        sim.add_particles(pos, vel)
+        sim.front()
+        d = sim.debug()
+    keys, perm = d["keys"], d["perm"].astype(np.int64)
+    assert np.array_equal(np.sort(perm), np.arange(len(pos)))
+    before = np.empty_like(keys)
+    before[perm] = keys
+    assert np.array_equal(np.argsort(before, kind="stable"), perm)
