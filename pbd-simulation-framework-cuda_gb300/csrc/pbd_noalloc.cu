@@ -9,11 +9,11 @@
 //
 // The working memory is the file-scope array below: kNoAllocMaxKeys keys at most
 // (1,048,576), kScratchWords * 4 = 9,441,536 bytes (9.0 MiB).  Every GPU that loads the library
-// keeps that array until the process exits.  All calls share it: each call zeroes the parts that must
-// start at zero, the digit counts at its end and the rest at its start; calls whose GPU work
-// overlaps (different streams, or different host threads) race on it and must be serialised by
-// the caller.  Its error word holds the outcome of the last call on the device:
-// pbd_sort_noalloc_status reads it.
+// keeps that array until the process exits.  All calls share it and it keeps the last call's
+// contents, so each call first zeroes the parts that must start at zero and relies on nothing that an
+// earlier call, finished or not, left there; calls whose GPU work overlaps (different streams, or
+// different host threads) race on it and must be serialised by the caller.  Its error word holds the
+// outcome of the last call on the device: pbd_sort_noalloc_status reads it.
 //
 // Host code cannot use the array's name as a device address.  The first call on each device,
 // with that device current, looks the address up with cudaGetSymbolAddress and caches it;
@@ -44,8 +44,7 @@ constexpr size_t kOffHist = kOffVals + kNoAllocMaxKeys;
 constexpr size_t kOffStatus = kOffHist + (size_t)kMaxPasses * kRadix;
 constexpr size_t kOffTiles = kOffStatus + (size_t)kMaxPasses * kNoAllocMaxTiles * kRadix;
 constexpr size_t kOffErr = kOffTiles + kMaxPasses;
-constexpr size_t kOffDone = kOffErr + 1;   // finished tiles of a sort's last pass
-constexpr size_t kScratchWords = (kOffDone + 1 + 63) & ~size_t(63);
+constexpr size_t kScratchWords = (kOffErr + 1 + 63) & ~size_t(63);
 
 static_assert(kScratchWords * 4 == 9441536, "the fixed array's size is stated in pbd.h");
 static __device__ __align__(256) uint32_t g_sort_scratch[kScratchWords];
@@ -57,12 +56,20 @@ uint32_t* g_scratch_ptr[kMaxDevices] = {};
 uint32_t g_spin_limit = kSpinLimit;
 uint32_t g_hold = 0;
 
+// Zero the histograms, the tile counters and the error word: 2 us of a call (1,048,576 keys 64 -> 66 us).  The
+// last tile of a call could leave them zero for the next one, but then a call that did not finish would
+// spoil every later one.
+__global__ void __launch_bounds__(kMaxPasses * kRadix)
+noalloc_clear_kernel(uint32_t* base) {
+    base[kOffHist + threadIdx.x] = 0u;
+    if (threadIdx.x < kMaxPasses) base[kOffTiles + threadIdx.x] = 0u;
+    if (threadIdx.x == 0) base[kOffErr] = 0u;
+}
+
 // Digit histograms of every pass (the sim counts them in its predict kernel), after zeroing the look-back
-// rows the call will use, the tile counters and the error word.  The histograms are zero when a call
-// starts: the array starts as zeros and every sort's last tile zeroes them (SortScratch::done).  Two
-// blocks of 512 per SM and keys four at a time where they are aligned: with 1,024 blocks of 256 the
-// flush of the blocks' histograms took most of the time (with the clearing kernel before it 16 us for
-// 1,048,576 keys).
+// rows the call will use.  Two blocks of 512 per SM and keys four at a time where they are aligned: with
+// 1,024 blocks of 256 the flush of the blocks' histograms took most of the time (with the clearing kernel
+// before it 16 us for 1,048,576 keys).
 __global__ void __launch_bounds__(512)
 noalloc_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* base, uint32_t ntiles, int npasses,
                     uint32_t key_bits) {
@@ -72,8 +79,6 @@ noalloc_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* bas
     for (int pass = 0; pass < npasses; ++pass)
         for (uint32_t k = t; k < ntiles * kRadix; k += stride)
             base[kOffStatus + (size_t)pass * kNoAllocMaxTiles * kRadix + k] = 0u;
-    if (t < kMaxPasses) base[kOffTiles + t] = 0u;
-    if (t == 0) base[kOffErr] = 0u;
     __syncthreads();
     const uint32_t n4 = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u ? n / 4u : 0u;
     const uint32_t warp0 = t & ~31u;
@@ -166,6 +171,7 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
     }
 
     const uint32_t gh = std::min<uint32_t>((n + 2047) / 2048, 2u * kSortSpread);
+    noalloc_clear_kernel<<<1, kMaxPasses * kRadix, 0, st>>>(base);
     noalloc_hist_kernel<<<gh, 512, 0, st>>>(d_keys_in, n, base, plan.ntiles, npasses, key_bits);
     // Ping-pong between the caller's outputs and the fixed array so that the last pass
     // writes the outputs: pass p writes the outputs when (npasses - 1 - p) is even.
@@ -177,7 +183,6 @@ extern "C" int pbd_sort_keys_noalloc(const uint32_t* d_keys_in, uint32_t* d_keys
         const bool to_out = ((npasses - 1 - pass) % 2) == 0;
         uint32_t* dk = to_out ? d_keys_out : tmp_k;
         uint32_t* dv = to_out ? d_perm_out : tmp_v;
-        if (pass == npasses - 1) S.done = base + kOffDone;
         sort_pass(st, plan, src_k, src_v, dk, dv, n, pass, S);
         src_k = dk;
         src_v = dv;

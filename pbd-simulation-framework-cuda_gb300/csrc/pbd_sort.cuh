@@ -76,7 +76,6 @@ struct SortScratch {
     uint32_t max_tiles;
     uint32_t spin_limit = kSpinLimit;   // polls of one look-back wait before it gives up
     uint32_t hold = 0;                  // 1: the first tile of each pass never publishes (tests)
-    uint32_t* done = nullptr;           // given to a sort's last pass: its last tile zeroes hist and this word
     uint32_t key_bits = 32;             // only bits [0, key_bits) order the keys
 };
 
@@ -263,15 +262,6 @@ onesweep_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin
             vout[o] = s_vals[i];
         }
     }
-    if (S.done) {   // every tile has read its counts: the last one leaves them zero for the next sort
-        __syncthreads();
-        if (tid == 0) s_tile = atomicAdd(S.done, 1u);
-        __syncthreads();
-        if (s_tile == gridDim.x - 1) {
-            for (int b = tid; b < kMaxPasses * kRadix; b += kThreads) S.hist[b] = 0u;
-            if (tid == 0) *S.done = 0u;
-        }
-    }
 }
 
 template <int kItems>
@@ -387,10 +377,10 @@ sort_small_kernel(const uint32_t* kin, uint32_t* kout, uint32_t* vout, uint32_t 
         vout[i] = s_vals[i];
     }
 }
-// Most keys of one block's sort.  A sort by itself (three passes, 21 bits): 1,000 keys 18 -> 6.8 us, 4,000
-// 22.5 -> 14.3, but 6,000 22.5 against 20.5 and 8,192 22.5 the same.  Inside a frame, where the passes
-// overlap their launches and the histogram comes with the keys: 1,000 particles 47.0 -> 43.6 us per
-// frame, 2,016 48.1 -> 45.4, but 4,096 68.7 against 70.5.
+// Most keys of one block's sort.  A sort by itself (three passes, 21 bits), the tiles' passes against one
+// block: 1,000 keys 20 / 6.8 us, 4,000 24 / 14.3, 8,192 24.6 / 22.5 with eight keys per thread, 12,000 more
+// than the tiles' time.  Inside a frame, where the passes overlap their launches and the histogram comes
+// with the keys: 1,000 particles 47.0 -> 43.6 us per frame, 2,016 48.1 -> 45.4, but 4,096 68.7 against 70.5.
 constexpr uint32_t kSortSmall = 4096;
 constexpr uint32_t kSortSmallFrame = 2048;
 template <int kItems>

@@ -168,3 +168,49 @@ def test_step_sort_of_few_particles_by_one_block(need_gpu, pbd, scenes, shape, f
     before = np.empty_like(keys)
     before[perm] = keys
     assert np.array_equal(np.argsort(before, kind="stable"), perm)
+
+
+def _cut_short(pbd, keys, key_bits):
+    """A sort whose last pass never runs: the call recorded as a graph, its last node taken out."""
+    import torch
+    rt = C.CDLL("libcudart.so.13")
+    d = torch.tensor(keys.view(np.int32), device="cuda")
+    out, perm = torch.empty_like(d), torch.empty_like(d)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    graph, exe, count = C.c_void_p(), C.c_void_p(), C.c_size_t()
+    st = C.c_void_p(stream.cuda_stream)
+    assert rt.cudaStreamBeginCapture(st, 1) == 0
+    rc = pbd.lib().pbd_sort_keys_noalloc(d.data_ptr(), out.data_ptr(), perm.data_ptr(), len(keys), key_bits, st)
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0 and rc == pbd.OK
+    assert rt.cudaGraphGetNodes(graph, None, C.byref(count)) == 0
+    nodes = (C.c_void_p * count.value)()
+    assert rt.cudaGraphGetNodes(graph, nodes, C.byref(count)) == 0
+    last = []
+    for node in nodes:
+        after = C.c_size_t()
+        assert rt.cudaGraphNodeGetDependentNodes(C.c_void_p(node), None, None, C.byref(after)) == 0
+        if after.value == 0:
+            last.append(node)
+    assert len(last) == 1 and count.value > 2
+    assert rt.cudaGraphDestroyNode(C.c_void_p(last[0])) == 0
+    assert rt.cudaGraphInstantiate(C.byref(exe), graph, C.c_ulonglong(0)) == 0
+    assert rt.cudaGraphLaunch(exe, st) == 0
+    stream.synchronize()
+    rt.cudaGraphExecDestroy(exe)
+    rt.cudaGraphDestroy(graph)
+
+
+@pytest.mark.parametrize("n,after", [(50000, 30000), (30000, 50000), (1 << 20, 5000), (5000, 1 << 20)])
+def test_noalloc_sort_after_a_call_that_did_not_finish(need_gpu, pbd, n, after):
+    # a call leaves nothing that the next one relies on: when its last pass never ran (a launch that
+    # failed), the next sort, of more or of fewer tiles, and the one after it are right all the same
+    rng = np.random.default_rng(n)
+    first, second = (rng.integers(0, 1 << 21, size=k, dtype=np.uint64).astype(np.uint32) for k in (n, after))
+    _sort_noalloc(pbd, first, key_bits=21)
+    _cut_short(pbd, first, 21)
+    for keys in (second, first):
+        k, p = _sort_noalloc(pbd, keys, key_bits=21)
+        order = np.argsort(keys, kind="stable")
+        assert np.array_equal(p, order.astype(np.uint32)) and np.array_equal(k, keys[order])
+        assert pbd.lib().pbd_sort_noalloc_status(None) == pbd.OK
