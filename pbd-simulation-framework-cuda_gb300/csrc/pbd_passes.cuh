@@ -540,9 +540,13 @@ template <class V> struct AddIf<V, std::void_t<decltype(&V::add_if)>> : std::tru
 // passes are bound by instruction issue and the gathers together: 54 -> 43 instructions per entry for
 // delta and 43 -> 31 for lambda made them 211 -> 185 and 169 -> 147 us (1M particles, ~124 entries;
 // positions loaded a group ahead instead: 210 and 180, the registers cost warps).  i itself as an entry
-// must add nothing to its sums.
+// must add nothing to its sums; where it might (self_adds), the list is summed once more, entry by entry (after
+// the loop, where it costs nothing: as a second loop for the last group lambda took 154 us, as a test of
+// every entry 165).
 template <class V, class = void> struct AddTwo : std::false_type {};
 template <class V> struct AddTwo<V, std::void_t<decltype(V::kAddTwo)>> : std::bool_constant<V::kAddTwo> {};
+template <class V, class = void> struct SelfAdds : std::false_type {};
+template <class V> struct SelfAdds<V, std::void_t<decltype(&V::self_adds)>> : std::true_type {};
 // A visitor with load(j, pj, ex) takes an entry's position and extra data from an array of its own.
 template <class V, class = void> struct OwnLoad : std::false_type {};
 template <class V> struct OwnLoad<V, std::void_t<decltype(&V::load)>> : std::true_type {};
@@ -598,6 +602,16 @@ __device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t 
     } else {
 #pragma unroll 1
         while (kb < n) group(std::true_type{});
+        if constexpr (SelfAdds<V>::value) {
+            if (vis.self_adds()) {
+                vis.reset();
+#pragma unroll 1
+                for (uint32_t k = 0; k < n; ++k) {
+                    const uint32_t j = *full_at(F, i, k);
+                    vis.add(contrib_of(vis, j, __ldg(p + j), fetch_extra(vis, j), k < nc), k < nc);
+                }
+            }
+        }
     }
     vis.end_contacts(nc);
 }
@@ -1122,8 +1136,11 @@ struct LambdaVisitT {
                 : "+f"(Cw) : "r"(k), "r"(n), "f"(c.r2), "f"(P.cut2), "f"(c.s), "f"(c.rw));
     }
     // The kernels are tested where they are added: within spiky's range (or NaN, which add() passes on)
-    // r^2 < cut2 holds, and i itself (r = 0) is in neither range.
+    // r^2 < cut2 holds, and i itself (r = 0) is in neither range unless its position is infinite (r NaN).
     static constexpr bool kAddTwo = true;
+    __device__ __forceinline__ bool self_adds() const {
+        return !(fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z) < __int_as_float(0x7f800000));
+    }
     template <bool>
     __device__ __forceinline__ void add_two(uint32_t, const float4& p0, bool, uint32_t, const float4& p1, bool) {
         float x[2], y[2], z[2], w[2], d[2], a[2], W[2], s[2], B2[2];
@@ -1554,7 +1571,8 @@ struct DeltaVisitT {
         }
         if (c.c && k < n) add_contact(c.rx, c.ry, c.rz, c.t);
     }
-    // LambdaVisitT::add_two; a pass of unknown kind (kDeltaAny) adds every entry by itself
+    // LambdaVisitT::add_two (a NaN adds nothing here, so i itself never does); a pass of unknown kind
+    // (kDeltaAny) adds every entry by itself
     static constexpr bool kAddTwo = kKnow;
     template <bool kContacts>   // some entry of the group is a contact (k0, k1: this one)
     __device__ __forceinline__ void add_two(uint32_t j0, const float4& p0, bool k0, uint32_t j1, const float4& p1, bool k1) {

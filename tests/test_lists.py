@@ -320,3 +320,34 @@ def test_two_entries_at_a_time_bit_identical_to_full_walk(need_gpu, pbd, scenes,
     pos[a + 1, :3] = pos[a, :3]
     pos[a + 1, a % 3] += gaps[a // 3 % len(gaps)]
     _same(_run(pbd, params, pos, vel, 2), _run(pbd, params, pos, vel, 2, full_walk=True))
+
+
+@pytest.mark.parametrize("collision_type", [0, 1])
+def test_infinite_positions_in_the_solver(need_gpu, pbd, scenes, collision_type):
+    """isolated pairs that s_corr (a reference density close to zero) throws to infinity in the first
+    iteration: in the second every entry of a pair's list is out of range, so lambda is 1 / eps for both,
+    whichever way the entries are read (lists of one entry, padded to a group of four with the particle
+    itself, whose difference is inf - inf)"""
+    params = scenes.workload_params(pbd, 128, 1000.0, iterations=2)
+    params.lambda_epsilon = 0.1
+    params.gravity = 0.0
+    params.collision_type = collision_type
+    params.kernel_width_poly, params.kernel_width_spiky, params.q_scorr = 1.6, 1.5, 1.598 / 1.5
+    params.flags &= ~pbd.FLAG_CELL_END_QUIRK
+    g = np.stack(np.meshgrid(*[np.arange(24)] * 3, indexing="ij"), -1).reshape(-1, 3) * 5.0 + 3.0
+    pos = np.zeros((2 * len(g), 4), np.float32)
+    pos[0::2, :3] = g
+    pos[1::2, :3] = g + np.array([0.6, 0.7, 0.75])
+    out = []
+    for flags in (0, pbd.FLAG_FULL_WALK):
+        p = params.copy()
+        p.flags |= flags
+        with pbd.Sim(p, len(pos)) as sim:
+            sim.add_particles(pos, np.zeros_like(pos))
+            sim.step(1)
+            sim.sync()
+            out.append((sim.debug()["lambda"], sim.state()["x"][:, :3]))
+    lists, walk = out
+    assert np.isinf(walk[1]).all()
+    assert np.array_equal(walk[0], np.full(len(pos), np.float32(1) / np.float32(0.1), np.float32))
+    assert np.array_equal(lists[0], walk[0]) and np.array_equal(lists[1], walk[1])
