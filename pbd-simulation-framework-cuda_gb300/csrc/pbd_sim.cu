@@ -134,7 +134,7 @@ struct pbd_sim {
     float4* adj_gom = nullptr;                // with vorticity: each particle's own dL/domega
     bool adj_last_taped = false;   // the tape holds the forward's last segment
     uint64_t gen = 0, adj_gen = 0; // bumped by every call that changes the state or parameters
-    uint64_t pgen = 0;             // bumped by every call that changes the parameters, the use of masses or the block size
+    uint64_t pgen = 0;             // bumped by every call that changes the parameters, the use of masses, the block size or the sort's settings
     int anchor = -1;               // p buffer holding the last frame's anchors (-1: none since the state changed)
     // collisionType 1 workspace (allocated when the parameters select it, never inside a frame)
     void* ct_arena = nullptr;
@@ -1320,7 +1320,8 @@ int pbd_debug_set_wait_limit(pbd_sim* s, uint32_t spins, int hold_first_tile) {
     if (int rc = check_sim(s, "pbd_debug_set_wait_limit")) return rc;
     s->sort_spin_limit = spins ? spins : kSpinLimit;
     s->sort_hold = hold_first_tile ? 1u : 0u;
-    s->dirty = true;   // the frame graphs hold the sort's settings
+    s->dirty = true;   // the frame graphs hold the sort's settings, and so do
+    ++s->pgen;         // the adjoint's recorded segments
     return PBD_OK;
 }
 
@@ -1920,7 +1921,7 @@ static cudaError_t enqueue_segment(pbd_sim* s, cudaStream_t st, Cur& cur, int nf
 }
 
 // Run one adjoint segment from the current buffer record as a recorded graph (recorded on first
-// use and kept while the parameters, N, the block size and the workspace's layout stay the same, also
+// use and kept while the parameters, N, the block size, the sort's settings and the workspace's layout stay the same, also
 // when the particles are set anew: a training loop resets them for every rollout, and recording its
 // segments took 1.8 ms of a 7.3 ms forward and reverse pass of 20 frames of 65,536 particles):
 // kind 0: nf taped forward frames; 1: recompute nf taped frames, then their reverse pass;

@@ -107,3 +107,25 @@ def golden_lists(g):
 
 def scale(a):
     return max(1.0, float(np.max(np.abs(a))))
+
+
+def device_events(fn):
+    """Names of the kernels and copies that fn() has the GPU run (those of graph launches too), as torch's
+    profiler reports them; empty where it reports nothing."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    def traced(f):
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            f()
+            torch.cuda.synchronize()
+        return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+    if not device_events.ready:   # a process's first trace comes back empty
+        traced(lambda: torch.zeros(1, device="cuda"))
+        device_events.ready = True
+    return traced(fn)
+
+
+device_events.ready = False

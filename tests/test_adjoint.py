@@ -609,3 +609,29 @@ def test_gpu_recorded_segments_are_not_mixed_up(need_gpu, pbd, scenes):
         for a, b in zip(*got):
             assert np.array_equal(a, b), (frames, every, n, mass)
     sim.close()
+
+
+@pytest.mark.gpu
+def test_gpu_recorded_segments_follow_the_sort_settings(need_gpu, pbd, scenes):
+    """a segment holds the sort's wait limit and test switch as they were when it was recorded: a rollout
+    after a change of them records again.  Up to 1,024 particles the switch takes a frame's sort to the
+    tiles' passes (one tile, which no other waits for: the same results).  The first eight rollouts record a
+    segment for every set of buffers that one can start from"""
+    from helpers import device_events
+    prm, pos, vel, w = adjoint_scene(pbd, scenes)
+    g = np.zeros((len(pos), 4), np.float32)
+    g[:, :3] = w
+    sorts, grads = [], []
+    with pbd.Sim(prm, len(pos)) as sim:
+        for hold in (0,) * 8 + (1, 1, 0, 0):
+            pbd.check(pbd.lib().pbd_debug_set_wait_limit(sim.h, 0, hold))
+            sim.clear()
+            sim.add_particles(pos, vel)
+            names = device_events(lambda: sim.adjoint_forward(2, 2))
+            sorts.append(any("onesweep_pass" in s for s in names))
+            grads.append(sim.adjoint_backward(g))
+            if not names:
+                pytest.skip("no kernel names on this machine")
+    assert sorts == [False] * 8 + [True, True, False, False]
+    for got in grads[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(got, grads[0]))
