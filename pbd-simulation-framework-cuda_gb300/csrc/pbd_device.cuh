@@ -83,11 +83,13 @@ __device__ __forceinline__ uint32_t coarse_axis(float c) {
 __device__ __forceinline__ uint2 coarse_pos(float4 p) {
     return make_uint2(coarse_axis(p.x) | (coarse_axis(p.y) << 16), coarse_axis(p.z));
 }
-// Whether two coarse positions may be within the cut (limit = near_coarse; 0: never).
-__device__ __forceinline__ bool coarse_near(uint2 a, uint2 b, uint32_t limit) {
-    const uint32_t d = a.x - b.x;
-    const int dx = (int)d >> 16, dy = (int)(int16_t)(d & 0xFFFFu), dz = (int)(a.y - b.y);
-    return (uint32_t)(dx * dx) + (uint32_t)(dy * dy) + (uint32_t)(dz * dz) < limit;
+// Whether two coarse positions may be within the cut (limit = near_coarse; 0: never).  Differences beyond
+// 64 cells (the cell-end range) wrap around, in x and y to a smaller one and in the sum of squares modulo
+// 2^32: such a pair may count as near, which costs an entry and nothing else.
+__host__ __device__ __forceinline__ bool coarse_near(uint2 a, uint2 b, uint32_t limit) {
+    const uint32_t d = a.x - b.x, dz = a.y - b.y;
+    const int dx = (int)d >> 16, dy = (int)(int16_t)(d & 0xFFFFu);
+    return (uint32_t)(dx * dx) + (uint32_t)(dy * dy) + dz * dz < limit;
 }
 
 // The scene a particle belongs to, as the walk and the per-scene constants see it.
