@@ -73,8 +73,8 @@ struct DevParams {
 };
 
 // A position in steps of 1/512 cell, clamped to the 128 cells the enclosure's limits leave (x | y << 16,
-// z); a position that is not a number goes to the far corner, away from every wall.  Two positions
-// closer than the cut are also near by coarse_near: rounding moves a difference by at most 1.01 steps
+// z); a coordinate that is not a number goes to the far end, and the sums leave such an entry out.  Two
+// positions closer than the cut are also near by coarse_near: rounding moves a difference by at most 1.01 steps
 // per axis (clamping by none), coarse_near's packed subtraction another one in x, together 2.5 steps.
 __device__ __forceinline__ uint32_t coarse_axis(float c) {
     const float q = c * 512.0f;

@@ -1124,15 +1124,16 @@ struct LambdaVisitT {
     // add() of entry k when k < n, as predicated instructions: as a branch the compiler moves the
     // contribution's arithmetic into it, and the entries of a group run one after the other. The tests
     // belong to the same block of instructions: as a flag handed to it they cost a select and a compare
-    // per entry more (1M particles, full lists: delta 244 -> 211 us, lambda 173 -> 169).
+    // per entry more (1M particles, full lists: delta 244 -> 211 us, lambda 173 -> 169).  Near lists only: an
+    // entry whose distance is not a number is left out, as the test of exact positions leaves it out.
     __device__ __forceinline__ void add_if(uint32_t k, uint32_t n, const Contrib& c) {
-        asm("{ .reg .pred q; setp.lt.u32 q, %5, %6; setp.ltu.and.f32 q, %7, %8, q;"
+        asm("{ .reg .pred q; setp.lt.u32 q, %5, %6; setp.lt.and.f32 q, %7, %8, q;"
             " @q add.rn.f32 %0, %0, %9; @q add.rn.f32 %1, %1, %10; @q fma.rn.f32 %2, %11, %12, %2;"
             " @q fma.rn.f32 %3, %11, %13, %3; @q fma.rn.f32 %4, %11, %14, %4; }"
             : "+f"(A), "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz)
             : "r"(k), "r"(n), "f"(c.r2), "f"(P.cut2), "f"(c.a), "f"(c.b), "f"(c.s), "f"(c.rx), "f"(c.ry), "f"(c.rz));
         if constexpr (!kUnitW)
-            asm("{ .reg .pred q; setp.lt.u32 q, %1, %2; setp.ltu.and.f32 q, %3, %4, q; @q fma.rn.f32 %0, %5, %6, %0; }"
+            asm("{ .reg .pred q; setp.lt.u32 q, %1, %2; setp.lt.and.f32 q, %3, %4, q; @q fma.rn.f32 %0, %5, %6, %0; }"
                 : "+f"(Cw) : "r"(k), "r"(n), "f"(c.r2), "f"(P.cut2), "f"(c.s), "f"(c.rw));
     }
     // The kernels are tested where they are added: within spiky's range (or NaN, which add() passes on)

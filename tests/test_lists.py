@@ -351,3 +351,26 @@ def test_infinite_positions_in_the_solver(need_gpu, pbd, scenes, collision_type)
     assert np.isinf(walk[1]).all()
     assert np.array_equal(walk[0], np.full(len(pos), np.float32(1) / np.float32(0.1), np.float32))
     assert np.array_equal(lists[0], walk[0]) and np.array_equal(lists[1], walk[1])
+
+
+def test_near_lists_leave_out_positions_that_are_not_numbers(need_gpu, pbd, scenes):
+    """a pair in line with the x axis that s_corr throws to (+-inf, NaN, NaN) in the first iteration, beside a
+    particle in the enclosure's far corner, where the coarse position of a NaN lies within the kernels'
+    reach (3.2 cells): its lambda in the second iteration, with nothing finite in range, is 1 / eps"""
+    params = scenes.workload_params(pbd, 128, 1000.0, iterations=2)
+    params.lambda_epsilon = 0.1
+    params.gravity = 0.0
+    params.kernel_width_poly, params.q_scorr, params.kernel_width_neighbours = 3.2, 3.198, 3
+    params.flags &= ~pbd.FLAG_CELL_END_QUIRK
+    g = np.stack(np.meshgrid(*[np.arange(30)] * 3, indexing="ij"), -1).reshape(-1, 3) * 4.0 + 3.0   # alone, for their number
+    pos = np.zeros((len(g) + 3, 4), np.float32)
+    pos[3:, :3] = g
+    pos[:3, :3] = [(126.4, 126.4, 126.4), (124.0, 126.0, 126.0), (124.8, 126.0, 126.0)]
+    with pbd.Sim(params, len(pos)) as sim:
+        sim.add_particles(pos, np.zeros_like(pos))
+        sim.step(1)
+        sim.sync()
+        lam, x = sim.debug()["lambda"], sim.state()["x"][:, :3]
+    assert np.isnan(x).any(axis=1).sum() == 2 and np.isinf(x[:, 0]).sum() == 2
+    corner = np.where((x > 126).all(axis=1))[0]
+    assert len(corner) == 1 and lam[corner[0]] == np.float32(1) / np.float32(0.1)
