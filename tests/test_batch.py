@@ -106,3 +106,28 @@ def test_batch_state_with_interleaved_adds(need_gpu, pbd, scenes):
             s.sync()
             ref = s.state()
         assert np.array_equal(before[k]["x"], ref["x"]) and np.array_equal(before[k]["v"], ref["v"]), k
+
+
+def test_batch_state_after_many_small_adds(need_gpu, pbd, scenes):
+    """a scene filled a particle at a time, alone or in turns with another scene: its state comes in a few
+    copies, not two for every add, and in the order of the adds"""
+    from helpers import device_events
+    shared = _shared(pbd, scenes)
+    sl = _scene_list(scenes)
+    descs = [pbd.scene_desc(len(sc["pos"]), sc["rho"], sc["g"], sc["box"]) for sc in sl]
+    with pbd.Batch(shared, descs) as b:
+        for i in range(len(sl[0]["pos"])):
+            b.add_particles(0, sl[0]["pos"][i:i + 1], sl[0]["vel"][i:i + 1])
+        for i in range(len(sl[1]["pos"])):
+            for k in (1, 2):
+                b.add_particles(k, sl[k]["pos"][i:i + 1], sl[k]["vel"][i:i + 1])
+        for frames in (0, 2):
+            b.step(frames)
+            for k in (0, 1, 2):
+                got = []
+                names = device_events(lambda: got.append(b.state(k)))
+                assert sum("Memcpy" in s for s in names) <= 16, (frames, k, len(names))
+                n = min(len(sl[k]["pos"]), len(sl[1]["pos"])) if k else len(sl[0]["pos"])
+                assert len(got[0]["x"]) == n
+                if not frames:
+                    assert np.array_equal(got[0]["x"], sl[k]["pos"][:n]) and np.array_equal(got[0]["v"], sl[k]["vel"][:n])
