@@ -12,7 +12,7 @@ pairs, solids, and the stored lists against the cell walk."""
 import numpy as np
 import pytest
 
-from helpers import maxdiff, setup_pair, by_id
+from helpers import by_id, device_events, maxdiff, setup_pair
 
 TOL_X1, TOL_X5 = 2e-5, 2e-3
 
@@ -164,3 +164,29 @@ def test_gpu_contact_batches_both_claim_variants(need_gpu, pbd, scenes, n_side):
         x = by_id(sim.state())["x"]
     r = np.linalg.norm(x[0::2, :3].astype(np.float64) - x[1::2, :3], axis=1)
     assert np.allclose(r, 0.964, atol=6e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_side,spacing,per_sm", [(45, 2.6, 6), (50, 2.4, 4), (53, 2.3, 4), (55, 2.2, 6)])
+def test_gpu_contact_batches_on_both_sides_of_the_claim_rule(need_gpu, pbd, scenes, n_side, spacing, per_sm):
+    """the claim pass takes 4 blocks per SM where they need at most two waves and 6 would need as many
+    (152 SMs: up to 155,000 particles, 233,000 to 311,000), else 6: 182,250 (6), 250,000 and 297,754 (4) and
+    332,750 (6) particles in isolated pairs, each constraint of which is solved once (0.6 apart, 0.88, 0.964).
+    A pair has two where either particle's 27 cells, p - 1, p and p + 1 rounded to 32 bits, hold the other.
+    Tolerance as in the test above"""
+    p, _, _ = pair_scene(pbd, scenes)
+    q = scenes.workload_params(pbd, 128, 1000.0, iterations=1)
+    q.collision_type, q.max_collision_batches, q.gravity = 1, 4, 0.0
+    q.flags, q.active = p.flags, p.active
+    _, pos, vel = pair_scene(pbd, scenes, n_side=n_side, spacing=spacing)
+    assert pos[:, :3].max() < 126.5
+    with pbd.Sim(q, len(pos)) as sim:
+        sim.add_particles(pos, vel)
+        names = device_events(lambda: sim.step(1))
+        x = by_id(sim.state())["x"]
+    assert not names or any(f"contact_claim_kernel<{per_sm}>" in s for s in names)
+    r = np.linalg.norm(x[0::2, :3].astype(np.float64) - x[1::2, :3], axis=1)
+    cell = [np.floor(pos[:, :3] + np.float32(c)) for c in (-1, 0, 1)]
+    sees = [np.all([np.any([c[k::2, a] == cell[1][1 - k::2, a] for c in cell], axis=0) for a in range(3)], axis=0) for k in (0, 1)]
+    want = np.array([0.6, 0.88, 0.964])[sees[0].astype(int) + sees[1]]
+    assert (want == 0.964).mean() > 0.99 and np.allclose(r, want, atol=6e-5)

@@ -8,6 +8,8 @@ cell-end quirk's long ranges, fast motion)."""
 import numpy as np
 import pytest
 
+from helpers import device_events
+
 pytestmark = pytest.mark.gpu
 
 
@@ -374,3 +376,107 @@ def test_near_lists_leave_out_positions_that_are_not_numbers(need_gpu, pbd, scen
     assert np.isnan(x).any(axis=1).sum() == 2 and np.isinf(x[:, 0]).sum() == 2
     corner = np.where((x > 126).all(axis=1))[0]
     assert len(corner) == 1 and lam[corner[0]] == np.float32(1) / np.float32(0.1)
+
+
+def _one_lane(pbd, params, pos, vel, frames, kernels, inv_mass=None):
+    """lists against the full walk with more than 24,576 particles (a thread per particle), and that the
+    frames ran `kernels` (parts of their names)"""
+    assert len(pos) > 24576
+    got = []
+    names = device_events(lambda: got.append(_run(pbd, params, pos, vel, frames, inv_mass=inv_mass)))
+    for k in kernels if names else ():
+        assert any(k in s for s in names), (k, sorted(set(names)))
+    _same(got[0], _run(pbd, params, pos, vel, frames, inv_mass=inv_mass, full_walk=True))
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("n_scorr,mass,known", [(4, False, 1), (4, True, 2), (3, False, 0), (0, True, 0)])
+def test_delta_variants_with_one_lane(need_gpu, pbd, scenes, dense, n_scorr, mass, known):
+    """delta_list_kernel knows nSCorr = 4 and the absence (1) or presence (2) of inverse masses at compile time,
+    or nothing (0): over near lists and over full lists, each against the walk of every cell"""
+    params = scenes.workload_params(pbd, 40, 1995.0 if dense else 1000.0)
+    params.lambda_epsilon = 0.0001 if dense else 0.1
+    params.n_scorr = n_scorr
+    if dense:
+        params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 4.1, 3.5, 2
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(31, 29, 30, seed=23, spacing=0.95)
+    w = np.where(np.arange(len(pos)) % 7 == 0, 0.0, 1.0).astype(np.float32) if mass else None
+    full = "true" if dense else "false"
+    _one_lane(pbd, params, pos, vel, 3, [f"delta_list_kernel<{m}u, {full}, {known}u>" for m in (7, 39)], w)
+
+
+@pytest.mark.parametrize("cap", [20, 40])
+def test_small_cap_with_one_lane(need_gpu, pbd, scenes, cap):
+    params = scenes.workload_params(pbd, 40, 1000.0, vorticity=0.0005, viscosity=0.01, max_neighbours=cap)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(30, 29, 31, spacing=0.9, seed=8)
+    _one_lane(pbd, params, pos, vel, 4, ["lambda_kernel<true>", "lambda_list_kernel<true, true>", "omega_list_kernel<true, true>"])
+
+
+def test_solids_with_one_lane(need_gpu, pbd, scenes):
+    pos, vel, w = scenes.solids_scene(fluid_shape=(30, 30, 30), n_boxes=2, box_shape=(6, 6, 8), box=64, seed=5)
+    params = scenes.workload_params(pbd, 64, 1000.0)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    _one_lane(pbd, params, pos, vel, 10, ["delta_list_kernel<7u, false, 2u>"], w)
+
+
+@pytest.mark.parametrize("vort,visc", [(0.0, 0.0), (0.0005, 0.01), (0.0, 0.01)])
+def test_dense_blob_with_one_lane(need_gpu, pbd, scenes, vort, visc):
+    """a blob at spacing 0.35 inside a lattice at spacing 1, as above: particles with neither list among
+    those with both"""
+    params = scenes.workload_params(pbd, 48, 1000.0, vorticity=vort, viscosity=visc)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    params.flags &= ~pbd.FLAG_CELL_END_QUIRK
+    pos, vel = scenes.lattice(31, 30, 29, spacing=1.0, seed=6)
+    lo, sp = np.array([8.0, 6.0, 8.0]), 0.35
+    blob, bv = scenes.lattice(9, 9, 9, origin=tuple(lo), spacing=sp, jitter=0.02, seed=7)
+    inside = np.all((pos[:, :3] > lo - 0.5) & (pos[:, :3] < lo + 8 * sp + 0.5), axis=1)
+    pos = np.concatenate([pos[~inside], blob]); vel = np.concatenate([vel[~inside], bv])
+    _one_lane(pbd, params, pos, vel, 4, ["lambda_list_kernel<true, true>"])
+
+
+@pytest.mark.parametrize("shells,cap", [(1, 512), (2, 20), (2, 100), (2, 512), (2, 513), (2, 1500), (3, 300), (3, 512)])
+def test_long_rows_with_one_lane(need_gpu, pbd, scenes, shells, cap):
+    """32^3 particles around cell 32767 = (31, 31, 31), whose range the cell-end quirk stretches"""
+    params = scenes.workload_params(pbd, 48, 1995.0, vorticity=0.0005, viscosity=0.00015, max_neighbours=cap)
+    params.lambda_epsilon = 0.0001
+    params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 4.1, 3.5, shells
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(32, 32, 32, seed=21)
+    _one_lane(pbd, params, pos, vel, 2, ["lambda_kernel<true>", "lambda_long_kernel", "lambda_list_kernel<true, false>"])
+
+
+def test_more_rows_than_slots_with_one_lane(need_gpu, pbd, scenes):
+    """a blob of 29,791 particles at spacing 0.35: more particles without a list than rows (8,192); the first
+    lambda pass walks the cells for the rest itself"""
+    params = scenes.workload_params(pbd, 32, 1000.0, vorticity=0.0005, viscosity=0.01)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(31, 31, 31, origin=(6.0, 6.0, 6.0), spacing=0.35, jitter=0.02, seed=22)
+    _one_lane(pbd, params, pos, vel, 2, ["lambda_kernel<true>", "lambda_long_kernel"])
+
+
+@pytest.mark.parametrize("collision_type,mass", [(0, False), (0, True), (1, False)])
+def test_two_entries_at_a_time_over_full_lists(need_gpu, pbd, scenes, collision_type, mass):
+    """lambda and delta over full lists (kernels of 2.6 cells in a list of 5: no near lists) take two entries
+    per call and test each kernel's range where its term is added: pairs on both sides of every limit,
+    pairs at one place, rows of every remainder"""
+    params = scenes.workload_params(pbd, 64, 1995.0, vorticity=0.0005, viscosity=0.00015)
+    params.lambda_epsilon = 0.1
+    params.collision_type = collision_type
+    params.kernel_width_poly, params.kernel_width_spiky, params.kernel_width_neighbours = 2.6, 2.5, 2
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(29, 31, 30, origin=(8.0, 8.0, 8.0), spacing=0.93, seed=27)
+    gaps = np.array([0.0, 1e-5, 2e-5, 9.99e-5, 1e-4, 1.01e-4, 9.99e-4, 1e-3, 1.01e-3, 0.5, 1.0, 2.4998, 2.4999, 2.5, 2.5989, 2.599, 2.6, 2.6002], np.float32)
+    a = np.arange(0, len(pos) - 1, 3)
+    pos[a + 1, :3] = pos[a, :3]
+    pos[a + 1, a % 3] += gaps[a // 3 % len(gaps)]
+    w = np.where(np.arange(len(pos)) % 7 == 0, 0.0, 1.0).astype(np.float32) if mass else None
+    known = 0 if collision_type else (2 if mass else 1)
+    unit = "false" if collision_type else "true"
+    delta = "delta_list_kernel<0u, true, 0u>" if collision_type else f"delta_list_kernel<7u, true, {known}u>"
+    _one_lane(pbd, params, pos, vel, 2, [f"lambda_list_kernel<{unit}, false>", delta], w)
