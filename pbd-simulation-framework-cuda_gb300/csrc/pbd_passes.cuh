@@ -710,37 +710,28 @@ __device__ __forceinline__ uint32_t filter_list(const DevParams& P, const NbList
     return m > L.kmax ? kListOff : (m | (mc << 8));
 }
 
-// Wraps the visitor of a walking pass and keeps particle i's near list (when `list` is set)
-// and its full list (when `flist` is set) as the walk goes.  Holds everything by value so the
-// visitor stays in registers.
+// Wraps the visitor of a walking pass and keeps particle i's near list as the walk goes.  Holds
+// everything by value so the visitor stays in registers.
 template <class V>
 struct Recorder {
     using Contrib = typename V::Contrib;
     using Extra = typename ExtraOf<V>::type;
     V inner;
     uint32_t* list;
-    uint32_t* flist;
-    uint32_t stride, fstride, kmax, fkmax, i;
+    uint32_t stride, kmax, i;
     float4 pi;
     float cut2;
-    uint32_t n = 0, nc = 0xFFFFFFFFu, fn = 0, fnc = 0xFFFFFFFFu;
-    __device__ Recorder(const V& v, const NbList& L, const NbList& F, bool full, uint32_t i_, float4 p_i, float c2)
-        : inner(v), list(L.list), flist(full ? F.list : nullptr), stride(L.stride), fstride(F.stride), kmax(L.kmax),
-          fkmax(F.kmax), i(i_), pi(p_i), cut2(c2) {}
+    uint32_t n = 0, nc = 0xFFFFFFFFu;
+    __device__ Recorder(const V& v, const NbList& L, uint32_t i_, float4 p_i, float c2)
+        : inner(v), list(L.list), stride(L.stride), kmax(L.kmax), i(i_), pi(p_i), cut2(c2) {}
     __device__ static Contrib zero() { return V::zero(); }
-    __device__ __forceinline__ void end_contacts(uint32_t c) { nc = n; fnc = fn; inner.end_contacts(c); }
+    __device__ __forceinline__ void end_contacts(uint32_t c) { nc = n; inner.end_contacts(c); }
     __device__ __forceinline__ Extra fetch(uint32_t j) const { return fetch_extra(inner, j); }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, const Extra& ex, bool contact) {
-        if (flist) {
-            if (fn < fkmax) flist[(size_t)fn * fstride + i] = j;
-            ++fn;
-        }
-        if (list) {
-            const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-            if (dist2(rx, ry, rz) < cut2) {
-                if (n < kmax) list[(size_t)n * stride + i] = j;
-                ++n;
-            }
+        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+        if (dist2(rx, ry, rz) < cut2) {
+            if (n < kmax) list[(size_t)n * stride + i] = j;
+            ++n;
         }
         return contrib_of(inner, j, pj, ex, contact);
     }
@@ -748,10 +739,6 @@ struct Recorder {
     __device__ __forceinline__ uint32_t meta() const {
         const uint32_t c = nc == 0xFFFFFFFFu ? n : nc;
         return n > kmax ? kListOff : (n | (c << 8));
-    }
-    __device__ __forceinline__ uint32_t fmeta() const {
-        const uint32_t c = fnc == 0xFFFFFFFFu ? fn : fnc;
-        return fn > fkmax ? kListOff : (fn | (c << 8));
     }
 };
 
@@ -982,7 +969,7 @@ __device__ __forceinline__ uint32_t store_full_list(const DevParams& P, const Sc
     return meta();
 }
 
-// A visitor that sums nothing: a walk with Recorder<NullVisit> only stores the lists.
+// A visitor that sums nothing: a walk with Recorder<NullVisit> only stores the near list.
 struct NullVisit {
     struct Contrib {};
     __device__ static Contrib zero() { return Contrib{}; }
@@ -1258,7 +1245,7 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
         return;
     } else if (L.list) {
         // the walk stores the near list; the sums then run over it when it fits
-        Recorder<NullVisit> rec(NullVisit{}, L, F, false, i, pi, P.cut2);
+        Recorder<NullVisit> rec(NullVisit{}, L, i, pi, P.cut2);
         walk_seq(P, S, i, pa[i], p, cs, ce, rec, true, &deferred);
         const uint32_t lm = deferred ? kListOff : rec.meta();
         L.meta[i] = lm;
@@ -1849,7 +1836,7 @@ omega_kernel(DevParams P, const float4* __restrict__ p, const float4* __restrict
     OmegaVisit vis(P, v, pi, v[i]);
     bool deferred = false;
     if (L.list) {
-        Recorder<OmegaVisit> rec(vis, L, L, false, i, pi, P.cut2);
+        Recorder<OmegaVisit> rec(vis, L, i, pi, P.cut2);
         walk_seq(P, S, i, pa[i], p, cs, ce, rec, true, &deferred);
         L.meta[i] = deferred ? kListOff : rec.meta();
         if (L.meta[i] == kListOff) note_particle(DN, i);
