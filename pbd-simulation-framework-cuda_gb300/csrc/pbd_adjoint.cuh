@@ -160,7 +160,7 @@ struct AdjViscVisit {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ float4 fetch(uint32_t j) const { return __ldg(vu + j); }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, const float4& vj, bool) {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
@@ -205,7 +205,7 @@ struct AdjVortVisit {   // the entries' terms for etabar
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ float4 fetch(uint32_t j) const { return __ldg(om + j); }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, const float4& oj, bool) {
         const float ux = oj.x - oi.x, uy = oj.y - oi.y, uz = oj.z - oi.z;
@@ -251,7 +251,7 @@ struct BothVisit {
     __device__ __forceinline__ void end_contacts(uint32_t n) { va.end_contacts(n); vb.end_contacts(n); }
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ Extra fetch(uint32_t j) const { return Extra{fetch_extra(va, j), fetch_extra(vb, j)}; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, const Extra& ex, bool contact) {
         contrib_of(va, j, pj, ex.a, contact);
@@ -337,7 +337,7 @@ struct AdjOmegaVisit {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ float4 fetch(uint32_t j) const { return __ldg(vu + j); }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, const float4& vj, bool) {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
@@ -430,7 +430,7 @@ struct AdjDeltaVisit {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, bool contact) {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
         const float r2 = dist2(rx, ry, rz);
@@ -538,7 +538,7 @@ struct AdjCollideVisit {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, bool contact) {
         if (!contact) return zero();
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
@@ -600,7 +600,7 @@ struct AdjLambdaBwd {
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ static Contrib zero() { return Contrib{0}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4& pj, bool) {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
         const float r2 = dist2(rx, ry, rz);

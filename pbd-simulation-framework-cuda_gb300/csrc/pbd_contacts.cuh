@@ -94,7 +94,7 @@ struct ContactListVisit {
     __device__ ContactListVisit(const ContactStore& C, uint32_t i_) : L(contact_entries(C)), i(i_) {}
     __device__ static Contrib zero() { return Contrib{0u}; }
     __device__ static bool effective(const Contrib&) { return true; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_u(c.j, k, width)}; }
+    __device__ static Contrib shfl(const Contrib& c, int k) { return Contrib{shfl_u(c.j, k)}; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) const { return Contrib{j}; }
     __device__ __forceinline__ void add(const Contrib& c, bool) { *full_at(L, i, n) = c.j; ++n; }

@@ -215,7 +215,6 @@ __device__ __forceinline__ float powi(float x, int n) {
         case 1: return x;
         case 2: return x * x;
         case 3: return (x * x) * x;
-        case 4: return ((x * x) * x) * x;
         default: break;
     }
     int m = n < 0 ? -n : n;

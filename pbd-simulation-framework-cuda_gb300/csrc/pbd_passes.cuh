@@ -9,7 +9,7 @@
 //
 // Each pass is split into a per-candidate contribution (`contrib`) and an in-order
 // accumulation (`add`); a visitor may also name per-neighbour data (`Extra`, loaded by
-// `fetch(j)`) that the walkers load together with the neighbour's position.  Three walkers
+// `fetch(j)`) that the walkers load together with the neighbour's position.  These walkers
 // drive them:
 //  - walk_seq: one thread per particle over the cells;
 //  - walk_coop: one warp per particle.  Lanes evaluate 32 candidates at once and the
@@ -18,8 +18,8 @@
 //    kLongRange -- in practice the range that SortReorder.h:183-184 extends to N (up to M
 //    entries) -- which would otherwise serialise a whole warp behind one thread;
 //  - walk_full, walk_near: one thread per particle over a stored list;
-//  - walk_group: G lanes per particle over a stored list (the long lists, LongLists, with a warp; small
-//    simulations with fewer lanes).
+//  - walk_list_warp: one warp per particle over a stored list (the long lists, LongLists);
+//  - walk_group_sums: G lanes per particle over a stored list (small simulations).
 #pragma once
 #include <type_traits>
 #include "pbd_device.cuh"
@@ -60,9 +60,8 @@ constexpr uint32_t kLongRange = 32;
 constexpr uint32_t kFullMask = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
-// a value of lane k of the caller's group of `width` lanes
-__device__ __forceinline__ float shfl_f(float v, int k, int width) { return __shfl_sync(kFullMask, v, k, width); }
-__device__ __forceinline__ uint32_t shfl_u(uint32_t v, int k, int width) { return __shfl_sync(kFullMask, v, k, width); }
+__device__ __forceinline__ float shfl_f(float v, int k) { return __shfl_sync(kFullMask, v, k); }
+__device__ __forceinline__ uint32_t shfl_u(uint32_t v, int k) { return __shfl_sync(kFullMask, v, k); }
 __device__ __forceinline__ uint32_t lanemask_lt_u() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -365,20 +364,18 @@ __device__ __forceinline__ uint32_t store_row(const DevParams& P, const SceneCtx
     return R.n > kLongMax ? kListOff : (R.n | (R.nc << 16));
 }
 
-// G lanes per particle over a stored list (entry k at entry(k); n and nc the same in all lanes of a
-// group): each lane evaluates every G-th entry, two position loads in flight and the next indices
-// loaded meanwhile, and the contributions that change a sum are added in list order through
-// shuffles, as in walk_coop, so every lane of the group ends with the sums.  Every lane of the warp
-// calls it.
-template <int G, class E, class V>
-__device__ __forceinline__ void walk_group(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
+// One warp per particle over a stored list (entry k at entry(k); n and nc the same in all lanes): each
+// lane evaluates every 32nd entry, two position loads in flight and the next indices loaded
+// meanwhile, and the contributions that change a sum are added in list order through shuffles, as
+// in walk_coop, so every lane ends with the sums.
+template <class E, class V>
+__device__ __forceinline__ void walk_list_warp(E&& entry, uint32_t n, uint32_t nc, uint32_t i, const float4* __restrict__ p,
                                            V& vis) {
-    const uint32_t t = lane_id() & (uint32_t)(G - 1);
-    constexpr uint32_t kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
+    const uint32_t t = lane_id();
     uint32_t jn[2];
 #pragma unroll
-    for (uint32_t b = 0; b < 2u; ++b) jn[b] = b * G + t < n ? *entry(b * G + t) : i;
-    for (uint32_t kb = 0; __any_sync(kFullMask, kb < n); kb += 2u * G) {
+    for (uint32_t b = 0; b < 2u; ++b) jn[b] = b * 32u + t < n ? *entry(b * 32u + t) : i;
+    for (uint32_t kb = 0; kb < n; kb += 64u) {
         uint32_t j[2];
         float4 pj[2];
         typename ExtraOf<V>::type ex[2];
@@ -390,28 +387,26 @@ __device__ __forceinline__ void walk_group(E&& entry, uint32_t n, uint32_t nc, u
         }
 #pragma unroll
         for (uint32_t b = 0; b < 2u; ++b) {
-            const uint32_t k = kb + (2u + b) * G + t;
+            const uint32_t k = kb + (2u + b) * 32u + t;
             jn[b] = k < n ? *entry(k) : i;
         }
 #pragma unroll
         for (uint32_t b = 0; b < 2u; ++b) {
-            const uint32_t k = kb + b * G + t;
+            const uint32_t k = kb + b * 32u + t;
             const typename V::Contrib c = k < n ? contrib_of(vis, j[b], pj[b], ex[b], k < nc) : V::zero();
             uint32_t take = __ballot_sync(kFullMask, k < n && V::effective(c));
-#pragma unroll
-            for (int o = G; o < 32; o <<= 1) take |= take >> o;   // the entries any group of the warp adds
-            take &= kGroup;
             while (take) {
                 const int q = __ffs(take) - 1;
                 take &= take - 1u;
-                vis.add(V::shfl(c, q, G), true);   // a contribution without effect leaves the sums alone
+                vis.add(V::shfl(c, q), true);
             }
         }
     }
     vis.end_contacts(nc);
 }
 
-// walk_group with the sums split over the group's lanes, for a pass whose main walk it is.  Every sum
+// A stored list with G lanes per particle and the sums split over the lanes (every lane of the warp calls
+// it; a group with n = 0 only takes part in the shuffles).  Every sum
 // of a visitor is a chain acc = fma(mul, val, acc) over the entries (mul = 1 where a contribution is
 // added as it is: the same rounding as an addition).  Each lane puts its entry's numbers (V::rows,
 // zeros where the entry has no effect, which leave a chain alone) into shared memory, a row per
@@ -752,7 +747,7 @@ struct ListRecorder {
     __device__ ListRecorder(const NbList& F_, uint32_t i_) : F(F_), i(i_) {}
     __device__ static Contrib zero() { return Contrib{}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ void end_contacts(uint32_t) { nc = n; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) {
         if (n < F.kmax) *full_at(F, i, n) = j;
@@ -974,7 +969,7 @@ struct NullVisit {
     struct Contrib {};
     __device__ static Contrib zero() { return Contrib{}; }
     __device__ static bool effective(const Contrib&) { return false; }
-    __device__ static Contrib shfl(const Contrib& c, int, int = 32) { return c; }
+    __device__ static Contrib shfl(const Contrib& c, int) { return c; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4&, bool) const { return Contrib{}; }
     __device__ __forceinline__ void add(const Contrib&, bool) {}
@@ -1066,7 +1061,7 @@ __device__ __forceinline__ void walk_warp(const DevParams& P, const SceneCtx& S,
                                           const float4* __restrict__ p, const uint32_t* __restrict__ cs,
                                           const uint32_t* __restrict__ ce, const LongLists& LL, const NbList& F, V& vis) {
     const WarpList W = warp_list(LL, F, i);
-    if (W.row) walk_group<32>([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, i, p, vis);
+    if (W.row) walk_list_warp([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, i, p, vis);
     else walk_coop(P, S, i, anchor, p, cs, ce, vis);
 }
 
@@ -1087,9 +1082,9 @@ struct LambdaVisitT {
     __device__ void reset() { A = B = Cx = Cy = Cz = Cw = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, false}; }
     __device__ static bool effective(const Contrib& c) { return c.near; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
-        return Contrib{shfl_f(c.a, k, width), shfl_f(c.b, k, width), shfl_f(c.s, k, width), shfl_f(c.rx, k, width), shfl_f(c.ry, k, width),
-                       shfl_f(c.rz, k, width), shfl_f(c.rw, k, width), 0.f, shfl_u(c.near, k, width) != 0u};
+    __device__ static Contrib shfl(const Contrib& c, int k) {
+        return Contrib{shfl_f(c.a, k), shfl_f(c.b, k), shfl_f(c.s, k), shfl_f(c.rx, k), shfl_f(c.ry, k),
+                       shfl_f(c.rz, k), shfl_f(c.rw, k), 0.f, shfl_u(c.near, k) != 0u};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
@@ -1293,7 +1288,7 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
             if (lm == kListOff) note_particle(DN, i);
         }
     }
-    if (lm != kListOff) walk_group<32>([&](uint32_t k) { return L.list + (size_t)k * L.stride + i; }, lm & 0xFFu, lm >> 8, i, p, vis);
+    if (lm != kListOff) walk_list_warp([&](uint32_t k) { return L.list + (size_t)k * L.stride + i; }, lm & 0xFFu, lm >> 8, i, p, vis);
     else walk_warp(P, S, i, pa[i], p, cs, ce, LL, F, vis);
     if (lane_id() == 0) {
         const float li = vis.finish(S.rho0);
@@ -1489,10 +1484,10 @@ struct DeltaVisitT {
     __device__ void reset() { ax = ay = az = aw = 0.f; pacc = pi; xacc = xi; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, false, false}; }
     __device__ static bool effective(const Contrib& c) { return c.d || c.c; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
-        const uint32_t f = shfl_u((c.d ? 1u : 0u) | (c.c ? 2u : 0u), k, width);
-        return Contrib{shfl_f(c.coef, k, width), shfl_f(c.rx, k, width), shfl_f(c.ry, k, width), shfl_f(c.rz, k, width), shfl_f(c.rw, k, width),
-                       shfl_f(c.t, k, width), 0.f, 0.f, (f & 1u) != 0u, (f & 2u) != 0u};
+    __device__ static Contrib shfl(const Contrib& c, int k) {
+        const uint32_t f = shfl_u((c.d ? 1u : 0u) | (c.c ? 2u : 0u), k);
+        return Contrib{shfl_f(c.coef, k), shfl_f(c.rx, k), shfl_f(c.ry, k), shfl_f(c.rz, k), shfl_f(c.rw, k),
+                       shfl_f(c.t, k), 0.f, 0.f, (f & 1u) != 0u, (f & 2u) != 0u};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float;   // lambda_j
@@ -1787,8 +1782,8 @@ struct OmegaVisitT {
     __device__ void reset() { ox = oy = oz = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, false}; }
     __device__ static bool effective(const Contrib& c) { return c.near; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
-        return Contrib{shfl_f(c.ox, k, width), shfl_f(c.oy, k, width), shfl_f(c.oz, k, width), 0.f, 0.f, shfl_u(c.near, k, width) != 0u};
+    __device__ static Contrib shfl(const Contrib& c, int k) {
+        return Contrib{shfl_f(c.ox, k), shfl_f(c.oy, k), shfl_f(c.oz, k), 0.f, 0.f, shfl_u(c.near, k) != 0u};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = float4;   // v_j
@@ -1976,10 +1971,10 @@ struct VortViscVisitT {
     __device__ void reset() { gx = gy = gz = sx = sy = sz = sw = 0.f; }
     __device__ static Contrib zero() { return Contrib{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, false, false}; }
     __device__ static bool effective(const Contrib& c) { return c.vo || c.vs; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) {
-        const uint32_t f = shfl_u((c.vo ? 1u : 0u) | (c.vs ? 2u : 0u), k, width);
-        return Contrib{shfl_f(c.gx, k, width), shfl_f(c.gy, k, width), shfl_f(c.gz, k, width), shfl_f(c.sx, k, width),
-                       shfl_f(c.sy, k, width), shfl_f(c.sz, k, width), shfl_f(c.sw, k, width), 0.f, 0.f, (f & 1u) != 0u, (f & 2u) != 0u};
+    __device__ static Contrib shfl(const Contrib& c, int k) {
+        const uint32_t f = shfl_u((c.vo ? 1u : 0u) | (c.vs ? 2u : 0u), k);
+        return Contrib{shfl_f(c.gx, k), shfl_f(c.gy, k), shfl_f(c.gz, k), shfl_f(c.sx, k),
+                       shfl_f(c.sy, k), shfl_f(c.sz, k), shfl_f(c.sw, k), 0.f, 0.f, (f & 1u) != 0u, (f & 2u) != 0u};
     }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     using Extra = VortViscExtra<kTerms>;
@@ -2225,7 +2220,7 @@ struct DensityVisit {
     __device__ DensityVisit(const DevParams& P_, float4 pi_) : P(P_), pi(pi_) {}
     __device__ static Contrib zero() { return Contrib{0.f, 0u}; }
     __device__ static bool effective(const Contrib& c) { return c.near != 0u; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_f(c.a, k, width), shfl_u(c.near, k, width)}; }
+    __device__ static Contrib shfl(const Contrib& c, int k) { return Contrib{shfl_f(c.a, k), shfl_u(c.near, k)}; }
     __device__ __forceinline__ void end_contacts(uint32_t) {}
     __device__ __forceinline__ Contrib contrib(uint32_t, const float4& pj, bool) const {
         const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
@@ -2298,7 +2293,7 @@ struct ListVisit {
     __device__ ListVisit(uint32_t* o, uint32_t c) : out(o), cap(c) {}
     __device__ static Contrib zero() { return Contrib{0u}; }
     __device__ static bool effective(const Contrib&) { return true; }
-    __device__ static Contrib shfl(const Contrib& c, int k, int width = 32) { return Contrib{shfl_u(c.j, k, width)}; }
+    __device__ static Contrib shfl(const Contrib& c, int k) { return Contrib{shfl_u(c.j, k)}; }
     __device__ __forceinline__ void end_contacts(uint32_t c) { contacts = c; }
     __device__ __forceinline__ Contrib contrib(uint32_t j, const float4&, bool) const { return Contrib{j}; }
     __device__ __forceinline__ void add(const Contrib& c, bool) {
