@@ -363,9 +363,25 @@ static void launch_delta_staged(uint32_t N, cudaStream_t st, const DevParams& P,
 }
 
 // Lanes per particle of the list passes: more than one while the particles alone leave most of the
-// GPU idle and a pass is one thread's chain of loads.  Measured (GB300, us a frame, 1 / 4 / 8 / 16
-// lanes): 4,275 particles 87 / 64 / 62 / 60; 15,525 (config.txt's 72 entries) 136 / 126 / 117 / 121;
-// 32,768 103 / 103 / 120 / 143; at 65,536 four lanes are 13% slower than one.
+// GPU idle and a pass is one thread's chain of loads.  Measured (GB300, us a frame of four in a row,
+// 1 / 4 / 8 / 16 lanes; unit kernels with vorticity: near lists of ~6 of 31 entries; config.txt: full lists
+// of ~72; density-active kernels: full lists of ~124; * the cell-end range lies inside the fluid):
+//   particles  unit kernels             config.txt               density-active
+//    2,940      89 /  63 /  59 /  56    *140 / 136 / 128 / 122   *267 / 257 / 249 / 245
+//    5,832      91 /  66 /  62 /  62      84 /  76 /  58 /  54    194 / 184 / 124 / 108
+//    8,000      93 /  67 /  64 /  75      89 /  81 /  64 /  61    193 / 185 / 135 / 133
+//    9,240      93 /  68 /  66 /  79      87 /  81 /  64 /  65    193 / 195 / 144 / 142
+//   12,167      95 /  70 /  70 /  87      87 /  85 /  74 /  75    197 / 204 / 167 / 164
+//   16,250      97 /  74 /  87 / 104    *146 / 155 / 148 / 151    211 / 231 / 211 / 201
+//   17,576      97 /  74 /  90 / 108      96 /  95 /  90 /  91    211 / 229 / 222 / 212
+//   20,412      97 /  77 /  95 / 116      98 / 100 /  95 /  98    214 / 262 / 242 / 233
+//   24,389    *159 / 152 / 166 / 186    *126 / 146 / 141 / 144   *245 / 324 / 302 / 304
+//   27,000      99 /  86 / 108 / 141     102 / 119 / 118 / 123    279 / 359 / 344 / 357
+//   32,768    *158 / 162 / 180 / 204    *121 / 157 / 149 / 158   *264 / 376 / 349 / 363
+//   40,460     106 / 114 / 139 / 191     111 / 163 / 150 / 165    249 / 415 / 375 / 400
+// The lines lie where all kinds of list gain over one lane up to 16,384 particles; from there to 24,576 four
+// lanes take 4 to 24% off unit kernels' frames and add up to 32% to those over full lists.  By near lists
+// alone the lines would be ~6,000, ~12,000 and ~30,000, by full lists ~8,000 and ~16,000.
 int pass_lanes(uint32_t N) {
     return N <= 8192u ? 16 : (N <= 16384u ? 8 : (N <= 24576u ? 4 : 1));
 }
@@ -555,7 +571,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
             } else {
                 auto k = P.unit_w ? lambda_kernel<true> : lambda_kernel<false>;
                 k<<<gn, tn, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam, D, aux, Lr,
-                                                 use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots, pl);
+                                     use_full ? F : L0, use_full ? DF : DX, Lr.list ? DN : DX, s->ll.slots, pl);
                 if (use_full)
                     lambda_long_kernel<<<gc, kThreadsCoop, 0, st>>>(P, s->p[cur.p], pa, s->cell_start, s->cell_end, lam,
                                                                     DF, aux, s->ll, F, Lr, Lr.list ? DN : DX, pl);
@@ -577,8 +593,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 const int pout = next_p(cur.p);
                 if (by_list) {
                     (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
-                        gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                      s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, nullptr);
+                        gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf, s->delta,
+                        s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, nullptr);
                     nl += 1;
                 } else {
                     delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -657,8 +673,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 nl += 1;
             } else if (by_list) {
                 (use_lists ? launch_delta_list<false> : launch_delta_list<true>)(
-                    gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
-                                  s->delta, s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, pl);
+                    gn, tn, st, P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf, s->delta,
+                    s->cell_start, s->cell_end, use_lists ? CN : CF, use_lists ? L : F, F, s->ll, lanes, N, pl);
                 nl += 1;
             } else {
                 delta_kernel<<<gn, tn, 0, st>>>(P, mode, s->p[cur.p], pa, s->p[pout], s->x[cur.x], s->v[cur.v], lam, wf,
@@ -739,11 +755,11 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 kg<<<gl + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
                                                     s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, vh, F, s->ll);
             } else {
-            auto k = Ln.list ? vort_visc_list_kernel<kVortVisc>
-                             : (vfull ? vort_visc_list_kernel<kVortViscFull> : vort_visc_list_kernel<kViscNear>);
-            k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
-                                               s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, Ln, vh,
-                                               F, s->ll, po);
+                auto k = Ln.list ? vort_visc_list_kernel<kVortVisc>
+                                 : (vfull ? vort_visc_list_kernel<kVortViscFull> : vort_visc_list_kernel<kViscNear>);
+                k<<<gn + kCoopBlocks, tn, 0, st>>>(P, s->p[cur.p], pa, s->v[cur.v], s->v[cur.v ^ 1], s->omega, s->fext,
+                                                   s->cell_start, s->cell_end, vort, visc, wf, vfull ? CF : CN, Lv, Ln, vh,
+                                                   F, s->ll, po);
             }
             v_read = v_read || vh != nullptr;
             nl += 1;
@@ -763,6 +779,8 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     }
     return cudaGetLastError();
 }
+#undef BY_LANES
+#undef COMMA
 
 void destroy_graphs(pbd_sim* s) {
     for (int k = 0; k < kMaxGraphs; ++k) {
