@@ -64,7 +64,8 @@ struct DevParams {
     // sum_j |omega_j - omega_i| / (p_j - p_i + 1e-8)) here; null in every other frame
     float4* eta_tape;
     // every predicted position's w is 1 for the whole frame: applyForces sets it (Forces.h:94), and with
-    // collisionType 0 nothing but a 0 is ever added to it (collisionType 1 writes 0 there)
+    // collisionType 0 and the frame's own corrections nothing but a 0 is ever added to it (collisionType 1
+    // writes 0 there, and corrections that an earlier frame stored may hold what came of that)
     uint32_t unit_w;
     // the predicted positions in steps of 1/512 cell (coarse_pos), kept by every kernel that writes them
     // in a frame whose passes filter lists by them, else null; near_coarse: coarse_near's limit

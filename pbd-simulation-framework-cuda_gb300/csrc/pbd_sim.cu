@@ -298,7 +298,8 @@ DevParams make_dev_params(const pbd_sim* s) {
     P.scene_of = s->scene_of;
     P.scene_range = s->scene_range;
     P.eta_tape = nullptr;
-    P.unit_w = ((p.active & PBD_ACTIVE_APPLY_FORCES) && p.collision_type == 0) ? 1u : 0u;
+    const bool loads_delta = (p.active & PBD_ACTIVE_APPLY_DELTA_POSITIONS) && !(p.active & PBD_ACTIVE_COMPUTE_DELTA_POSITIONS);
+    P.unit_w = ((p.active & PBD_ACTIVE_APPLY_FORCES) && p.collision_type == 0 && !loads_delta) ? 1u : 0u;
     const float c = std::max(P.hp, std::max(P.hs, P.d));
     P.cut2 = c * c * 1.0001f;
     P.coarse = nullptr;

@@ -480,3 +480,32 @@ def test_two_entries_at_a_time_over_full_lists(need_gpu, pbd, scenes, collision_
     unit = "false" if collision_type else "true"
     delta = "delta_list_kernel<0u, true, 0u>" if collision_type else f"delta_list_kernel<7u, true, {known}u>"
     _one_lane(pbd, params, pos, vel, 2, [f"lambda_list_kernel<{unit}, false>", delta], w)
+
+
+def test_loaded_delta_with_a_w(need_gpu, pbd, scenes):
+    """collisionType 1 writes p.w = 0 for some particles, so the corrections it stores have a w; frames that
+    then apply them without computing new ones (collisionType 0) move p.w off 1, and the passes after that
+    see it in the spiky gradient: lists against the full walk"""
+    params = scenes.workload_params(pbd, 64, 1000.0, vorticity=0.0005, viscosity=0.01, iterations=3)
+    params.lambda_epsilon = 0.1
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(30, 30, 30, spacing=0.8, seed=31)
+    vel[:, :3] = np.random.default_rng(31).normal(0, 1.0, size=(len(vel), 3)).astype(np.float32)
+    out = []
+    for flags in (0, pbd.FLAG_FULL_WALK):
+        p = params.copy()
+        p.flags |= flags
+        p.collision_type = 1
+        with pbd.Sim(p, len(pos)) as sim:
+            sim.add_particles(pos, vel)
+            sim.step(2)
+            p.collision_type = 0
+            p.active &= ~pbd.ACTIVE["computeDeltaPositions"]
+            sim.set_params(p)
+            sim.step(2)
+            sim.sync()
+            out.append((sim.state(), sim.debug()))
+    assert np.ptp(out[1][0]["p"][:, 3]) > 0
+    _same(out[0][0], out[1][0])
+    for k in ("lambda", "omega"):
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
