@@ -339,9 +339,11 @@ static bool use_full_list(const pbd_sim* s) {
 // Near lists need kernels that vanish beyond the cut (far_pairs_zero), and they pay only when the
 // cut keeps a small part of the list: the cut's sphere against the cube of cells the list covers.
 // With kernel widths of a few cells (config.txt's 4.1 and 6.1 with kernelWidthNeighbours 2) the
-// sphere holds the whole cube, every entry is near, and the passes read the full list instead.
+// sphere holds the whole cube, every entry is near, and the passes read the full list instead.  The staged
+// passes record none.  The frame and the adjoint's reverse pass, which reads the lists that taped frames
+// recorded, both go by this.
 static bool near_lists_on(const pbd_sim* s, const DevParams& P) {
-    if ((s->prm.flags & PBD_FLAG_FULL_WALK) || P.far_pairs_zero == 0u) return false;
+    if ((s->prm.flags & (PBD_FLAG_FULL_WALK | PBD_FLAG_STAGED_PASSES)) || P.far_pairs_zero == 0u) return false;
     const bool shells = (P.active & PBD_ACTIVE_FIND_NEIGHBOURS) && P.K > 1;
     const double side = (2.0 * (shells ? P.K : 1u) + 1.0) * P.d;
     const double cut = std::sqrt((double)P.cut2 / 1.0001);
@@ -430,8 +432,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     const int np = sort_passes(s);
     const int tn = s->tpb_nbr;
     // the thread-per-particle passes filter their lists by the coarse positions where p.w needs no look
-    if (P.unit_w && pass_lanes(N) == 1 && use_full_list(s) && near_lists_on(s, P) && !(prm.flags & PBD_FLAG_STAGED_PASSES))
-        P.coarse = s->coarse;
+    if (P.unit_w && pass_lanes(N) == 1 && use_full_list(s) && near_lists_on(s, P)) P.coarse = s->coarse;
     SortScratch S{s->hist, s->status, s->tile_counter, s->err, s->max_tiles, s->sort_spin_limit, s->sort_hold};
     nl = 0;
 
@@ -505,7 +506,7 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
     const uint32_t I = prm.solver_iterations, Sx = prm.stabilization_iterations;
     // near lists: recorded by a walking pass for the pass after it at the same positions; they
     // need kernels that vanish beyond the cut (far_pairs_zero)
-    const bool use_lists = near_lists_on(s, P) && !(prm.flags & PBD_FLAG_STAGED_PASSES);
+    const bool use_lists = near_lists_on(s, P);
     const NbList Lf = use_lists ? NbList{s->nb_list, s->nb_meta, s->cap, kListMax} : NbList{nullptr, nullptr, 0u, 0u};
     const NbList L = Lf;
     const NbList L0{nullptr, nullptr, 0u, 0u};

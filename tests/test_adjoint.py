@@ -635,3 +635,21 @@ def test_gpu_recorded_segments_follow_the_sort_settings(need_gpu, pbd, scenes):
     assert sorts == [False] * 8 + [True, True, False, False]
     for got in grads[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(got, grads[0]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solids", [False, True])
+def test_gpu_adjoint_with_staged_passes(need_gpu, pbd, scenes, solids):
+    """PBD_FLAG_STAGED_PASSES records no near lists into the tape: the reverse pass walks the cells as it does
+    with PBD_FLAG_FULL_WALK, and gives the same bits"""
+    prm, pos, vel, w = adjoint_scene(pbd, scenes, shape=(10, 10, 10), box=18, viscosity=0.01, vorticity=0.01)
+    m = None
+    if solids:
+        vel, m = with_solids(pos, vel)
+    got = []
+    for flag in (pbd.FLAG_STAGED_PASSES, pbd.FLAG_FULL_WALK):
+        p = prm.copy()
+        p.flags |= flag
+        got.append(_gpu_grads(pbd, p, pos, vel, w, 5, 2, m)[3:])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
