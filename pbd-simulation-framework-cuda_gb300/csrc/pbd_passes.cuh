@@ -1589,7 +1589,10 @@ struct DeltaVisitT {
             if (k1 && contact_t(j1, d[1], t)) add_contact(x[1], y[1], z[1], t);
         }
     }
-    // walk_group_sums: the density part's sums, then the contacts' on p* and x, from coef, -t and r
+    // walk_group_sums: the density part's sums, then the contacts' on p* and x, from coef, -t and r.  The parts
+    // share r, times 0 in the sums that an entry is not part of: only for passes whose far pairs are exactly
+    // zero, where an entry of either part is in reach and its r finite (else a NaN position, which every pair
+    // beyond the kernels has a part in, would reach the contacts' sums, and x).
     static constexpr int kRows = 6, kSums = 10;
     __device__ static constexpr int mul_row(int s) { return s < 4 ? 0 : 1; }
     __device__ static constexpr int val_row(int s) { return s < 4 ? 2 + s : (s < 7 ? s - 2 : s - 5); }
@@ -1601,7 +1604,8 @@ struct DeltaVisitT {
         const bool f = live && (c.d || c.c);
         r[0] = (live && c.d) ? c.coef : 0.f;
         r[1] = (live && c.c) ? -c.t : 0.f;
-        r[2] = f ? c.rx : 0.f; r[3] = f ? c.ry : 0.f; r[4] = f ? c.rz : 0.f; r[5] = f ? c.rw : 0.f;
+        r[2] = f ? c.rx : 0.f; r[3] = f ? c.ry : 0.f; r[4] = f ? c.rz : 0.f;
+        r[5] = (live && c.d) ? c.rw : 0.f;
     }
 };
 using DeltaVisit = DeltaVisitT<kDeltaAny>;

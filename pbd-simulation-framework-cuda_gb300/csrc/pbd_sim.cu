@@ -401,7 +401,7 @@ static void launch_delta_list(uint32_t gn, int tn, cudaStream_t st, const DevPar
                               const float* w, float4* delta, const uint32_t* cs, const uint32_t* ce, const CoopSet& C,
                               const NbList& L, const NbList& F, const LongLists& LL, int lanes, uint32_t N,
                               const float4* pl) {
-    if (lanes > 1) {
+    if (lanes > 1 && P.far_pairs_zero != 0u) {   // see DeltaVisitT::rows
         auto k = BY_LANES(delta_list_group_kernel, kFull COMMA);
         k<<<div_up((uint64_t)N * lanes, tn) + C.blocks, tn, 0, st>>>(P, mode, pin, pa, pout, x, v, lam, w, delta, cs, ce, C, L, F, LL);
         return;

@@ -509,3 +509,24 @@ def test_loaded_delta_with_a_w(need_gpu, pbd, scenes):
     _same(out[0][0], out[1][0])
     for k in ("lambda", "omega"):
         assert np.array_equal(out[0][1][k], out[1][1][k]), k
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 3), (6, 7, 8), (22, 21, 23), (27, 28, 28)])
+@pytest.mark.parametrize("stab", [1, 2])
+def test_far_pairs_that_are_not_numbers(need_gpu, pbd, scenes, shape, stab):
+    """a negative nSCorr makes s_corr of a pair beyond the kernels infinite and its correction NaN: p* becomes
+    NaN, but the contacts alone move x (updatePositions off), which stays a number in the walk of the cells and
+    so it must with several lanes per particle"""
+    params = scenes.workload_params(pbd, 40, 1000.0, iterations=3)
+    params.lambda_epsilon = 0.1
+    params.n_scorr = -1
+    params.stabilization_iterations = stab
+    params.kernel_width_neighbours = 2
+    params.active |= pbd.ACTIVE["findNeighbours"]
+    params.active &= ~pbd.ACTIVE["updatePositions"]
+    params.flags |= pbd.FLAG_TRACK_IDS
+    pos, vel = scenes.lattice(*shape, spacing=0.9, seed=33)
+    a, b = (_run(pbd, params, pos, vel, 1, full_walk=fw) for fw in (False, True))
+    assert np.isfinite(b["x"][:, :3]).all()
+    for k in ("x", "v", "p"):
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
