@@ -608,6 +608,12 @@ cudaError_t enqueue_frame(pbd_sim* s, cudaStream_t st, Cur& cur, bool front_only
                 PROF_END();
                 cur.p = pout;
             }
+            // the batches move p* in place: not the anchors, whose cells the frame's lists come from
+            if (cur.p == anchor && Sx > 0) {
+                const int pout = next_p(cur.p);
+                cudaMemcpyAsync(s->p[pout], s->p[cur.p], (size_t)N * 16, cudaMemcpyDeviceToDevice, st);
+                cur.p = pout;
+            }
             // the batches' keys alternate between two buffers; each solve pass clears the other
             ContactStore C = s->ct;
             unsigned long long* const keys[2] = {s->ct.best, s->ct.best + s->ct.stride};

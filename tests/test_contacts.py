@@ -190,3 +190,39 @@ def test_gpu_contact_batches_on_both_sides_of_the_claim_rule(need_gpu, pbd, scen
     sees = [np.all([np.any([c[k::2, a] == cell[1][1 - k::2, a] for c in cell], axis=0) for a in range(3)], axis=0) for k in (0, 1)]
     want = np.array([0.6, 0.88, 0.964])[sees[0].astype(int) + sees[1]]
     assert (want == 0.964).mean() > 0.99 and np.allclose(r, want, atol=6e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("apply", [False, True])
+@pytest.mark.parametrize("shape,spacing", [((9, 8, 9), 0.45), ((10, 12, 10), 0.8)])
+def test_gpu_contact_batches_leave_the_anchors_alone(need_gpu, pbd, scenes, oracle_mod, shape, spacing, apply):
+    """with computeDeltaPositions off the batches are the frame's first pass to move p*: they must not move the
+    positions whose cells the frame's lists come from.  Lists against the full walk over three frames (with lists
+    beyond a full list's room, kept as rows, and without), and one frame against the oracle"""
+    p, pos, vel = contact_scene(pbd, scenes, shape=shape, spacing=spacing, iterations=3)
+    p.kernel_width_neighbours = 2
+    p.kernel_width_poly = 1.6
+    p.c_viscosity, p.e_vorticity = 0.01, 0.0005
+    p.active |= pbd.ACTIVE["findNeighbours"] | pbd.ACTIVE["computeOmegas"] | pbd.ACTIVE["computeVorticity"] | pbd.ACTIVE["computeViscosity"]
+    p.active &= ~pbd.ACTIVE["computeDeltaPositions"]
+    if not apply:
+        p.active &= ~pbd.ACTIVE["applyDeltaPositions"]
+    out = []
+    for flags in (0, 0, pbd.FLAG_FULL_WALK):
+        q = p.copy()
+        q.flags |= flags
+        with pbd.Sim(q, len(pos)) as sim:
+            sim.add_particles(pos, vel)
+            sim.step(3)
+            out.append((sim.state(), sim.debug()))
+    for a in out[1:]:
+        for k in ("x", "v", "p", "ids"):
+            assert np.array_equal(a[0][k], out[0][0][k]), k
+        for k in ("lambda", "omega", "fext"):
+            assert np.array_equal(a[1][k], out[0][1][k]), k
+    sim, orc = setup_pair(pbd, oracle_mod, p, pos, vel)
+    sim.step(1)
+    orc.step(1)
+    g, o = by_id(sim.state()), by_id(orc.state())
+    assert maxdiff(g["x"][:, :3], o["x"][:, :3]) <= TOL_X1
+    assert maxdiff(g["v"][:, :3], o["v"][:, :3]) <= TOL_X1 * 100
