@@ -2036,6 +2036,7 @@ int pbd_adjoint_backward(pbd_sim* s, const float* dL_dx_final, float* dL_dv0, fl
     CK(cudaMemsetAsync(s->adj_acc, 0, (size_t)nblk * 16, st));
     CK(cudaMemsetAsync(s->adj_scat, 0, (size_t)N * 32, st));
     CK(cudaMemsetAsync(s->adj_scat2, 0, (size_t)N * 32, st));
+    if (s->adj_scat3) CK(cudaMemsetAsync(s->adj_scat3, 0, (size_t)N * 32, st));
     for (int ck = s->adj_nck - 1; ck >= 0; --ck) {
         const int f0 = ck * s->adj_every;
         const int nf = std::min(s->adj_every, s->adj_steps - f0);

@@ -653,3 +653,30 @@ def test_gpu_adjoint_with_staged_passes(need_gpu, pbd, scenes, solids):
         got.append(_gpu_grads(pbd, p, pos, vel, w, 5, 2, m)[3:])
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vorticity,stab", [(0.01, 1), (0.0, 3), (0.01, 2)])
+def test_gpu_gradients_after_rollouts_of_another_layout(need_gpu, pbd, scenes, vorticity, stab):
+    """the workspace is laid out by the checkpoint distance: what the reverse pass adds to (the vorticity's and the
+    later contact passes' partner terms among it) starts at zero wherever it lies, so a rollout's gradients do
+    not depend on how the rollouts before it were cut into segments (on the same simulation: the first frame
+    applies the force that the last rollout left)"""
+    prm, pos, vel, w = adjoint_scene(pbd, scenes, viscosity=0.01, vorticity=vorticity)
+    prm.stabilization_iterations = stab
+    g = np.zeros((len(pos), 4), np.float32)
+    g[:, :3] = w
+    runs = []
+    for cuts in ((3, 2, 1), (3, 1, 1), (2, 1, 7), (7, 2, 1), (6, 2, 1), (8, 2, 3), (1, 1, 1)):
+        got = []
+        with pbd.Sim(prm, len(pos)) as sim:
+            for frames, every in zip((8, 2, 7), cuts):
+                sim.clear()
+                sim.add_particles(pos, vel)
+                sim.adjoint_forward(frames, every)
+                got.append(sim.adjoint_backward(g))
+        runs.append(got)
+    for got in runs[1:]:
+        for a, b in zip(got, runs[0]):
+            for k in range(4):
+                assert np.array_equal(a[k], b[k])
