@@ -535,9 +535,13 @@ template <class V> struct AddIf<V, std::void_t<decltype(&V::add_if)>> : std::tru
 // passes are bound by instruction issue and the gathers together: 54 -> 43 instructions per entry for
 // delta and 43 -> 31 for lambda made them 211 -> 185 and 169 -> 147 us (1M particles, ~124 entries;
 // positions loaded a group ahead instead: 210 and 180, the registers cost warps).  i itself as an entry
-// must add nothing to its sums.
+// must add nothing to its sums; where it might (self_adds), the list is summed once more, entry by entry (after
+// the loop, where it costs nothing: as a second loop for the last group lambda took 154 us, as a test of
+// every entry 165).
 template <class V, class = void> struct AddTwo : std::false_type {};
 template <class V> struct AddTwo<V, std::void_t<decltype(V::kAddTwo)>> : std::bool_constant<V::kAddTwo> {};
+template <class V, class = void> struct SelfAdds : std::false_type {};
+template <class V> struct SelfAdds<V, std::void_t<decltype(&V::self_adds)>> : std::true_type {};
 // A visitor with load(j, pj, ex) takes an entry's position and extra data from an array of its own.
 template <class V, class = void> struct OwnLoad : std::false_type {};
 template <class V> struct OwnLoad<V, std::void_t<decltype(&V::load)>> : std::true_type {};
@@ -593,6 +597,16 @@ __device__ __forceinline__ void walk_full(const NbList& F, uint32_t i, uint32_t 
     } else {
 #pragma unroll 1
         while (kb < n) group(std::true_type{});
+        if constexpr (SelfAdds<V>::value) {
+            if (vis.self_adds()) {
+                vis.reset();
+#pragma unroll 1
+                for (uint32_t k = 0; k < n; ++k) {
+                    const uint32_t j = *full_at(F, i, k);
+                    vis.add(contrib_of(vis, j, __ldg(p + j), fetch_extra(vis, j), k < nc), k < nc);
+                }
+            }
+        }
     }
     vis.end_contacts(nc);
 }
@@ -1079,9 +1093,8 @@ struct LambdaVisitT {
         const float dist = sqrt_fast(r2);
         const float r2w = kUnitW ? r2 : __fmaf_rn(rw, rw, r2);
         const float s = spiky_scale(P, dist, r2w);
-        // beyond the cut every kernel is exactly 0: add() leaves the sums alone, as it does for a distance that is
-        // not a number, which lies in neither kernel's range (Density.h:14-42)
-        return Contrib{poly6(P, dist), __fmul_rn(__fmul_rn(s, s), r2w), s, rx, ry, rz, rw, r2, r2 < P.cut2};
+        // beyond the cut every kernel is exactly 0: add() leaves the sums alone
+        return Contrib{poly6(P, dist), __fmul_rn(__fmul_rn(s, s), r2w), s, rx, ry, rz, rw, r2, !(r2 >= P.cut2)};
     }
     __device__ __forceinline__ void add(const Contrib& c, bool) {
         if (!c.near) return;
@@ -1093,7 +1106,8 @@ struct LambdaVisitT {
     // add() of entry k when k < n, as predicated instructions: as a branch the compiler moves the
     // contribution's arithmetic into it, and the entries of a group run one after the other. The tests
     // belong to the same block of instructions: as a flag handed to it they cost a select and a compare
-    // per entry more (1M particles, full lists: delta 244 -> 211 us, lambda 173 -> 169).
+    // per entry more (1M particles, full lists: delta 244 -> 211 us, lambda 173 -> 169).  Near lists only: an
+    // entry whose distance is not a number is left out, as the test of exact positions leaves it out.
     __device__ __forceinline__ void add_if(uint32_t k, uint32_t n, const Contrib& c) {
         asm("{ .reg .pred q; setp.lt.u32 q, %5, %6; setp.lt.and.f32 q, %7, %8, q;"
             " @q add.rn.f32 %0, %0, %9; @q add.rn.f32 %1, %1, %10; @q fma.rn.f32 %2, %11, %12, %2;"
@@ -1104,9 +1118,12 @@ struct LambdaVisitT {
             asm("{ .reg .pred q; setp.lt.u32 q, %1, %2; setp.lt.and.f32 q, %3, %4, q; @q fma.rn.f32 %0, %5, %6, %0; }"
                 : "+f"(Cw) : "r"(k), "r"(n), "f"(c.r2), "f"(P.cut2), "f"(c.s), "f"(c.rw));
     }
-    // The kernels are tested where they are added: within spiky's range r^2 < cut2 holds, and i itself (r = 0, or
-    // NaN where a coordinate is infinite) is in neither range.
+    // The kernels are tested where they are added: within spiky's range (or NaN, which add() passes on)
+    // r^2 < cut2 holds, and i itself (r = 0) is in neither range unless its position is infinite (r NaN).
     static constexpr bool kAddTwo = true;
+    __device__ __forceinline__ bool self_adds() const {
+        return !(fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z) < __int_as_float(0x7f800000));
+    }
     template <bool>
     __device__ __forceinline__ void add_two(uint32_t, const float4& p0, bool, uint32_t, const float4& p1, bool) {
         float x[2], y[2], z[2], w[2], d[2], a[2], W[2], s[2], B2[2];
@@ -1131,12 +1148,12 @@ struct LambdaVisitT {
             asm("{ .reg .pred q; setp.gt.f32 q, %1, %2; setp.lt.and.f32 q, %1, %3, q; @q add.rn.f32 %0, %0, %4; }"
                 : "+f"(A) : "f"(d[b]), "f"(0.001f), "f"(P.hp_lim), "f"(W[b]));
             if constexpr (kUnitW)
-                asm("{ .reg .pred q; setp.gt.f32 q, %4, %6; setp.gt.and.f32 q, %5, %6, q; @q add.rn.f32 %0, %0, %7;"
+                asm("{ .reg .pred q; setp.gtu.f32 q, %4, %6; setp.gtu.and.f32 q, %5, %6, q; @q add.rn.f32 %0, %0, %7;"
                     " @q fma.rn.f32 %1, %8, %9, %1; @q fma.rn.f32 %2, %8, %10, %2; @q fma.rn.f32 %3, %8, %11, %3; }"
                     : "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz)
                     : "f"(d[b]), "f"(a[b]), "f"(0.0001f), "f"(B2[b]), "f"(s[b]), "f"(x[b]), "f"(y[b]), "f"(z[b]));
             else
-                asm("{ .reg .pred q; setp.gt.f32 q, %5, %7; setp.gt.and.f32 q, %6, %7, q; @q add.rn.f32 %0, %0, %8;"
+                asm("{ .reg .pred q; setp.gtu.f32 q, %5, %7; setp.gtu.and.f32 q, %6, %7, q; @q add.rn.f32 %0, %0, %8;"
                     " @q fma.rn.f32 %1, %9, %10, %1; @q fma.rn.f32 %2, %9, %11, %2; @q fma.rn.f32 %3, %9, %12, %3;"
                     " @q fma.rn.f32 %4, %9, %13, %4; }"
                     : "+f"(B), "+f"(Cx), "+f"(Cy), "+f"(Cz), "+f"(Cw)
@@ -1537,7 +1554,8 @@ struct DeltaVisitT {
         }
         if (c.c && k < n) add_contact(c.rx, c.ry, c.rz, c.t);
     }
-    // LambdaVisitT::add_two; a pass of unknown kind (kDeltaAny) adds every entry by itself
+    // LambdaVisitT::add_two (a NaN adds nothing here, so i itself never does); a pass of unknown kind
+    // (kDeltaAny) adds every entry by itself
     static constexpr bool kAddTwo = kKnow;
     template <bool kContacts>   // some entry of the group is a contact (k0, k1: this one)
     __device__ __forceinline__ void add_two(uint32_t j0, const float4& p0, bool k0, uint32_t j1, const float4& p1, bool k1) {
