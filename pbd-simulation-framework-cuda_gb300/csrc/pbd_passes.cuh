@@ -482,8 +482,9 @@ __device__ __forceinline__ void walk_group_sums(E&& entry, uint32_t n, uint32_t 
 
 // filter_list with G lanes per particle (entry k at entry(k), n entries, nc of them contacts; 0 for a
 // group that only takes part): each lane tests every G-th entry, its slot among the group's lanes
-// from a ballot.
-template <int G, class E>
+// from a ballot.  kWalk: an entry whose distance is not a number counts as near, as a walk of the cells
+// counts it.
+template <int G, bool kWalk = false, class E>
 __device__ __forceinline__ uint32_t filter_group(E&& entry, uint32_t n, uint32_t nc, const NbList& L, uint32_t i,
                                                  const float4& pi, float cut2, const float4* __restrict__ p) {
     const uint32_t lane = lane_id(), t = lane & (uint32_t)(G - 1);
@@ -500,7 +501,8 @@ __device__ __forceinline__ uint32_t filter_group(E&& entry, uint32_t n, uint32_t
         for (uint32_t b = 0; b < 4u; ++b) {
             const uint32_t k = kb + b * G + t;
             const float rx = pi.x - pj[b].x, ry = pi.y - pj[b].y, rz = pi.z - pj[b].z;
-            const bool near = k < n && dist2(rx, ry, rz) < cut2;
+            const float r2 = dist2(rx, ry, rz);
+            const bool near = k < n && (kWalk ? !(r2 >= cut2) : r2 < cut2);
             const uint32_t all = (__ballot_sync(kFullMask, near) >> shift) & gmask;
             const uint32_t con = (__ballot_sync(kFullMask, near && k < nc) >> shift) & gmask;
             const uint32_t at = m + __popc(all & ((1u << t) - 1u));
@@ -1270,7 +1272,9 @@ lambda_kernel(DevParams P, const float4* __restrict__ p, const float4* __restric
 
 // One warp computes lambda_i.  With L, it also leaves the particle's near list for the delta pass (and
 // sums over that), or notes the particle in DN: the cell-end range's 512 entries hold ~6 near ones, and
-// walked again in the delta pass they held it up (21 us against 13 for lambda_list with 33k particles).
+// walked again in the delta pass they held it up (21 us against 13 for lambda_list with 33k particles).  Which
+// particles have a row is a matter of which came first: the sums are those of the walk, also of positions that
+// are not numbers.
 __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __restrict__ p, const float4* __restrict__ pa,
                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ ce,
                                             float* __restrict__ lambda, float4* __restrict__ aux, uint32_t i,
@@ -1282,7 +1286,7 @@ __device__ __noinline__ void coop_lambda(const DevParams& P, const float4* __res
     uint32_t lm = kListOff;
     if (L.list) {
         const WarpList W = warp_list(LL, F, i);
-        if (W.row) lm = filter_group<32>([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, L, i, pi, P.cut2, p);
+        if (W.row) lm = filter_group<32, true>([&](uint32_t k) { return W.grouped ? full_at(F, i, k) : W.row + k; }, W.n, W.nc, L, i, pi, P.cut2, p);
         if (lane_id() == 0) {
             L.meta[i] = lm;
             if (lm == kListOff) note_particle(DN, i);

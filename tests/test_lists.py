@@ -530,3 +530,27 @@ def test_far_pairs_that_are_not_numbers(need_gpu, pbd, scenes, shape, stab):
     assert np.isfinite(b["x"][:, :3]).all()
     for k in ("x", "v", "p"):
         assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("numbers", [(20, 20, 20), (30, 30, 30)])
+def test_rows_of_positions_that_are_not_numbers(need_gpu, pbd, scenes, numbers):
+    """9,000 particles whose positions are not numbers (all in cell 0) beside a fluid at the wall: they and the
+    fluid's particles next to them have long rows or, beyond 8,192 of them, walk the cells; what an entry that is
+    not a number does to a sum must not depend on which"""
+    params = scenes.workload_params(pbd, 40, 1000.0, iterations=1)
+    params.lambda_epsilon = 0.1
+    pos, vel = scenes.lattice(*numbers, origin=(1.6, 1.6, 1.6), spacing=0.9, seed=34)
+    lost = np.full((9000, 4), np.nan, np.float32)
+    pos, vel = np.concatenate([pos, lost]), np.concatenate([vel, np.zeros_like(lost)])
+    out = []
+    for flags in (0, 0, pbd.FLAG_FULL_WALK):
+        p = params.copy()
+        p.flags |= flags
+        with pbd.Sim(p, len(pos)) as sim:
+            sim.add_particles(pos, vel)
+            sim.step(1)
+            sim.sync()
+            out.append({**sim.state(), "lambda": sim.debug()["lambda"]})
+    for a in out[:2]:
+        for k in ("x", "v", "p", "lambda"):
+            assert np.array_equal(a[k], out[2][k], equal_nan=True), k
