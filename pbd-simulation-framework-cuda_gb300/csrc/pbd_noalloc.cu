@@ -59,7 +59,7 @@ uint32_t g_hold = 0;
 // Zero the histograms, the tile counters and the error word.  The last tile of a call could leave them zero
 // for the next one, but then a call that did not finish would spoil every later one.  The histogram kernel
 // may start beside this one (a launch that waits for it costs 2 us: 1,048,576 keys 66.5 against 64.6 us,
-// 8,192 25.6 against 23.9; without this kernel 64.9 and 22.6).
+// 8,192 25.6 against 23.6; without this kernel 64.9 and 22.6).
 __global__ void __launch_bounds__(kMaxPasses * kRadix)
 noalloc_clear_kernel(uint32_t* base) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -378,8 +378,8 @@ sort_small_kernel(const uint32_t* kin, uint32_t* kout, uint32_t* vout, uint32_t 
     }
 }
 // Most keys of one block's sort.  A sort by itself (three passes, 21 bits), the tiles' passes against one
-// block: 1,000 keys 18 / 7 us, 4,097 23.9 / (4,096) 14.3, 8,192 23.9 / 22.5 with eight keys per thread, 12,000
-// 23.9 / 39 with sixteen.  Inside a frame, where the passes overlap their launches and the histogram comes
+// block: 1,000 keys 17.4 / 7.1 us, 4,097 23.6 / (4,096) 14.3, 8,192 23.6 / 22.5 with eight keys per thread, 12,000
+// 23.6 / 39 with sixteen.  Inside a frame, where the passes overlap their launches and the histogram comes
 // with the keys: 1,000 particles 47.0 -> 43.6 us per frame, 2,016 48.1 -> 45.4, but 4,096 68.7 against 70.5.
 constexpr uint32_t kSortSmall = 4096;
 constexpr uint32_t kSortSmallFrame = 2048;
